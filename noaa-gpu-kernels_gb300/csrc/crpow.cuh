@@ -73,7 +73,7 @@ CRPOW_HD double crpow_from_bits(uint64_t b)
 #endif
 }
 
-#if defined(__CUDA_ARCH__)
+#if defined(__CUDACC__)
 // Float <-> double conversions for the seed, on the integer pipe (the FP64
 // pipe is the solver's bottleneck): y in [1, 8) truncated to float; a normal
 // float (or +0) widened exactly.
@@ -278,6 +278,58 @@ CRPOW_HD void pow23_53(double x, double* p23, double* p53)
     *p23 = crpow_scale(z23, 2 * k);
     *p53 = crpow_scale(z53, 5 * k);
 }
+
+#if defined(__CUDACC__)
+// x^fl(2/3) and x^fl(5/3) for x in [2^-36, 2^18) with 21 FP64 instructions (the
+// general form above takes 35); where `doubt` comes back set (x outside that
+// range, or a result within 2^-69 relative of a rounding midpoint: ~1 argument
+// in 2^14) the caller takes pow23_53 instead.
+//
+// With the single-precision seed r ~ y^(-1/3) (24 significant bits, so r^2 is
+// exact) and the exact product wh + wl = y r, the defect g = 1 - y r^3 =
+// 1 - (wh + wl) r^2 costs two FMAs and is within 2^-72 of its exact value,
+// |g| < 2^-19.7. Then y^(2/3) = y r (1 - g)^(-1/3) = (wh + wl)(1 + s) with the
+// binomial series s = g/3 + 2 g^2/9 + 14 g^3/81 (the next term is below
+// 2^-77), and x^fl(2/3) = z + (wl + wh (s + c)), x^fl(5/3) = y times that with
+// its own offset -2c, where c = (fl(2/3) - 2/3) ln x comes from the seed's
+// log2 in single precision (|c| < 2^-50, within 2^-74). Relative errors of the
+// sums: g/3 2^-73.6, s, s + c and the product 2^-75 each, wl s 2^-74.4:
+// together below 2^-71.5, a fifth of the rounding test's margin.
+__device__ __forceinline__ void pow23_53_near(double x, double* p23, double* p53, bool& doubt)
+{
+    const int hi = __double2hiint(x);
+    const int u = (hi >> 20) - (1023 - 36);           // exponent + 36
+    doubt |= (unsigned)u >= 54u;                      // also x <= 0, infinite, NaN
+    const int k3 = (u * 43) >> 7;                     // u / 3 for 0 <= u < 127
+    const int k = k3 - 12;
+    const double y = __hiloint2double((hi & 0xfffff) | ((1023 + u - 3 * k3) << 20), __double2loint(x));
+    float l;
+    double r;
+    crpow_seed(y, &l, &r);
+    const float lnx = (l + 3.0f * (float)k) * 0.6931472f;
+    const double c = crpow_widen((float)kFl23Minus23 * lnx);
+    const double wh = y * r;
+    const double wl = __fma_rn(y, r, -wh);
+    const double r2 = r * r;
+    const double g = __fma_rn(-wl, r2, __fma_rn(-wh, r2, 1.0));
+    const double s = g * __fma_rn(g, __fma_rn(g, 14.0 / 81.0, 2.0 / 9.0), 1.0 / 3.0);
+    const double a23 = __fma_rn(wh, s + c, wl);
+    const double z23 = wh + a23;
+    const double w0 = y * wh;
+    const double we = __fma_rn(y, wl, __fma_rn(y, wh, -w0));
+    const double a53 = __fma_rn(w0, __fma_rn(-2.0, c, s), we);   // fl(5/3) - 5/3 = -2 (fl(2/3) - 2/3)
+    const double z53 = w0 + a53;
+    // rounding test on the high words (Fast2Sum: wh >= |a23|, w0 >= |a53|)
+    const double e23 = a23 - (z23 - wh), e53 = a53 - (z53 - w0);
+    const int h23 = __double2hiint(z23), h53 = __double2hiint(z53);
+    // (1 - 2^-15) ulp(z) / 2 = 2^(field(z) - 1077) (2 - 2^-14): see crpow_near_midpoint
+    const int t23 = (((h23 & 0x7ff00000) - (54 << 20)) | 0x000fffc0), t53 = (((h53 & 0x7ff00000) - (54 << 20)) | 0x000fffc0);
+    doubt |= ((__double2hiint(e23) & 0x7fffffff) >= t23) | ((h23 & 0xfffff) == 0) |
+             ((__double2hiint(e53) & 0x7fffffff) >= t53) | ((h53 & 0xfffff) == 0);
+    *p23 = __hiloint2double(h23 + ((2 * k) << 20), __double2loint(z23));
+    *p53 = __hiloint2double(h53 + ((5 * k) << 20), __double2loint(z53));
+}
+#endif
 
 CRPOW_HD double pow23(double x)
 {

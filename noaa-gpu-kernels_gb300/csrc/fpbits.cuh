@@ -101,46 +101,98 @@ __device__ __forceinline__ double twice_chain(double g1, double g2, double g, do
 
 namespace tr {
 
-// Correctly rounded quotients that share one reciprocal.
-//
-// With y = RN(1/b) (CUDA's correctly rounded __drcp_rn), each quotient costs
-// one product and four FMAs instead of a full division: q0 = RN(a y) is within
-// 2 ulp of a/b; one correction q1 = RN(q0 + RN(a - b q0) y) is faithful; then
-// the residual a - b q1 is exact and q2 = RN(q1 + (a - b q1) y) is the
-// correctly rounded a/b (Markstein's theorem, P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
-// Dev. 34(1), 1990; also Muller et al., Handbook of Floating-Point
-// Arithmetic, the FMA-based division section). The theorem needs normal
-// operands and a normal quotient away from overflow: operands whose exponents
-// are far from that range, zeros, infinities and NaNs take the IEEE division.
-struct SharedRcp {
-    double b, y;
-    bool ok;  // b normal, |b| in [2^-500, 2^501)
-};
-
 __device__ __forceinline__ int dexp(double x) { return (int)(((unsigned long long)dbits(x) >> 52) & 0x7ff); }
 
-__device__ __forceinline__ SharedRcp shared_rcp(double b)
+// Quotients with three FP64 instructions each on a shared reciprocal of three.
+//
+// near_rcp: y = 1/b within (1/2 + 2^-11) ulp. A single-precision reciprocal of
+// b's significand (relative error below 2^-21.9, argument truncation included)
+// is scaled on the integer pipe to y0; with e = RN(1 - b y0) the cubic step
+// y = RN(y0 + y0 (e + e^2)) leaves e^3 < 2^-65 before its own rounding (the
+// Newton-Raphson / Householder family, e.g. Muller et al., Handbook of
+// Floating-Point Arithmetic, chapter on division with an FMA).
+//
+// near_quot: q0 = RN(a y), r = RN(a - b q0), q = RN(q0 + r y). y's error and
+// q0's rounding put q0 at most 1.5 ulp (+2^-11) from a/b (1 ulp when a's
+// significand is at least b's), r carries a relative error of at most 2^-53,
+// so q0 + r y before the last rounding is a/b to within 2^-50 ulp and q is the
+// IEEE quotient unless a/b lies that close to a rounding midpoint. Seen from
+// q0 the midpoints lie at +-1/2 and +-3/2 ulp, i.e. at |r| = T and 3 T with
+// T = |b| ulp(q0) / 2, whose bit pattern is b's with q0's exponent added. The
+// high words of |r| and T (20 significand bits) tell when r is within 2^-19 of
+// T; the difference of two high words is a piecewise linear logarithm, and
+// |r| >= 3 T always shows as a difference of at least 1.5 * 2^20 (1.49 is
+// tested; below 3 T it is met only by b's with a significand above 1.96 and a
+// next to them). When q0's significand starts with 20 zeros the quotient may
+// lie in the binade below, with midpoints elsewhere. In these cases -- a few
+// per million quotients -- the caller must divide instead: `doubt` is set
+// and never cleared. Zero residuals never doubt: q0 is then the quotient.
+// Operands: |b| in [2^-400, 2^400], and a = +0 or |a| and |a/b| in the same
+// range (nothing underflows in r). The IEEE division takes about 10 FP64
+// instructions; the correctly rounded reciprocal and two Markstein
+// corrections used before took 8 per divisor and 5 per quotient.
+constexpr int kHalfUlp = 1076 << 20;   // exponent bias plus 53
+constexpr int kThreeHalves = (int)(1.49 * 1048576);
+
+struct NearRcp {
+    double b, y;
+};
+
+__device__ __forceinline__ NearRcp near_rcp(double b)
 {
-    SharedRcp r;
-    r.b = b;
-    const int eb = dexp(b);
-    r.ok = eb >= 1023 - 500 && eb <= 1023 + 500;
-    r.y = r.ok ? __drcp_rn(b) : 0.0;
-    return r;
+    const int hi = __double2hiint(b), lo = __double2loint(b);
+    const float m = __int_as_float((__funnelshift_l(lo, hi, 3) & 0x7fffff) | 0x3f800000);
+    float s;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(m));
+    const int sb = __float_as_int(s);
+    // exponent field 1023 + (field(s) - 127) - (field(b) - 1023), b's sign
+    const int yh = ((sb >> 3) + (1919 << 20) - (hi & 0x7ff00000)) | (hi & 0x80000000);
+    const double y0 = __hiloint2double(yh, sb << 29);
+    const double e = __fma_rn(-b, y0, 1.0);
+    return {b, __fma_rn(y0, __fma_rn(e, e, e), y0)};
 }
 
-__device__ __forceinline__ double shared_div(double a, const SharedRcp& d)
+// Whether the quotient near q0 with residual r may round differently (see above).
+__device__ __forceinline__ bool quot_doubt(double b, double q0, double r)
 {
-    const int ea = dexp(a);
-    // a normal and |a|, |b| in [2^-500, 2^501): |a/b| is far inside the normal
-    // range; else the IEEE division
-    if (!d.ok || ea < 1023 - 500 || ea > 1023 + 500) return a / d.b;
-    double q = a * d.y;
-    double r = __fma_rn(-d.b, q, a);
-    q = __fma_rn(r, d.y, q);
-    r = __fma_rn(-d.b, q, a);
-    return __fma_rn(r, d.y, q);
+    const int hq = __double2hiint(q0), hr = __double2hiint(r) & 0x7fffffff;
+    const int t = max((__double2hiint(b) & 0x7fffffff) - kHalfUlp + (hq & 0x7ff00000), 4);
+    const int d = hr - t;
+    return ((unsigned)(d + 1) <= 2u) | (d >= kThreeHalves) | (((hq & 0xfffff) == 0) & (hr != 0));
+}
+
+__device__ __forceinline__ double near_quot(double a, const NearRcp& d, bool& doubt)
+{
+    const double q0 = a * d.y;
+    const double r = __fma_rn(-d.b, q0, a);
+    doubt |= quot_doubt(d.b, q0, r);
+    return __fma_rn(r, d.y, q0);
+}
+
+// 1 / b: the reciprocal itself takes q0's place.
+__device__ __forceinline__ double near_one_over(double b, bool& doubt)
+{
+    const double q0 = near_rcp(b).y;
+    const double r = __fma_rn(-b, q0, 1.0);
+    doubt |= quot_doubt(b, q0, r);
+    return __fma_rn(r, q0, q0);
+}
+
+// |x| in [2^-n, 2^n) by the exponent field
+__device__ __forceinline__ bool fp_within(double x, int n)
+{
+    return (unsigned)((__double2hiint(x) & 0x7fffffff) - ((1023 - n) << 20)) < ((unsigned)n << 21);
+}
+
+// The IEEE quotient a / b for any operands, by near_quot where it applies.
+__device__ __forceinline__ double quot_ieee(double a, double b)
+{
+    if (fp_within(b, 400) && fp_within(a, 400)) {
+        bool doubt = false;
+        const double q = near_quot(a, near_rcp(b), doubt);
+        if (!doubt) return q;
+    }
+    return a / b;
 }
 
 // RN(a / b) > c -- the IEEE quotient compared with c -- for any a, b > 0 and

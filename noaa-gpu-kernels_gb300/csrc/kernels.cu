@@ -218,11 +218,7 @@ __global__ void velocity_kernel(NetDev net)
         double vel = 0.0;
         if (!(p.n_ch <= 0.0 || p.s0 <= 0.0 || p.z <= 0.0 || p.bw <= 0.0)) {
             const double h = __ldcg(net.d + s);
-            const double twl = p.bw + p.z2 * h;
-            double Rv = (h * (p.bw + twl) / 2.0) /
-                        (p.bw + 2.0 * sqrt(((twl - p.bw) / 2.0) * ((twl - p.bw) / 2.0) + h * h));
-            if (Rv < 0.0) Rv = 0.0;
-            vel = (1.0 / p.n_ch) * pow23(Rv) * p.sq_s0;
+            vel = seg_velocity(p, h);
         }
         __stcg(net.v + s, vel);
     }
@@ -232,7 +228,7 @@ __global__ void debug_div_kernel(const double* __restrict__ a, const double* __r
                                  double* __restrict__ out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = shared_div(a[i], shared_rcp(b[i]));
+    if (i < n) out[i] = quot_ieee(a[i], b[i]);
 }
 
 __global__ void debug_quot_gt_kernel(const double* __restrict__ a, const double* __restrict__ b, double c, int n,
@@ -246,7 +242,9 @@ __global__ void debug_pow_kernel(const double* __restrict__ x, int n, double* __
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         double a, b;
-        pow23_53(x[i], &a, &b);
+        bool doubt = false;
+        pow23_53_near(x[i], &a, &b, doubt);
+        if (doubt) pow23_53(x[i], &a, &b);
         out[i] = a;
         out[n + i] = b;
         out[2 * n + i] = pow(x[i], 2.0 / 3.0);

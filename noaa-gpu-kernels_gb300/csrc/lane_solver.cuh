@@ -18,7 +18,6 @@
 #pragma once
 
 #include "device_common.cuh"
-#include "fpbits.cuh"
 
 namespace tr {
 
@@ -119,11 +118,12 @@ struct Lane {
     double qup_head, quc_head, q_up_old, q_up_new, q_last;
     // current segment
     long long s;
-    double qup, quc, qdp, ql;
+    double qup, quc, qdp, qldt;   // qldt = ql dt
     double h, h_0, Qj_0, qdc;
     double dpp;            // previous depth (clamped at 0): the plain bracket's centre
     DepthEval e0;
     int need0, iter, attempt, maxiter, total, retried, warm;
+    bool irregular;        // outside the ranges of the short arithmetic (mc_solve.cuh)
 };
 
 // The plain starting bracket from the previous depth (troute_mc_final.cu:193).
@@ -159,12 +159,11 @@ __device__ __forceinline__ bool begin_segment(Lane& L, const NetDev& net, const 
         const double dpp = __ldcg(net.d + L.s);
         const double2 tail = buf[kParamPlanes * kSegSmemStride];
         const long long tw = __double_as_longlong(tail.y);
-        L.ql = __ldg(qlat_row + (int)(unsigned)(tw & 0xffffffffll)) * tail.x;   // column: the low word
+        const double ql = __ldg(qlat_row + (int)(unsigned)(tw & 0xffffffffll)) * tail.x;   // column: the low word
         const SegP p = staged_seg(buf);
         L.qup = (L.i == 0) ? L.qup_head : L.q_up_old;
         L.quc = (L.i == 0) ? L.quc_head : L.q_up_new;
-        if (p.n_ch <= 0.0 || p.s0 <= 0.0 || p.z <= 0.0 || p.bw <= 0.0 ||
-            (L.ql <= 0.0 && L.qup <= 0.0 && L.quc <= 0.0 && L.qdp <= 0.0)) {
+        if (exits_early(p, ql, L.qup, L.quc, L.qdp)) {
             __stcg(net.q + L.s, 0.0);
             __stcg(net.d + L.s, 0.0);
             __stcg(net.v + L.s, 0.0);
@@ -180,6 +179,9 @@ __device__ __forceinline__ bool begin_segment(Lane& L, const NetDev& net, const 
             ++L.i;
             continue;
         }
+        L.qldt = ql * run.dt;
+        L.irregular = !(seg_regular(p, run.dt) && flow_regular(L.qup) && flow_regular(L.quc) && flow_regular(L.qdp) &&
+                        flow_regular(L.qldt));
         L.dpp = fmax(dpp, 0.0);
         plain_bracket(L, run.tol);
         L.total = 0;
@@ -210,123 +212,24 @@ __device__ __forceinline__ void lane_pass(Lane& L, const NetDev& net, const RunD
                                           unsigned int* hist_s, double2* slot)
 {
     const Tol& tol = run.tol;
-    const double dt = run.dt;
-    const double dt2 = run.dt_half;  // dt / 2 (exact), formed on the host
     if (L.mode == L_SOLVE) {
         // the segment's parameters, staged in shared memory
         const SegP p = staged_seg(seg_buf(slot, L.i));
-        const double x = L.need0 ? L.h_0 : L.h;  // >= +0
-        // Every comparison, minimum and maximum of the pass runs on the integer
-        // pipes (fpbits.cuh: the IEEE results, bit for bit), leaving the FP64
-        // pipe to the arithmetic.
-        const bool twcc_pos = fp_gt0(p.twcc);
-        const double twl = p.bw + p.z2 * x;  // bw + 2 z x
-        double above = fp_max0(x - p.bfd);
-        double below = fp_min_pos(p.bfd, x);
-        if (fp_gt0(above) && (fp_lt0(p.twcc) || fp_eq0(p.twcc))) {
-            above = 0.0;
-            below = x;
-        }
-        const double A = (p.bw + below * p.z) * below;
-        const double WP = p.bw + below * p.sq2;  // bw + 2 below sqrt(1+z^2)
-        // the compound-channel terms: area A + AC, wetted perimeter P = WP + WPC,
-        // conveyance weight WP n + WPC ncc
-        double AAC, P, WPn;
-        if (fp_gt0(above) || !fp_finite(p.twcc) || !fp_finite(p.ncc)) {
-            const double AC = p.twcc * above;
-            const double WPC = fp_gt0(above) ? (p.twcc + 2.0 * above) : 0.0;
-            AAC = A + AC;
-            P = WP + WPC;
-            WPn = WP * p.n_ch + WPC * p.ncc;
-        } else {
-            // in bank (above = +0) with finite twcc, ncc: AC = +-0 and WPC = 0,
-            // and adding a zero to A >= +0, WP > 0 or WP n > 0 returns it unchanged
-            AAC = A;
-            P = WP;
-            WPn = WP * p.n_ch;
-        }
-        const bool P_pos = fp_gt0(P);
-        // the two quotients by P share one correctly rounded reciprocal
-        const SharedRcp rP = shared_rcp(P_pos ? P : 1.0);
-        const double R = P_pos ? shared_div(AAC, rP) : 0.0;
-        double r23, r53;
-        pow23_53(R, &r23, &r53);
+        const PassFlow f = {L.qup, L.quc, L.qdp, L.qldt, run.dt, run.dt_half};
         {
             DepthEval e;
-            e.Ck = 0.0;
-            // 2 sqrt(1+z^2) / (bw + 2 x z): the denominator is twl
-            if (fp_gt0(x)) e.Ck = fp_max0(p.ck_fac * ((5.0 / 3.0) * r23 - (2.0 / 3.0) * r53 * (p.sq2 / twl)));
-            e.Km = fp_gt0(e.Ck) ? fp_max_pos(dt, p.dx / e.Ck) : dt;
-            e.twu = (fp_gt_pos(x, p.bfd) && twcc_pos) ? p.twcc : twl;
-            // 1.0 / t is the correctly rounded reciprocal of t
-            e.Qmn = P_pos ? __drcp_rn(shared_div(WPn, rP)) * AAC * r23 * p.sq_s0 : 0.0;
+            PassOut o;
+            secant_pass(p, f, L.need0 ? L.h_0 : L.h, L.need0, L.h, L.h_0, L.Qj_0, L.e0, L.irregular, e, o);
+            L.e0 = e;
             if (L.need0) {
-                L.e0 = e;
                 L.need0 = 0;
             } else {
-                const double qup = L.qup, quc = L.quc, qdp = L.qdp, ql = L.ql;
-                const DepthEval& e0 = L.e0;
-                // X at the lower depth, clamped to [0, 0.5] (troute_mc_final.cu:86)
-                double X0 = 0.5;
-                {
-                    const double g1 = e0.twu * p.s0, g2 = g1 * e0.Ck, g = g2 * p.dx;
-                    if (fp_gt0(e0.Ck) && fp_gt0(g))
-                        X0 = fp_min_pos(0.5, fp_max0(fp_half(1.0 - L.Qj_0 / twice_chain(g1, g2, g, e0.twu, p.s0, e0.Ck, p.dx))));
-                }
-                double D0 = e0.Km * (1.0 - X0) + dt2;
-                if (fp_eq0(D0)) D0 = 1.0;
-                const SharedRcp r0 = shared_rcp(D0);
-                const double c1 = shared_div(e0.Km * X0 + dt2, r0);
-                const double c2 = shared_div(dt2 - e0.Km * X0, r0);
-                const double c3 = shared_div(e0.Km * (1.0 - X0) - dt2, r0);
-                const double c4 = shared_div(ql * dt, r0);
-                const double qmc0 = c1 * qup + c2 * quc + c3 * qdp + c4;
-                L.Qj_0 = qmc0 - e0.Qmn;
-                // X at the upper depth, clamped to [0.25, 0.5] (troute_mc_final.cu:105)
-                double X = 0.5;
-                {
-                    const double g1 = e.twu * p.s0, g2 = g1 * e.Ck, g = g2 * p.dx;
-                    if (fp_gt0(e.Ck) && fp_gt0(g))
-                        X = fp_min_pos(0.5, fp_max_pos(0.25, fp_half(1.0 - qmc0 / twice_chain(g1, g2, g, e.twu, p.s0, e.Ck, p.dx))));
-                }
-                double D1 = e.Km * (1.0 - X) + dt2;
-                if (fp_eq0(D1)) D1 = 1.0;
-                const SharedRcp r1 = shared_rcp(D1);
-                const double C1 = shared_div(e.Km * X + dt2, r1);
-                const double C2 = shared_div(dt2 - e.Km * X, r1);
-                const double C3 = shared_div(e.Km * (1.0 - X) - dt2, r1);
-                double C4 = shared_div(ql * dt, r1);
-                const double S3 = C1 * qup + C2 * quc + C3 * qdp;
-                if (fp_lt0(C4) && fp_abs_gt(C4, S3)) C4 = -S3;
-                const double Qj = (S3 + C4) - e.Qmn;
-                // outflow of the last evaluated coefficients (troute_mc_final.cu:125-130)
-                const double Qmc = S3 + C4;
-                if (fp_lt0(Qmc)) {
-                    if (fp_lt0(C4) && fp_abs_gt(C4, S3))
-                        L.qdc = 0.0;
-                    else
-                        L.qdc = fmax(C1 * qup + C2 * quc + C4, C1 * qup + C3 * qdp + C4);
-                } else {
-                    L.qdc = Qmc;
-                }
+                L.Qj_0 = o.Qj_0;
+                L.qdc = o.qdc;
                 const double h = L.h;
-                const double dQ = L.Qj_0 - Qj;
-                double h_1 = !fp_eq0(dQ) ? h - (Qj * (L.h_0 - h)) / dQ : h;
-                if (fp_lt0(h_1)) h_1 = h;
-                // the reference's test rerr > rtol && aerr >= atol with
-                // rerr = |(h_1 - h) / h|, aerr = |h_1 - h| (rerr = 0, aerr = 0.9
-                // for h <= 0); the relative error's quotient is only compared
-                // with rtol, which quot_gt_pos does exactly without dividing
-                bool more;
-                if (fp_gt0(h)) {
-                    const double aerr = fp_abs(h_1 - h);
-                    more = fp_ge_nonneg(aerr, tol.atol) && quot_gt_pos(aerr, h, tol.rtol);
-                } else {
-                    more = fp_gt_pos(0.0, tol.rtol) && fp_ge_nonneg(0.9, tol.atol);
-                }
+                const bool more = secant_more(h, o.h_1, tol);
                 L.h_0 = fp_max0(h);
-                L.h = fp_max0(h_1);
-                L.e0 = e;
+                L.h = fp_max0(o.h_1);
                 ++L.iter;
                 ++L.total;
                 bool stop;
@@ -369,7 +272,9 @@ __device__ __forceinline__ void lane_pass(Lane& L, const NetDev& net, const RunD
                             pr[0] = (float)L.qup;
                             pr[1] = (float)L.quc;
                             pr[2] = (float)L.qdp;
-                            pr[3] = (float)L.ql;
+                            const double2 tail = seg_buf(slot, L.i)[kParamPlanes * kSegSmemStride];
+                            const int col = (int)(unsigned)(__double_as_longlong(tail.y) & 0xffffffffll);
+                            pr[3] = (float)(__ldg(run.qlat + (size_t)L.tau * (size_t)run.qlat_ld + col) * tail.x);
                             pr[4] = (float)p.dx;
                             pr[5] = (float)p.s0;
                             pr[6] = (float)p.n_ch;

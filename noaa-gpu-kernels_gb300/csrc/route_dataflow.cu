@@ -103,12 +103,16 @@ __device__ __forceinline__ void start_item(Lane& L, int ri, int tau, int t_base,
 }
 
 // Threads per block, and the register budget: resident blocks per SM the
-// allocation is sized for, or (TROUTE_DF_MAXNREG) a register cap.
+// allocation is sized for, or (TROUTE_DF_MAXNREG) a register cap. Three blocks
+// of 128 (164 registers; 178 without the bound, which would leave two): four
+// blocks spill 176 B and are slower everywhere (64 members of a 20,000-segment
+// tree, warm start, 16 steps: 128.5 against 124.0 ms; a 200,000-segment tree, 24
+// steps: 218 against 196 ms), 64-thread blocks at 14-16 warps likewise.
 #ifndef TROUTE_DF_THREADS
 #define TROUTE_DF_THREADS 128
 #endif
 #ifndef TROUTE_DF_MINB
-#define TROUTE_DF_MINB 1
+#define TROUTE_DF_MINB 3
 #endif
 #ifdef TROUTE_DF_MAXNREG
 #define TROUTE_DF_BOUNDS __maxnreg__(TROUTE_DF_MAXNREG)
