@@ -127,8 +127,8 @@ __device__ __forceinline__ int dexp(double x) { return (int)(((unsigned long lon
 // lie in the binade below, with midpoints elsewhere. In these cases -- a few
 // per million quotients -- the caller must divide instead: `doubt` is set
 // and never cleared. Zero residuals never doubt: q0 is then the quotient.
-// Operands: |b| in [2^-400, 2^400], and a = +0 or |a| and |a/b| in the same
-// range (nothing underflows in r). The IEEE division takes about 10 FP64
+// Operands: b normal, |b| < 2^1022; a = +0 or |a| >= 2^-900; q0 normal (nothing
+// underflows in y or r). The IEEE division takes about 10 FP64
 // instructions; the correctly rounded reciprocal and two Markstein
 // corrections used before took 8 per divisor and 5 per quotient.
 constexpr int kHalfUlp = 1076 << 20;   // exponent bias plus 53
@@ -138,7 +138,8 @@ struct NearRcp {
     double b, y;
 };
 
-__device__ __forceinline__ NearRcp near_rcp(double b)
+// y0: single-precision 1/b as a double
+__device__ __forceinline__ double rcp_seed(double b)
 {
     const int hi = __double2hiint(b), lo = __double2loint(b);
     const float m = __int_as_float((__funnelshift_l(lo, hi, 3) & 0x7fffff) | 0x3f800000);
@@ -147,7 +148,12 @@ __device__ __forceinline__ NearRcp near_rcp(double b)
     const int sb = __float_as_int(s);
     // exponent field 1023 + (field(s) - 127) - (field(b) - 1023), b's sign
     const int yh = ((sb >> 3) + (1919 << 20) - (hi & 0x7ff00000)) | (hi & 0x80000000);
-    const double y0 = __hiloint2double(yh, sb << 29);
+    return __hiloint2double(yh, sb << 29);
+}
+
+__device__ __forceinline__ NearRcp near_rcp(double b)
+{
+    const double y0 = rcp_seed(b);
     const double e = __fma_rn(-b, y0, 1.0);
     return {b, __fma_rn(y0, __fma_rn(e, e, e), y0)};
 }

@@ -124,6 +124,8 @@ struct Lane {
     DepthEval e0;
     int need0, iter, attempt, maxiter, total, retried, warm;
     bool irregular;        // outside the ranges of the short arithmetic (mc_solve.cuh)
+    bool ahead;            // qmc0_n and Qj0_n hold the next pass's lower discharge and residual (narrow_pass.cuh)
+    double qmc0_n, Qj0_n;
 };
 
 // The plain starting bracket from the previous depth (troute_mc_final.cu:193).
@@ -137,6 +139,7 @@ __device__ __forceinline__ void plain_bracket(Lane& L, const Tol& tol)
     L.attempt = 0;
     L.iter = 0;
     L.need0 = 1;
+    L.ahead = false;
 }
 
 // Starts segment L.i of the lane's reach; consecutive segments that exit early
@@ -207,94 +210,106 @@ __device__ __forceinline__ bool begin_segment(Lane& L, const NetDev& net, const 
     return false;
 }
 
-// One evaluation pass of a lane in SOLVE or VEL mode (no-op otherwise).
+// Books one secant iteration of a lane whose pass produced o and (already in
+// L.e0) the upper depth's evaluation: the bracket, the stop test, and at a stop
+// the stores and the move to the next segment.
+__device__ __forceinline__ void lane_finish(Lane& L, const PassOut& o, const NetDev& net, const RunDev& run,
+                                            LocalStats& ls, unsigned int* hist_s, double2* slot)
+{
+    const Tol& tol = run.tol;
+    L.Qj_0 = o.Qj_0;
+    L.qdc = o.qdc;
+    const double h = L.h;
+    const bool more = secant_more(h, o.h_1, tol);
+    L.h_0 = fp_max0(h);
+    L.h = fp_max0(o.h_1);
+    ++L.iter;
+    ++L.total;
+    bool stop;
+    if (L.warm == W_ACTIVE) {
+        // warm phase: accepted once the stop test passes at a depth of at
+        // least kMinDepth; otherwise, after warm_k passes (or below
+        // kMinDepth), the plain solve restarts from the previous depth
+        const bool below_min = fp_lt_pos(L.h, kMinDepth);
+        stop = !more && !below_min;
+        if (!stop && (below_min || L.iter >= run.warm_k)) {
+            L.warm = W_PLAIN;
+            ls.warm_fallback++;
+            plain_bracket(L, tol);
+        }
+    } else {
+        stop = fp_lt_pos(L.h, kMinDepth) || !(more && L.iter <= L.maxiter);
+    }
+    if (stop) {
+        bool done = true;
+        if (L.warm == W_PLAIN && L.iter >= L.maxiter) {
+            // widen the bracket (also after the last attempt, as the reference does)
+            L.h *= 1.33;
+            L.h_0 *= 0.67;
+            L.maxiter += 25;
+            L.retried = 1;
+            if (++L.attempt < tol.attempts) {
+                L.iter = 0;
+                L.need0 = 1;
+                L.ahead = false;
+                done = false;
+            }
+        }
+        if (done) {
+            // store the segment (its velocity is derived from the final depth
+            // once the run is over, see velocity_kernel) and start the next one
+            __stcg(net.q + L.s, L.qdc);
+            __stcg(net.d + L.s, L.h);
+            if (run.q_hist) __stcg(run.q_hist + (size_t)L.tau * (size_t)net.n_seg_int + L.s, L.qdc);
+            if (run.pairs) {
+                float* pr = run.pairs + ((size_t)L.tau * (size_t)net.n_seg_int + L.s) * 9;
+                pr[0] = (float)L.qup;
+                pr[1] = (float)L.quc;
+                pr[2] = (float)L.qdp;
+                const SegP p = staged_seg(seg_buf(slot, L.i));
+                const double2 tail = seg_buf(slot, L.i)[kParamPlanes * kSegSmemStride];
+                const int col = (int)(unsigned)(__double_as_longlong(tail.y) & 0xffffffffll);
+                pr[3] = (float)(__ldg(run.qlat + (size_t)L.tau * (size_t)run.qlat_ld + col) * tail.x);
+                pr[4] = (float)p.dx;
+                pr[5] = (float)p.s0;
+                pr[6] = (float)p.n_ch;
+                pr[7] = (float)p.bw;
+                pr[8] = (float)L.h;
+            }
+            L.q_up_old = L.qdp;
+            L.q_up_new = L.qdc;
+            L.q_last = L.qdc;
+            SolveOut o;
+            o.iters = L.total;
+            o.retried = L.retried;
+            o.early = 0;
+            count_solve(ls, hist_s, o);
+            ++L.i;
+            L.mode = L.i < L.ns ? L_BEGIN : L_DONE;
+        }
+    }
+}
+
+// One evaluation pass of a lane in SOLVE mode (no-op otherwise).
+__device__ __forceinline__ bool lane_eval(Lane& L, const RunDev& run, double2* slot, PassOut& o)
+{
+    const SegP p = staged_seg(seg_buf(slot, L.i));
+    const PassFlow f = {L.qup, L.quc, L.qdp, L.qldt, run.dt, run.dt_half};
+    DepthEval e;
+    secant_pass(p, f, L.need0 ? L.h_0 : L.h, L.need0, L.h, L.h_0, L.Qj_0, L.e0, L.irregular, e, o);
+    L.e0 = e;
+    L.ahead = false;
+    const bool iterated = !L.need0;
+    L.need0 = 0;
+    return iterated;
+}
+
 __device__ __forceinline__ void lane_pass(Lane& L, const NetDev& net, const RunDev& run, LocalStats& ls,
                                           unsigned int* hist_s, double2* slot)
 {
-    const Tol& tol = run.tol;
     if (L.mode == L_SOLVE) {
-        // the segment's parameters, staged in shared memory
-        const SegP p = staged_seg(seg_buf(slot, L.i));
-        const PassFlow f = {L.qup, L.quc, L.qdp, L.qldt, run.dt, run.dt_half};
-        {
-            DepthEval e;
-            PassOut o;
-            secant_pass(p, f, L.need0 ? L.h_0 : L.h, L.need0, L.h, L.h_0, L.Qj_0, L.e0, L.irregular, e, o);
-            L.e0 = e;
-            if (L.need0) {
-                L.need0 = 0;
-            } else {
-                L.Qj_0 = o.Qj_0;
-                L.qdc = o.qdc;
-                const double h = L.h;
-                const bool more = secant_more(h, o.h_1, tol);
-                L.h_0 = fp_max0(h);
-                L.h = fp_max0(o.h_1);
-                ++L.iter;
-                ++L.total;
-                bool stop;
-                if (L.warm == W_ACTIVE) {
-                    // warm phase: accepted once the stop test passes at a depth of at
-                    // least kMinDepth; otherwise, after warm_k passes (or below
-                    // kMinDepth), the plain solve restarts from the previous depth
-                    const bool below_min = fp_lt_pos(L.h, kMinDepth);
-                    stop = !more && !below_min;
-                    if (!stop && (below_min || L.iter >= run.warm_k)) {
-                        L.warm = W_PLAIN;
-                        ls.warm_fallback++;
-                        plain_bracket(L, tol);
-                    }
-                } else {
-                    stop = fp_lt_pos(L.h, kMinDepth) || !(more && L.iter <= L.maxiter);
-                }
-                if (stop) {
-                    bool done = true;
-                    if (L.warm == W_PLAIN && L.iter >= L.maxiter) {
-                        // widen the bracket (also after the last attempt, as the reference does)
-                        L.h *= 1.33;
-                        L.h_0 *= 0.67;
-                        L.maxiter += 25;
-                        L.retried = 1;
-                        if (++L.attempt < tol.attempts) {
-                            L.iter = 0;
-                            L.need0 = 1;
-                            done = false;
-                        }
-                    }
-                    if (done) {
-                        // store the segment (its velocity is derived from the final depth
-                        // once the run is over, see velocity_kernel) and start the next one
-                        __stcg(net.q + L.s, L.qdc);
-                        __stcg(net.d + L.s, L.h);
-                        if (run.q_hist) __stcg(run.q_hist + (size_t)L.tau * (size_t)net.n_seg_int + L.s, L.qdc);
-                        if (run.pairs) {
-                            float* pr = run.pairs + ((size_t)L.tau * (size_t)net.n_seg_int + L.s) * 9;
-                            pr[0] = (float)L.qup;
-                            pr[1] = (float)L.quc;
-                            pr[2] = (float)L.qdp;
-                            const double2 tail = seg_buf(slot, L.i)[kParamPlanes * kSegSmemStride];
-                            const int col = (int)(unsigned)(__double_as_longlong(tail.y) & 0xffffffffll);
-                            pr[3] = (float)(__ldg(run.qlat + (size_t)L.tau * (size_t)run.qlat_ld + col) * tail.x);
-                            pr[4] = (float)p.dx;
-                            pr[5] = (float)p.s0;
-                            pr[6] = (float)p.n_ch;
-                            pr[7] = (float)p.bw;
-                            pr[8] = (float)L.h;
-                        }
-                        L.q_up_old = L.qdp;
-                        L.q_up_new = L.qdc;
-                        L.q_last = L.qdc;
-                        SolveOut o;
-                        o.iters = L.total;
-                        o.retried = L.retried;
-                        o.early = 0;
-                        count_solve(ls, hist_s, o);
-                        ++L.i;
-                        L.mode = L.i < L.ns ? L_BEGIN : L_DONE;
-                    }
-                }
-            }
-        }
+        PassOut o;
+        if (lane_eval(L, run, slot, o)) lane_finish(L, o, net, run, ls, hist_s, slot);
     }
 }
 

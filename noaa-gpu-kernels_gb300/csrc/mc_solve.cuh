@@ -75,8 +75,13 @@ struct PassOut {
 };
 
 // Parameter and time-step ranges in which the short forms are proven: with
-// these, depths in [2^-100, 2^60) and flows below 2^100 every intermediate is
-// zero or far inside the normal range.
+// these, depths of +0 or in [2^-100, 2^480) and flows below 2^100 every
+// intermediate but the secant's numerator (checked) is zero or inside the normal
+// range with room for its residual. The depths reach that far in earnest: where
+// the secant does not converge it doubles its bracket pass after pass, to 1e136
+// and beyond, until maxiter (at rtol 1e-8 one iteration in four is spent at
+// depths above 1e18 m). Above the bank the area is bounded by linear terms, so
+// R tends to twcc / 2 and the discharge grows like the depth.
 __device__ __forceinline__ bool seg_regular(const SegP& p, double dt)
 {
     const double v[13] = {p.dx, p.bw, p.twcc, p.n_ch, p.ncc, p.s0, p.z, p.bfd, p.sq_s0, p.sq2, p.ck_fac, p.z2, dt};
@@ -86,6 +91,15 @@ __device__ __forceinline__ bool seg_regular(const SegP& p, double dt)
     return ok;
 }
 
+// A positive depth in [2^-100, 2^480).
+__device__ __forceinline__ bool depth_regular(double x)
+{
+    return (unsigned)(__double2hiint(x) - (923 << 20)) < (580u << 20);
+}
+
+// The secant's numerator is below 2^1000.
+__device__ __forceinline__ bool numerator_regular(double v) { return (__double2hiint(v) & 0x7fffffff) < (2023 << 20); }
+
 // +0, or a magnitude in [2^-150, 2^100).
 __device__ __forceinline__ bool flow_regular(double q)
 {
@@ -93,11 +107,22 @@ __device__ __forceinline__ bool flow_regular(double q)
     return (unsigned)((h & 0x7fffffff) - (873 << 20)) < (250u << 20) || (h | __double2loint(q)) == 0;
 }
 
-// Evaluation at x (a regular segment, x = +0 or in [2^-100, 2^60), else doubt).
+// X = (1 - q) / 2 clamped to [lo, 1/2] from v = 1 - q, on the high words: below 1
+// the half is the exponent lowered by one (v is at least 2^-53 there). lo2 is the
+// high word of 2 lo: 0 for lo = 0, 0x3fe00000 for lo = 1/4.
+__device__ __forceinline__ double clamped_half(double v, int lo2)
+{
+    const int h = __double2hiint(v);
+    const double x = __hiloint2double(h - (1 << 20), __double2loint(v));
+    const double lo = __hiloint2double(lo2 ? lo2 - (1 << 20) : 0, 0);
+    return h >= 0x3ff00000 ? 0.5 : h <= 0 || h < lo2 ? lo : x;
+}
+
+// Evaluation at x (a regular segment; doubt when x is neither +0 nor regular).
 __device__ __forceinline__ void eval_near(double x, const SegP& p, double dt, DepthEval& e, bool& doubt)
 {
     const bool wet = (__double2hiint(x) | __double2loint(x)) != 0;
-    bool unsure = (unsigned)(__double2hiint(x) - (923 << 20)) >= (160u << 20);
+    bool unsure = !depth_regular(x);
     const double twl = p.bw + p.z2 * x;  // bw + 2 z x
     const bool over = dbits(x) > dbits(p.bfd);
     const double below = over ? p.bfd : x;
@@ -122,7 +147,7 @@ __device__ __forceinline__ void eval_near(double x, const SegP& p, double dt, De
     e.Qmn = near_one_over(near_quot(WPn, rP, unsure), unsure) * AAC * r23 * p.sq_s0;
     bool unsure_k = false;
     const double K = near_quot(p.dx, near_rcp(Ck), unsure_k);
-    const bool moves = wet && fp_gt0(Ck);
+    const bool moves = wet && __double2hiint(Ck) > 0;
     e.Km = moves ? fp_max_pos(dt, K) : dt;
     const double g = (over ? p.twcc : twl) * p.s0 * Ck * p.dx;
     // 2.0 * tw * s0 * Ck * dx is exactly twice the undoubled product
@@ -138,7 +163,7 @@ __device__ __forceinline__ void update_near(const DepthEval& e0, const DepthEval
 {
     // X at the lower depth, clamped to [0, 0.5] (troute_mc_final.cu:86)
     bool d0 = false, d1 = false, d2 = false;
-    double X0 = fp_min_pos(0.5, fp_max0(fp_half(1.0 - near_quot(Qj_0, {e0.G, e0.yG}, d0))));
+    double X0 = clamped_half(1.0 - near_quot(Qj_0, {e0.G, e0.yG}, d0), 0);
     const bool v0 = dbits(e0.yG) != 0, v1 = dbits(e.yG) != 0;
     if (!v0) X0 = 0.5;
     const double KX0 = e0.Km * X0, K10 = e0.Km * (1.0 - X0);
@@ -150,7 +175,7 @@ __device__ __forceinline__ void update_near(const DepthEval& e0, const DepthEval
     const double qmc0 = c1 * f.qup + c2 * f.quc + c3 * f.qdp + c4;
     o.Qj_0 = qmc0 - e0.Qmn;
     // X at the upper depth, clamped to [0.25, 0.5] (troute_mc_final.cu:105)
-    double X = fp_min_pos(0.5, fp_max_pos(0.25, fp_half(1.0 - near_quot(qmc0, {e.G, e.yG}, d1))));
+    double X = clamped_half(1.0 - near_quot(qmc0, {e.G, e.yG}, d1), 0x3fe00000);
     if (!v1) X = 0.5;
     const double KX = e.Km * X, K1 = e.Km * (1.0 - X);
     const NearRcp r1 = near_rcp(K1 + f.dt2);
@@ -172,7 +197,9 @@ __device__ __forceinline__ void update_near(const DepthEval& e0, const DepthEval
     }
     const double dQ = o.Qj_0 - Qj;
     const bool slope = !fp_eq0(dQ);
-    o.h_1 = slope ? h - near_quot(Qj * (h_0 - h), near_rcp(dQ), d2) : h;
+    const double num = Qj * (h_0 - h);
+    o.h_1 = slope ? h - near_quot(num, near_rcp(dQ), d2) : h;
+    d2 |= !numerator_regular(num);
     if (fp_lt0(o.h_1)) o.h_1 = h;
     doubt |= (v0 & d0) | (v1 & d1) | (slope & d2);
 }
@@ -258,30 +285,35 @@ static __device__ __noinline__ void exact_pass(ExactPass* a)
     a->o.h_1 = h_1;
 }
 
+// exact_pass on the values of a pass; irregular is set when a depth or
+// denominator has left the ranges of the short forms.
+__device__ __forceinline__ void redo_pass(const SegP& p, const PassFlow& f, double x, bool need0, double h, double h_0,
+                                          double Qj_0, const DepthEval& e0, bool& irregular, DepthEval& e, PassOut& o)
+{
+    ExactPass a;
+    a.p = p;
+    a.f = f;
+    a.x = x;
+    a.h = h;
+    a.h_0 = h_0;
+    a.Qj_0 = Qj_0;
+    a.e0 = e0;
+    a.need0 = need0;
+    exact_pass(&a);
+    e = a.e;
+    if (!need0) o = a.o;
+    irregular |= !(x == 0.0 || depth_regular(x)) || !fp_within(e.G, 400);
+}
+
 // One pass: the evaluation at x into e; unless need0 also the update from e0
-// into o. irregular: the segment or its flows are outside the proven ranges (set
-// here when a depth is).
+// into o. irregular: the segment or its flows are outside the proven ranges.
 __device__ __forceinline__ void secant_pass(const SegP& p, const PassFlow& f, double x, bool need0, double h, double h_0,
                                             double Qj_0, const DepthEval& e0, bool& irregular, DepthEval& e, PassOut& o)
 {
     bool doubt = irregular;
     eval_near(x, p, f.dt, e, doubt);
     if (!need0) update_near(e0, e, f, h, h_0, Qj_0, o, doubt);
-    if (doubt) {
-        ExactPass a;
-        a.p = p;
-        a.f = f;
-        a.x = x;
-        a.h = h;
-        a.h_0 = h_0;
-        a.Qj_0 = Qj_0;
-        a.e0 = e0;
-        a.need0 = need0;
-        exact_pass(&a);
-        e = a.e;
-        if (!need0) o = a.o;
-        irregular |= !(x == 0.0 || fp_within(x, 60)) || !(fp_within(e.G, 400));
-    }
+    if (doubt) redo_pass(p, f, x, need0, h, h_0, Qj_0, e0, irregular, e, o);
 }
 
 // The stop test's "go on": rerr > rtol && aerr >= atol with rerr = |(h_1 - h) / h|,

@@ -1,0 +1,284 @@
+// A pass of at most four solves by the whole warp, eight lanes each.
+//
+// A narrow river network keeps few lanes of a warp busy, and one FP64 warp
+// instruction costs 64-66 cycles whatever the number of its active lanes
+// (measured, dependent or not, with one to four warps per SM): the time of a
+// run is then the longest chain of passes times the FP64 instructions of a
+// pass. Here the idle lanes take part, so that a pass issues 64 FP64 warp
+// instructions instead of 148:
+//  - the eight lanes of a solve form two quads. Within a quad the lanes evaluate
+//    at the same time what one lane evaluates in turn: the geometry's linear
+//    forms, the reciprocals (wetted perimeter, top width; celerity, conveyance),
+//    the quotients by them, the two powers, the four coefficients;
+//  - the next pass's lower point has this pass's upper evaluation and this
+//    pass's residual, both known before the secant step. Quad A forms the
+//    upper coefficients of this pass while quad B forms the lower ones of the
+//    next with the same instructions (X differs in its numerator and clamp);
+//  - a solve's first pass evaluates h_0 (quad B) and h (quad A) together and so
+//    saves the evaluation-only pass.
+// Each value is formed by the operations of secant_pass (mc_solve.cuh) in their
+// order, so the results are the same bit for bit; products that share an
+// instruction with another lane's FMA are FMAs with -0.0 (exact), sums FMAs
+// with 1.0. A lane's doubt about a rounding sends its solve's pass to exact_pass.
+#pragma once
+
+#include "lane_solver.cuh"
+
+namespace tr {
+
+constexpr int kNarrow = 4;   // solves of a narrow pass
+
+__device__ __forceinline__ double lane_get(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+
+// Constants the compiler does not see through: a select between one of them and
+// a variable would otherwise be turned into two FP64 instructions, one for each
+// side, where the point is to share one.
+struct Opaque {
+    double one, neg_zero, neg_two;
+};
+__device__ __forceinline__ Opaque opaque_constants()
+{
+    Opaque k;
+    asm("mov.b64 %0, 0x3ff0000000000000;" : "=d"(k.one));
+    asm("mov.b64 %0, 0x8000000000000000;" : "=d"(k.neg_zero));
+    asm("mov.b64 %0, 0xc000000000000000;" : "=d"(k.neg_two));
+    return k;
+}
+
+// v or -v, on the integer pipe
+__device__ __forceinline__ double neg_if(bool neg, double v)
+{
+    return __hiloint2double(__double2hiint(v) ^ (neg ? (int)0x80000000 : 0), __double2loint(v));
+}
+
+// One of x^fl(2/3) (odd = false) and x^fl(5/3) (odd = true) as pow23_53_near forms
+// them: the same instructions for both, y or 1 as the outer factor.
+__device__ __forceinline__ double pow_near_one(double x, bool odd, const Opaque& kc, bool& doubt)
+{
+    const int hi = __double2hiint(x);
+    const int u = (hi >> 20) - (1023 - 36);
+    doubt |= (unsigned)u >= 54u;
+    const int k3 = (u * 43) >> 7;
+    const int k = k3 - 12;
+    const double y = __hiloint2double((hi & 0xfffff) | ((1023 + u - 3 * k3) << 20), __double2loint(x));
+    float l;
+    double r;
+    crpow_seed(y, &l, &r);
+    const double c = crpow_widen((float)kFl23Minus23 * ((l + 3.0f * (float)k) * 0.6931472f));
+    const double wh = y * r;
+    const double wl = __fma_rn(y, r, -wh);
+    const double r2 = r * r;
+    const double g = __fma_rn(-wl, r2, __fma_rn(-wh, r2, 1.0));
+    const double s = g * __fma_rn(g, __fma_rn(g, 14.0 / 81.0, 2.0 / 9.0), 1.0 / 3.0);
+    const double m = odd ? y : kc.one;
+    const double w0 = m * wh;
+    const double we = __fma_rn(m, wl, __fma_rn(m, wh, -w0));
+    const double a = __fma_rn(w0, __fma_rn(odd ? kc.neg_two : kc.one, c, s), we);
+    const double z = w0 + a;
+    const double e = a - (z - w0);
+    const int h = __double2hiint(z);
+    doubt |= ((__double2hiint(e) & 0x7fffffff) >= (((h & 0x7ff00000) - (54 << 20)) | 0x000fffc0)) | ((h & 0xfffff) == 0);
+    return __hiloint2double(h + (((odd ? 5 : 2) * k) << 20), __double2loint(z));
+}
+
+// Coefficients and discharge of one quad's evaluation: X from num / G clamped to
+// [lo, 1/2] (lo2 as in clamped_half), C1..C4 on the quad's four lanes, their sum with the flows; beside X's
+// quotient (lanes 1, 2) lanes 0 and 3 form the Manning discharge.
+struct QuadFlow {
+    double q, C4, Qmn;   // on all lanes of the quad
+};
+
+__device__ __forceinline__ QuadFlow quad_flow(int r, int quad, const PassFlow& f, double num, int lo2, double Km, double G,
+                                              double yG, double it, double AAC, double r23, double sq_s0, const Opaque& kc, bool& doubt)
+{
+    const bool xl = r == 1 || r == 2;
+    const bool valid = dbits(yG) != 0;
+    const double q0 = (xl ? num : it) * (xl ? yG : AAC);
+    const double rr = __fma_rn(xl ? -G : q0, xl ? q0 : r23, xl ? num : kc.neg_zero);
+    const double qq = __fma_rn(rr, xl ? yG : sq_s0, xl ? q0 : kc.neg_zero);
+    doubt |= xl & valid & quot_doubt(G, q0, rr);
+    double X = clamped_half(1.0 - qq, lo2);
+    if (!valid) X = 0.5;
+    X = lane_get(X, quad | 1);
+    QuadFlow o;
+    o.Qmn = lane_get(qq, quad);
+    const double om = 1.0 - X;
+    const double t = Km * (r < 2 ? X : om);   // Km X on lanes 0, 1; Km (1 - X) on 2, 3
+    // numerators Km X + dt/2, dt/2 - Km X, Km (1 - X) - dt/2; lane 3: the denominator
+    const double n = neg_if(r == 1, t) + neg_if(r == 2, f.dt2);
+    const NearRcp rd = near_rcp(lane_get(n, quad | 3));
+    const double c = near_quot(r == 3 ? f.qldt : n, rd, doubt);
+    const double m = c * (r == 0 ? f.qup : r == 1 ? f.quc : r == 2 ? f.qdp : kc.one);
+    const double S3 = lane_get(m, quad) + lane_get(m, quad | 1) + lane_get(m, quad | 2);
+    double C4 = lane_get(m, quad | 3);
+    if (__any_sync(0xffffffffu, __double2hiint(C4) < 0))
+        if (lo2 && fp_lt0(C4) && fp_abs_gt(C4, S3)) C4 = -S3;
+    o.C4 = C4;
+    o.q = S3 + C4;
+    return o;
+}
+
+// The pass for the lanes of smask (at most kNarrow, none irregular). The whole
+// warp calls it; `warp_seg` is buffer 0 of the warp's lane 0. A lane of smask gets
+// o and its L.e0 (and what the next narrow pass starts from) as lane_eval leaves
+// them; returns whether it iterated (not after an exact evaluation at h_0 alone).
+__device__ __forceinline__ bool narrow_pass(Lane& L, unsigned smask, const RunDev& run, double2* warp_seg, PassOut& o)
+{
+    const int lane = threadIdx.x & 31;
+    const int r = lane & 3, quad = lane & ~3;
+    const bool B = lane & 4;
+    // this octet's solve: the (lane / 8)-th lane of smask (the first again when
+    // there are fewer)
+    unsigned m = smask;
+    const int j = lane >> 3;
+    if (j > 0) m &= m - 1;
+    if (j > 1) m &= m - 1;
+    if (j > 2) m &= m - 1;
+    const int home = __ffs(m ? m : smask) - 1;
+    const int flags = __shfl_sync(0xffffffffu, (L.i & 1) | (L.need0 << 1) | ((L.ahead ? 1 : 0) << 2), home);
+    const bool need0 = flags & 2, pre = !(flags & 4);
+    const double h = lane_get(L.h, home), h_0 = lane_get(L.h_0, home);
+    const PassFlow f = {lane_get(L.qup, home), lane_get(L.quc, home), lane_get(L.qdp, home), lane_get(L.qldt, home), run.dt,
+                        run.dt_half};
+    const Opaque kc = opaque_constants();
+    const SegP p = staged_seg(warp_seg + home + (flags & 1) * kSegBufStride);
+
+    // ---- geometry ----
+    const double x = (B && need0) ? h_0 : h;
+    const bool wet = (__double2hiint(x) | __double2loint(x)) != 0;
+    bool unsure = !depth_regular(x);
+    const bool over = dbits(x) > dbits(p.bfd);
+    const double below = over ? p.bfd : x;
+    // depth above the bank; lane 3: h_0 - h for the secant step
+    const double diff = (r == 3 ? h_0 : x) - (r == 3 ? h : p.bfd);
+    // lane 0: WP, WP n; lane 1: A; lanes 2, 3: bw + 2 z x and its product with s0
+    double s1 = p.bw + (r < 2 ? below : p.z2) * (r == 0 ? p.sq2 : r == 1 ? p.z : x);
+    double w = s1 * (r == 0 ? p.n_ch : r == 1 ? below : p.s0);
+    if (__any_sync(0xffffffffu, over)) {
+        const double t1 = __fma_rn(r == 0 ? 2.0 : p.twcc, r >= 2 ? p.s0 : diff, r == 0 ? p.twcc : kc.neg_zero);
+        const double t2 = (r == 0 ? s1 : w) + t1;
+        const double t3 = w + t1 * p.ncc;
+        if (over) {
+            if (r == 0) s1 = t2, w = t3;
+            else w = r == 1 ? t2 : t1;
+        }
+    }
+    const double P = lane_get(s1, quad), WPn = lane_get(w, quad);
+    // lane 1: R; lane 2: 2 sqrt(1+z^2) / (bw + 2 z x); lanes 0, 3: (WP n) / P
+    const double q1 = near_quot(r == 2 ? p.sq2 : r == 1 ? w : WPn, near_rcp(r == 2 ? s1 : P), unsure);
+    const double z = pow_near_one(lane_get(q1, quad | 1), r & 1, kc, unsure);
+    const double r23 = lane_get(z, quad);
+    const double sqt = lane_get(q1, quad | 2);
+    const double v = z * ((r & 1) ? 2.0 / 3.0 : 5.0 / 3.0) * ((r & 1) ? sqt : kc.one);
+    const double u = __shfl_xor_sync(0xffffffffu, v, 1);
+    const double Ck = p.ck_fac * (((r & 1) ? u : v) - ((r & 1) ? v : u));
+    const bool moves = wet && __double2hiint(Ck) > 0;
+    // lane 1: dx / Ck; lanes 0, 3: 1 / ((WP n) / P); lane 2: G = 2 tw s0 Ck dx, 1 / G
+    double G, yG, Km, it;
+    {
+        const bool g2 = r == 2;
+        const double b = r == 1 ? Ck : q1;
+        const double y0 = rcp_seed(b);
+        const double e1 = __fma_rn(g2 ? w : -b, g2 ? Ck : y0, g2 ? kc.neg_zero : kc.one);
+        const double e2 = __fma_rn(e1, g2 ? p.dx : e1, g2 ? kc.neg_zero : e1);
+        const double y = __fma_rn(y0, e2, y0);
+        G = __hiloint2double(__double2hiint(e2) + (1 << 20), __double2loint(e2));
+        const double yg0 = rcp_seed(G);
+        const double q0 = __fma_rn(g2 ? -G : (r == 1 ? p.dx : kc.one), g2 ? yg0 : y, g2 ? kc.one : kc.neg_zero);
+        const double rr = __fma_rn(g2 ? q0 : -b, q0, g2 ? q0 : (r == 1 ? p.dx : kc.one));
+        const double qq = __fma_rn(g2 ? yg0 : rr, g2 ? rr : y, g2 ? yg0 : q0);
+        unsure |= !g2 & (moves | (r != 1)) & quot_doubt(b, q0, rr);
+        it = qq;
+        // (shuffles outside the selects: the quads' moves differ)
+        G = lane_get(G, quad | 2);
+        yG = lane_get(qq, quad | 2);
+        Km = fp_max_pos(run.dt, lane_get(qq, quad | 1));
+        if (!moves) {
+            G = 1.0;
+            yG = 0.0;
+            Km = run.dt;
+        }
+    }
+    double AAC = lane_get(w, quad | 1);
+    bool doubt = wet & unsure;
+
+    // ---- the lower point of this pass, unless the last narrow pass formed it ----
+    double q0 = lane_get(L.qmc0_n, home), Qj_0 = lane_get(L.Qj0_n, home);
+    double r23u = r23, itu = it;
+    if (__any_sync(0xffffffffu, pre)) {
+        const double eK = lane_get(L.e0.Km, home), eG = lane_get(L.e0.G, home), ey = lane_get(L.e0.yG, home);
+        const double eQ = lane_get(L.e0.Qmn, home), Qp = lane_get(L.Qj_0, home);
+        bool d = false;
+        const QuadFlow a = quad_flow(r, quad, f, Qp, 0, need0 ? Km : eK, need0 ? G : eG, need0 ? yG : ey, it, AAC, r23,
+                                     p.sq_s0, kc, d);
+        const double Qmn = need0 ? (wet ? a.Qmn : 0.0) : eQ;
+        const double res = lane_get(a.q - Qmn, lane | 4), qa = lane_get(a.q, lane | 4);
+        if (pre) {
+            q0 = qa;
+            Qj_0 = res;
+            doubt |= B & d;
+        }
+        // quad B goes on with the upper evaluation
+        Km = lane_get(Km, lane & ~4);
+        G = lane_get(G, lane & ~4);
+        yG = lane_get(yG, lane & ~4);
+        r23u = lane_get(r23, lane & ~4);
+        itu = lane_get(it, lane & ~4);
+        AAC = lane_get(AAC, lane & ~4);
+    }
+
+    // ---- quad A: upper coefficients of this pass; quad B: lower ones of the next ----
+    const QuadFlow a = quad_flow(r, quad, f, B ? Qj_0 : q0, B ? 0 : 0x3fe00000, Km, G, yG, itu, AAC, r23u, p.sq_s0, kc, doubt);
+    const bool flowing = (__double2hiint(h) | __double2loint(h)) != 0;
+    const double Qmn = flowing ? a.Qmn : 0.0;
+    const double res = a.q - Qmn;
+    doubt |= !B & fp_lt0(a.q);   // the negative-flow fallbacks (troute_mc_final.cu:125-130)
+
+    // ---- secant step, on every lane of the octet ----
+    const double Qj = lane_get(res, lane & ~7);
+    const double hd = lane_get(diff, quad | 3);
+    // lane 0: Qj (h_0 - h); lane 1: Qj_0 - Qj
+    const double n = __fma_rn((r & 1) ? kc.one : Qj, neg_if(r & 1, (r & 1) ? Qj : hd), (r & 1) ? Qj_0 : kc.neg_zero);
+    const double dQ = lane_get(n, quad | 1), num = lane_get(n, quad);
+    const bool slope = !fp_eq0(dQ);
+    bool d2 = false;
+    const double q2 = near_quot(num, near_rcp(dQ), d2);
+    double h_1 = slope ? h - q2 : h;
+    if (fp_lt0(h_1)) h_1 = h;
+    doubt |= slope & (d2 | !numerator_regular(num));
+
+    // ---- back to the solve's own lane ----
+    const unsigned bad = __ballot_sync(0xffffffffu, doubt);
+    const int src = (8 * __popc(smask & ((1u << lane) - 1u))) & 31;
+    DepthEval e;
+    e.Km = lane_get(Km, src);
+    e.G = lane_get(G, src);
+    e.yG = lane_get(yG, src);
+    e.Qmn = lane_get(Qmn, src);
+    PassOut po;
+    po.Qj_0 = lane_get(Qj_0, src);
+    po.qdc = lane_get(a.q, src);
+    po.h_1 = lane_get(h_1, src);
+    const double qn = lane_get(a.q, src + 4), rn = lane_get(res, src + 4);
+    if (!((smask >> lane) & 1u)) return false;
+    if ((bad >> src) & 0xffu) {
+        const SegP pl = staged_seg(warp_seg + lane + (L.i & 1) * kSegBufStride);
+        const PassFlow fl = {L.qup, L.quc, L.qdp, L.qldt, run.dt, run.dt_half};
+        redo_pass(pl, fl, L.need0 ? L.h_0 : L.h, L.need0, L.h, L.h_0, L.Qj_0, L.e0, L.irregular, e, po);
+        L.e0 = e;
+        L.ahead = false;
+        const bool iterated = !L.need0;
+        L.need0 = 0;
+        o = po;
+        return iterated;
+    }
+    L.e0 = e;
+    L.need0 = 0;
+    L.ahead = true;
+    L.qmc0_n = qn;
+    L.Qj0_n = rn;
+    o = po;
+    return true;
+}
+
+}  // namespace tr

@@ -895,10 +895,12 @@ static int enqueue_chunk(troute_handle* H, const double* qlat_dev, int n_ts, con
         df.rq_head = H->rq_ctr.p;
         df.rq_tail = H->rq_ctr.p + 1;
         df.n_done = H->rq_ctr.p + 2;
+        df.n_avail = reinterpret_cast<int*>(H->rq_ctr.p + 3);
         df.rh = H->df_rh.p;
         df.heads = H->df_heads.p;
         df.n_heads = H->n_heads;
         df.continue_items = H->cfg.schedule_flags & 1;
+        df.n_primary = H->n_sms;
         df.n_items = (unsigned long long)H->R_real * (unsigned long long)n_ts;
         if (run.warm) {
             // the launch's learned starting depths: one tcgen05 GEMM over every
@@ -994,7 +996,7 @@ static int prepare_run(troute_handle* H, int n_ts, RunPlan* P)
         const size_t R = (size_t)std::max(1, H->R_int);
         const size_t T = (size_t)P->chunk;
         if ((rc = H->df_cnt.alloc(T * R)) || (rc = H->df_rh.alloc((T + 1) * R)) ||
-            (rc = H->df_rq.alloc(std::max<size_t>(1, (size_t)H->R_real * T))) || (rc = H->rq_ctr.alloc(3)))
+            (rc = H->df_rq.alloc(std::max<size_t>(1, (size_t)H->R_real * T))) || (rc = H->rq_ctr.alloc(4)))
             return rc;
     }
     return TROUTE_OK;

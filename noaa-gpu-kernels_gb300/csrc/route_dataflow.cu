@@ -18,27 +18,31 @@
 //               outflow of the step before the run (from the 4-slot ring of
 //               the handle's state); a whole run is kept, so upstream reaches
 //               never wait for downstream ones to consume a value.
-// The lane that makes an item ready continues with it itself when it has no
-// other work (the downstream item when two became ready), so busy lanes stay
-// in their warps and the queue carries only the rest. A warp claims only
+// In a warp of few items (and with continue_items in every warp) the lane that
+// makes an item ready continues with it itself (the downstream item when two
+// became ready), so the longest chain does not pass through the queue. A warp claims only
 // slots that are already written (or that a racing warp is about to see
 // written); the run ends when the count of completed items reaches n_items.
 // The head sums at a reach use the upstream order of the reference
 // (wavefront_mc.cu:525-531), and the solve is lane_solver.cuh's, i.e. the
 // reference's arithmetic.
-#include "lane_solver.cuh"
+#include "narrow_pass.cuh"
 
 namespace tr {
 
 namespace {
 constexpr unsigned kFullMask = 0xffffffffu;
 constexpr int L_FETCH = L_WAIT;  // claimed a queue slot, waiting for it to be written
-constexpr unsigned long long kWakeItems = 16;  // queued items that wake an idle warp
-constexpr long long kWakeCycles = 8000;        // ... or this long unclaimed (~4 us)
+#ifndef TROUTE_WIDE_ITEMS
+#define TROUTE_WIDE_ITEMS 1216
+#endif
+// Queued items from which on warps fill all their lanes instead of kNarrow.
+constexpr int kWideItems = TROUTE_WIDE_ITEMS;
 #ifndef TROUTE_SLEEP_MAX_NS
 #define TROUTE_SLEEP_MAX_NS 3200
 #endif
 constexpr unsigned kSleepMinNs = 200, kSleepMaxNs = TROUTE_SLEEP_MAX_NS;  // idle-warp polling back-off
+constexpr unsigned kPrimaryMaxNs = 800;
 
 __device__ __forceinline__ unsigned lanemask_lt_df()
 {
@@ -131,6 +135,7 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
     __shared__ unsigned int hist_s[16];
     __shared__ double2 seg_sm[kSegSmemPerThread * kDfThreads];
     double2* const seg_slot = seg_slot_of(seg_sm);
+    double2* const warp_seg = seg_slot - (threadIdx.x & 31);
     if (threadIdx.x < 16) hist_s[threadIdx.x] = 0;
     __syncthreads();
     LocalStats ls = {0, 0, 0, 0, 0, 0};
@@ -141,49 +146,46 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
     const int R = net.n_reach_int;
     bool failed = false;
     unsigned long long slot = 0;
-    long long queued_since = -1;  // lane 0: when this idle warp first saw unclaimed items
+    const bool primary = blockIdx.x < (unsigned)df.n_primary;
     Lane L;
     L.mode = L_IDLE;
     unsigned long long n_pass = 0, n_busy = 0, n_wait = 0, n_idle = 0, n_solve = 0;
     unsigned idle_ns = kSleepMinNs;  // warp-uniform
     unsigned long long idle_seen = ~0ull;  // warp-uniform: n_done when this warp last saw progress
     long long idle_t0 = clock64();
+    // lane 0: unclaimed items and error flag, read before each pass and used after
+    // it, so that a solving warp does not wait for them
+    int seen_avail = 0, seen_err = 0;
 
     while (true) {
         // ---- idle lanes claim queue slots (one atomic per warp) ----
-        // A warp claims only as many slots as there are queued items it could
-        // take (tail - head), so the ready work lands on few, full warps instead
-        // of one lane in each of many warps (a warp pays for every FP64
-        // instruction whatever the number of its busy lanes). Two warps can
-        // race past the tail; their extra lanes wait for the next items.
+        // A warp claims only as many slots as there are queued items that no
+        // other warp has claimed (n_avail, taken down before the slots are;
+        // claims that outran it would tie later items to whichever lanes raced,
+        // however full their warps). While little is queued, the
+        // primary warps -- one block per SM, one warp per scheduler -- and warps
+        // that have work hold at most kNarrow items, which they solve by
+        // narrow passes; once kWideItems are queued (more than the primary
+        // warps can take up) every warp fills all its lanes, so that the work
+        // lands on full warps: a warp pays for every FP64 instruction whatever
+        // the number of its busy lanes.
         const unsigned idle = __ballot_sync(kFullMask, L.mode == L_IDLE);
         if (idle) {
-            // a warp with busy lanes tops itself up with whatever is queued; a
-            // warp with none waits until enough is queued to fill a good part
-            // of it, or until queued items have not been taken for a while
-            const bool has_busy = idle != kFullMask;
             unsigned n = 0;
             unsigned long long base = 0;
             int err = 0;
             if (lane == 0) {
-                const unsigned long long tail = ld_volatile_ull(df.rq_tail);
-                const unsigned long long head = ld_volatile_ull(df.rq_head);
-                err = ld_volatile_int(&run.stats->error);
-                if (tail > head) {
-                    const unsigned long long avail = tail - head;
-                    bool take = has_busy || avail >= kWakeItems;
-                    if (!take) {
-                        const long long now = clock64();
-                        if (queued_since < 0) queued_since = now;
-                        take = now - queued_since > kWakeCycles;
+                err = seen_err;
+                if (seen_avail > 0) {
+                    const int held = 32 - __popc(idle);
+                    const int room = seen_avail >= kWideItems ? 32 - held : primary ? kNarrow - held : 0;
+                    const int want = min(room, seen_avail);
+                    if (want > 0) {
+                        const int had = atomicSub(df.n_avail, want);
+                        n = max(0, min(want, had));
+                        if ((int)n < want) atomicAdd(df.n_avail, want - (int)n);
+                        if (n) base = atomicAdd(df.rq_head, (unsigned long long)n);
                     }
-                    if (take) {
-                        queued_since = -1;
-                        n = (unsigned)min((unsigned long long)__popc(idle), avail);
-                        base = atomicAdd(df.rq_head, (unsigned long long)n);
-                    }
-                } else {
-                    queued_since = -1;
                 }
             }
             n = __shfl_sync(kFullMask, n, 0);
@@ -192,8 +194,6 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
             if (err) break;
             if (n && L.mode == L_IDLE) {
                 const unsigned rank = __popc(idle & lt);
-                // racing warps can push the head past the end of the queue;
-                // such slots do not exist and are never read
                 if (rank < n && base + rank < df.n_items) {
                     slot = base + rank;
                     L.mode = L_FETCH;
@@ -264,22 +264,34 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
         if (L.mode == L_START) start_item(L, L.ri, L.tau, t_base, net, run, df, ls, hist_s, seg_slot);
         if (L.mode == L_BEGIN) L.mode = begin_segment(L, net, run, ls, hist_s, seg_slot) ? L_SOLVE : L_DONE;
 
-        // ---- one depth evaluation per solving lane ----
-        if (__any_sync(kFullMask, L.mode >= L_SOLVE)) {
+        // ---- one pass of the solving lanes ----
+        const unsigned smask = __ballot_sync(kFullMask, L.mode == L_SOLVE);
+        if (smask && lane == 0) {
+            seen_avail = ld_volatile_int(df.n_avail);
+            seen_err = ld_volatile_int(&run.stats->error);
+        }
+        if (smask) {
             n_solve++;
-            lane_pass(L, net, run, ls, hist_s, seg_slot);
+            PassOut o;
+            bool iterated = false;
+            if (__popc(smask) <= kNarrow && !__any_sync(kFullMask, L.mode == L_SOLVE && L.irregular))
+                iterated = narrow_pass(L, smask, run, warp_seg, o);
+            else if (L.mode == L_SOLVE)
+                iterated = lane_eval(L, run, seg_slot, o);
+            if (iterated) lane_finish(L, o, net, run, ls, hist_s, seg_slot);
         }
 
         // ---- completed reaches: publish, count dependencies, queue ready items ----
         int npush = 0;
         int2 push0 = make_int2(-1, -1), push1 = make_int2(-1, -1);
         const unsigned dmask = __ballot_sync(kFullMask, L.mode == L_DONE);
+        const bool narrow = primary && __popc(__ballot_sync(kFullMask, L.mode != L_IDLE)) <= kNarrow;
         if (dmask && lane == 0) atomicAdd(df.n_done, (unsigned long long)__popc(dmask));
         if (L.mode == L_DONE) {
             __stcg(df.rh + (size_t)(L.tau + 1) * R + L.ri, L.q_last);
             __stcg(net.ring + (size_t)(L.g % kRing) * R + L.ri, L.q_last);
+            net.done[L.ri] = L.g + 1;   // read by later launches only
             __threadfence();
-            st_release(net.done + L.ri, L.g + 1);
             const int nup = L.ue - L.ub;
             if (L.tau + 1 < T) {
                 // own next step: needs its upstream reaches too
@@ -296,7 +308,7 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
                 }
             }
             L.mode = L_IDLE;
-            if (npush && df.continue_items) {
+            if (npush && (df.continue_items || narrow)) {
                 // continue with one newly ready item here (the downstream one when
                 // there are two: it lies toward the outlet); queue the other
                 __threadfence();  // other dependencies' writes, seen through the counters
@@ -310,18 +322,17 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
             }
         }
         // warp-aggregated append to the ready queue
-        unsigned total = npush;
-        for (int off = 16; off > 0; off >>= 1) total += __shfl_xor_sync(kFullMask, total, off);
-        if (total) {
-            unsigned incl = npush;
-            for (int off = 1; off < 32; off <<= 1) {
-                const unsigned v = __shfl_up_sync(kFullMask, incl, off);
-                if (lane >= off) incl += v;
-            }
+        const unsigned push_any = __ballot_sync(kFullMask, npush >= 1), push_two = __ballot_sync(kFullMask, npush == 2);
+        if (push_any) {
+            const unsigned total = __popc(push_any) + __popc(push_two);
+            const unsigned before = __popc(push_any & lt) + __popc(push_two & lt);
             unsigned long long base = 0;
-            if (lane == 31) base = atomicAdd(df.rq_tail, (unsigned long long)total);
+            if (lane == 31) {
+                base = atomicAdd(df.rq_tail, (unsigned long long)total);
+                atomicAdd(df.n_avail, (int)total);   // a claimer waits for a slot that is about to be written
+            }
             base = __shfl_sync(kFullMask, base, 31);
-            const unsigned long long pos = base + (incl - npush);
+            const unsigned long long pos = base + before;
             if (npush) __threadfence();  // every dependency's writes before the item is visible
             if (npush && pos + npush > df.n_items) {
                 // more items than the run has: an accounting error, never write past the queue
@@ -348,7 +359,12 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
                 __nanosleep(kSleepMinNs);
             } else {
                 __nanosleep(idle_ns);
-                idle_ns = idle_ns < kSleepMaxNs ? 2 * idle_ns : kSleepMaxNs;
+                const unsigned most = primary ? kPrimaryMaxNs : kSleepMaxNs;
+                idle_ns = idle_ns < most ? 2 * idle_ns : most;
+            }
+            if (lane == 0) {
+                seen_avail = ld_volatile_int(df.n_avail);
+                seen_err = ld_volatile_int(&run.stats->error);
             }
         } else {
             idle_ns = kSleepMinNs;
@@ -377,6 +393,7 @@ __global__ void dataflow_init_kernel(NetDev net, RunDev run, DataflowDev df)
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *df.rq_head = 0;
         *df.rq_tail = (unsigned long long)df.n_heads;
+        *df.n_avail = df.n_heads;
         *df.n_done = 0;
     }
 }

@@ -147,10 +147,12 @@ struct DataflowDev {
     unsigned long long* rq_head;    // claimed slots
     unsigned long long* rq_tail;    // written slots
     unsigned long long* n_done;     // completed items
+    int* n_avail;                   // queued items no warp has claimed (down to minus the claims in flight)
     double* rh;                     // [n_ts + 1][n_reach_int] reach outflow per step
     const int2* heads;              // (headwater reach, 0) items, ready at the start
     int n_heads;
-    int continue_items;             // 1: a lane continues with an item it made ready
+    int continue_items;             // 1: a lane continues with an item it made ready (0: in narrow warps only)
+    int n_primary;                  // blocks whose warps take queued items as they come (one per SM)
     unsigned long long n_items;     // real reaches x n_ts
 };
 

@@ -104,8 +104,8 @@ def test_device_quotients_near_midpoints():
 @pytest.mark.parametrize("tol", [O.REF_TOL, (1e-8, 1e-10, 100, 5)], ids=["ref_tol", "rtol_1e-8"])
 def test_solves_outside_the_short_ranges(tol):
     """Single-segment and longer reaches with flows of 1e-60, 1e-40 and negative
-    lateral inflow, channels of 1e-15 and 1e15 m, a dry bed, depths of 1e-40, 1e-5
-    and 1e20 m, roughness of 1e13, twcc = 0: bit-identical to the oracle."""
+    lateral inflow, channels of 1e-15 and 1e15 m, a dry bed, depths of 1e-40, 1e-5,
+    1e20 and 1e150 m, roughness of 1e13, twcc = 0: bit-identical to the oracle."""
     rng = np.random.default_rng(7)
     n = 1200
     p = synth.make_params(91, n)
@@ -119,7 +119,7 @@ def test_solves_outside_the_short_ranges(tol):
         ql[s], qu[s], qd[s] = v, v, v
     ql[600:640] = -1e-3
     ql[640:660] = -0.0
-    for k, v in enumerate((0.0, 1e-40, 1e-5, 1e20)):
+    for k, v in enumerate((0.0, 1e-40, 1e-5, 1e20, 1e150)):
         dp[700 + 40 * k:740 + 40 * k] = v
     p["tw"][900:940] = p["bw"][900:940]
     p["tw"][940:960] = 0.5 * p["bw"][940:960]
