@@ -30,6 +30,13 @@ __device__ __forceinline__ bool fp_lt0(double x)
     return b > 0x8000000000000000ull && b <= 0xfff0000000000000ull;
 }
 
+// x <= 0
+__device__ __forceinline__ bool fp_le0(double x)
+{
+    const long long b = dbits(x);
+    return b <= 0 && (unsigned long long)b <= 0xfff0000000000000ull;
+}
+
 // x == 0 (either sign)
 __device__ __forceinline__ bool fp_eq0(double x) { return ((unsigned long long)dbits(x) << 1) == 0; }
 

@@ -31,17 +31,18 @@ enum : int { L_IDLE = 0, L_WAIT = 1, L_SOLVE = 2, L_BEGIN = 3, L_DONE = 4, L_STA
 // solve, read by every pass. (Re-reading them from global memory every pass
 // misses L2 once a network's parameters outgrow it -- c1's are 260 MB -- and
 // costs a DRAM round trip per pass.) Each lane has two buffers: while segment
-// i is solved, segment i + 1's parameters, inflow column and scale and (warm
-// start) learned starting depth are copied into the other buffer by cp.async,
-// and its discharge and depth are prefetched into L2 -- all static during the
-// launch or final since the reach's previous step completed -- so the next
-// solve starts after one round trip (the inflow) instead of a chain of them.
-// Buffer of segment i: i & 1. A buffer holds kParamPlanes parameter double2
-// and one {inflow scale, inflow column | learned depth} double2.
+// i is solved, segment i + 1's parameters, inflow column and scale, discharge,
+// depth and (warm start) learned starting depth are copied into the other one by
+// cp.async, and one pass later, with the column at hand, its inflow -- all static
+// during the launch or final since the reach's previous step completed -- so the
+// next solve starts without a global load. Buffer of segment i: i & 1. Its planes,
+// in double2: parameters; {inflow scale, inflow column | flags}; the aligned pairs
+// of discharge and depth that hold the slot's; {inflow, learned depth}.
 // Layout [warp][buffer][plane][lane]: a warp's reads of one plane are 512
 // contiguous bytes, free of bank conflicts, whatever the block size.
 constexpr int kSegSmemStride = 32;
-constexpr int kSegBufPlanes = kParamPlanes + 1;
+constexpr int kTailPlane = kParamPlanes, kQPlane = kParamPlanes + 1, kDPlane = kParamPlanes + 2, kInPlane = kParamPlanes + 3;
+constexpr int kSegBufPlanes = kParamPlanes + 4;
 constexpr int kSegBufStride = kSegBufPlanes * kSegSmemStride;   // double2 from buffer 0 to 1
 // double2 of a block's staging array per thread
 constexpr int kSegSmemPerThread = 2 * kSegBufPlanes;
@@ -73,26 +74,27 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// Starts the copies of tile slot s's record (and learned depth for step tau)
-// into buffer buf, and the L2 prefetch of its discharge and depth. Only data
-// that no thread writes during the launch goes through the non-coherent
-// cp.async path (the records; the prediction plane, written before the
-// launch); the mutable discharge and depth are read later with ld.cg.
+// Starts the copies of tile slot s's record, discharge and depth (and learned
+// depth for step tau) into buffer buf. The discharge and depth, which other steps
+// of the launch write, are copied past L1 (cp.async.cg, whose 16 bytes are the
+// pair around the slot: the neighbour's value may be in flux and is not used).
 __device__ __forceinline__ void stage_seg_async(const NetDev& net, const RunDev& run, int tau, long long s,
                                                 double2* buf)
 {
     const SegRec* r = net.seg + s;
 #pragma unroll
     for (int k = 0; k < kParamPlanes; ++k) cp_async16(buf + k * kSegSmemStride, r->p + k);
-    double2* t = buf + kParamPlanes * kSegSmemStride;
-    cp_async8(&t->x, &r->qscale);
-    int* w = reinterpret_cast<int*>(&t->y);
-    cp_async4(w, &r->qcol);
-    if (run.warm) cp_async4(w + 1, run.start_pred + (size_t)tau * (size_t)net.n_seg_int + s);
-    prefetch_l2(net.q + s);
-    prefetch_l2(net.d + s);
+    cp_async16(buf + kTailPlane * kSegSmemStride, &r->qscale);
+    cp_async16(buf + kQPlane * kSegSmemStride, net.q + (s & ~1ll));
+    cp_async16(buf + kDPlane * kSegSmemStride, net.d + (s & ~1ll));
+    if (run.warm) cp_async4(&buf[kInPlane * kSegSmemStride].y, run.start_pred + (size_t)tau * (size_t)net.n_seg_int + s);
+}
+
+// Starts the copy of the inflow of column col at step tau into buffer buf.
+__device__ __forceinline__ void stage_inflow_async(const RunDev& run, int tau, int col, double2* buf)
+{
+    cp_async8(&buf[kInPlane * kSegSmemStride].x, run.qlat + (size_t)tau * (size_t)run.qlat_ld + col);
 }
 
 __device__ __forceinline__ SegP staged_seg(const double2* slot)
@@ -108,10 +110,16 @@ __device__ __forceinline__ SegP staged_seg(const double2* slot)
 // depth (read from the launch's prediction plane when the solve begins).
 enum : int { W_PLAIN = 0, W_ACTIVE = 2 };
 
+// Inflow of the segment to begin next: its column not yet known to have arrived,
+// or the copy under way (or done).
+enum : int { kInflowLater = 0, kInflowStaged = 1 };
+
 // Everything a lane carries for one (reach, step) and the segment it solves.
 struct Lane {
     int mode;
     int ri, tau, g, ns, i, ub, ue, dn;
+    int n_up, dn_n_up;     // upstream reaches of this reach and of the one downstream
+    int inflow;            // of the next segment (of this one when it begins): kInflow*
     long long base;        // tile slot of segment 0
     long long wait_t0;
     unsigned long long wait_tail;  // queue tail seen when the current wait budget began
@@ -128,11 +136,11 @@ struct Lane {
     double qmc0_n, Qj0_n;
 };
 
-// The plain starting bracket from the previous depth (troute_mc_final.cu:193).
-__device__ __forceinline__ void plain_bracket(Lane& L, const Tol& tol)
+// A solve's first attempt from the bracket [h_0, h].
+__device__ __forceinline__ void restart_bracket(Lane& L, const Tol& tol, double h, double h_0)
 {
-    L.h = L.dpp * 1.33 + kMinDepth;
-    L.h_0 = L.dpp * 0.67;
+    L.h = h;
+    L.h_0 = h_0;
     L.Qj_0 = 0.0;
     L.qdc = 0.0;
     L.maxiter = tol.maxiter;
@@ -142,31 +150,48 @@ __device__ __forceinline__ void plain_bracket(Lane& L, const Tol& tol)
     L.ahead = false;
 }
 
-// Starts segment L.i of the lane's reach; consecutive segments that exit early
-// (invalid parameters or no flow at all, troute_mc_final.cu:54-63) are stored
-// right away. Returns true when a secant solve is pending, false when the reach
-// is complete.
+// The plain starting bracket from the previous depth (troute_mc_final.cu:193).
+__device__ __forceinline__ void plain_bracket(Lane& L, const Tol& tol)
+{
+    restart_bracket(L, tol, L.dpp * 1.33 + kMinDepth, L.dpp * 0.67);
+}
+
+// Starts the copy of the next segment's inflow once its column has arrived (a
+// pass after the segment's other values were asked for).
+__device__ __forceinline__ void stage_next_inflow(Lane& L, const RunDev& run, double2* slot)
+{
+    if (L.inflow == kInflowLater && L.i + 1 < L.ns) {
+        cp_async_wait_all();
+        double2* const buf = seg_buf(slot, L.i + 1);
+        stage_inflow_async(run, L.tau, __double2loint(buf[kTailPlane * kSegSmemStride].y), buf);
+        L.inflow = kInflowStaged;
+    }
+}
+
+// Starts segment L.i of the lane's reach, staged by the caller (segment 0) or while
+// the previous one was solved; consecutive segments that exit early (invalid
+// parameters or no flow at all, troute_mc_final.cu:54-63) are stored right away.
+// Returns true when a secant solve is pending, false when the reach is complete.
 __device__ __forceinline__ bool begin_segment(Lane& L, const NetDev& net, const RunDev& run,
                                               LocalStats& ls, unsigned int* hist_s, double2* slot)
 {
-    const double* qlat_row = run.qlat + (size_t)L.tau * (size_t)run.qlat_ld;
     while (L.i < L.ns) {
         L.s = L.base + (long long)L.i * kLanes;
         double2* const buf = seg_buf(slot, L.i);
-        // segment 0 of an item is staged now; every later segment was staged
-        // while the previous one was solved
-        if (L.i == 0) stage_seg_async(net, run, L.tau, L.s, buf);
         cp_async_wait_all();
         if (L.i + 1 < L.ns) stage_seg_async(net, run, L.tau, L.s + kLanes, seg_buf(slot, L.i + 1));
-        L.qdp = __ldcg(net.q + L.s);
-        const double dpp = __ldcg(net.d + L.s);
-        const double2 tail = buf[kParamPlanes * kSegSmemStride];
-        const long long tw = __double_as_longlong(tail.y);
-        const double ql = __ldg(qlat_row + (int)(unsigned)(tw & 0xffffffffll)) * tail.x;   // column: the low word
-        const SegP p = staged_seg(buf);
+        const double2 tail = buf[kTailPlane * kSegSmemStride], in = buf[kInPlane * kSegSmemStride];
+        const double2 q2 = buf[kQPlane * kSegSmemStride], d2 = buf[kDPlane * kSegSmemStride];
+        L.qdp = (L.s & 1) ? q2.y : q2.x;
+        const double dpp = (L.s & 1) ? d2.y : d2.x;
+        double ql = L.inflow == kInflowStaged
+                        ? in.x
+                        : __ldg(run.qlat + (size_t)L.tau * (size_t)run.qlat_ld + __double2loint(tail.y));
+        if (dbits(tail.x) != 0x3ff0000000000000ll) ql = ql * tail.x;   // a scale of 1 changes nothing
+        L.inflow = kInflowLater;
         L.qup = (L.i == 0) ? L.qup_head : L.q_up_old;
         L.quc = (L.i == 0) ? L.quc_head : L.q_up_new;
-        if (exits_early(p, ql, L.qup, L.quc, L.qdp)) {
+        if (exits_early(staged_seg(buf), ql, L.qup, L.quc, L.qdp)) {
             __stcg(net.q + L.s, 0.0);
             __stcg(net.d + L.s, 0.0);
             __stcg(net.v + L.s, 0.0);
@@ -183,27 +208,25 @@ __device__ __forceinline__ bool begin_segment(Lane& L, const NetDev& net, const 
             continue;
         }
         L.qldt = ql * run.dt;
-        L.irregular = !(seg_regular(p, run.dt) && flow_regular(L.qup) && flow_regular(L.quc) && flow_regular(L.qdp) &&
-                        flow_regular(L.qldt));
-        L.dpp = fmax(dpp, 0.0);
-        plain_bracket(L, run.tol);
+        L.irregular = !((__double2hiint(tail.y) & 1) && run.dt_regular && flow_regular(L.qup) && flow_regular(L.quc) &&
+                        flow_regular(L.qdp) && flow_regular(L.qldt));
+        L.dpp = fp_max0(dpp);
         L.total = 0;
         L.retried = 0;
-        L.warm = W_PLAIN;
-        if (run.warm) {
-            // the learned starting depth of this solve, predicted before the launch:
-            // the bracket [p (1 - delta), p (1 + delta)] around a positive normal
-            // float p below 1e4 m (0x461c4000), else the plain bracket
-            const unsigned pb = (unsigned)((unsigned long long)tw >> 32);   // staged with the record
-            if (pb >= 0x00800000u && pb < 0x461c4000u) {
-                const double pr = __longlong_as_double(((long long)((pb >> 23) + 896) << 52) |
-                                                       ((long long)(pb & 0x7fffff) << 29));  // exact widening
-                L.h = pr * run.warm_hi;
-                L.h_0 = pr * run.warm_lo;
-                L.warm = W_ACTIVE;
-                ls.warm_used++;
-                if (run.start_hist) __stcg(run.start_hist + (size_t)L.tau * (size_t)net.n_seg_int + L.s, pr);
-            }
+        // the learned starting depth of this solve, predicted before the launch: the
+        // bracket [p (1 - delta), p (1 + delta)] around a positive normal float p
+        // below 1e4 m (0x461c4000), else the plain bracket
+        const unsigned pb = run.warm ? (unsigned)__double2loint(in.y) : 0u;
+        if (pb >= 0x00800000u && pb < 0x461c4000u) {
+            const double pr = __longlong_as_double(((long long)((pb >> 23) + 896) << 52) |
+                                                   ((long long)(pb & 0x7fffff) << 29));  // exact widening
+            restart_bracket(L, run.tol, pr * run.warm_hi, pr * run.warm_lo);
+            L.warm = W_ACTIVE;
+            ls.warm_used++;
+            if (run.start_hist) __stcg(run.start_hist + (size_t)L.tau * (size_t)net.n_seg_int + L.s, pr);
+        } else {
+            plain_bracket(L, run.tol);
+            L.warm = W_PLAIN;
         }
         return true;
     }
@@ -267,9 +290,8 @@ __device__ __forceinline__ void lane_finish(Lane& L, const PassOut& o, const Net
                 pr[1] = (float)L.quc;
                 pr[2] = (float)L.qdp;
                 const SegP p = staged_seg(seg_buf(slot, L.i));
-                const double2 tail = seg_buf(slot, L.i)[kParamPlanes * kSegSmemStride];
-                const int col = (int)(unsigned)(__double_as_longlong(tail.y) & 0xffffffffll);
-                pr[3] = (float)(__ldg(run.qlat + (size_t)L.tau * (size_t)run.qlat_ld + col) * tail.x);
+                const double2 tail = seg_buf(slot, L.i)[kTailPlane * kSegSmemStride];
+                pr[3] = (float)(__ldg(run.qlat + (size_t)L.tau * (size_t)run.qlat_ld + __double2loint(tail.y)) * tail.x);
                 pr[4] = (float)p.dx;
                 pr[5] = (float)p.s0;
                 pr[6] = (float)p.n_ch;

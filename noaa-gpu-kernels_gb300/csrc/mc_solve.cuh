@@ -74,23 +74,14 @@ struct PassOut {
     double h_1;    // secant estimate
 };
 
-// Parameter and time-step ranges in which the short forms are proven: with
-// these, depths of +0 or in [2^-100, 2^480) and flows below 2^100 every
-// intermediate but the secant's numerator (checked) is zero or inside the normal
-// range with room for its residual. The depths reach that far in earnest: where
-// the secant does not converge it doubles its bracket pass after pass, to 1e136
-// and beyond, until maxiter (at rtol 1e-8 one iteration in four is spent at
-// depths above 1e18 m). Above the bank the area is bounded by linear terms, so
-// R tends to twcc / 2 and the discharge grows like the depth.
-__device__ __forceinline__ bool seg_regular(const SegP& p, double dt)
-{
-    const double v[13] = {p.dx, p.bw, p.twcc, p.n_ch, p.ncc, p.s0, p.z, p.bfd, p.sq_s0, p.sq2, p.ck_fac, p.z2, dt};
-    bool ok = true;
-#pragma unroll
-    for (int i = 0; i < 13; ++i) ok &= (unsigned)(__double2hiint(v[i]) - (983 << 20)) < (80u << 20);   // [2^-40, 2^40), positive
-    return ok;
-}
-
+// Ranges in which the short forms are proven: with regular parameters and time
+// step (seg_regular, value_regular), depths of +0 or in [2^-100, 2^480) and flows
+// below 2^100 every intermediate but the secant's numerator (checked) is zero or
+// inside the normal range with room for its residual. The depths reach that far
+// in earnest: where the secant does not converge it doubles its bracket pass
+// after pass, to 1e136 and beyond, until maxiter (at rtol 1e-8 one iteration in
+// four is spent at depths above 1e18 m). Above the bank the area is bounded by
+// linear terms, so R tends to twcc / 2 and the discharge grows like the depth.
 // A positive depth in [2^-100, 2^480).
 __device__ __forceinline__ bool depth_regular(double x)
 {
@@ -349,8 +340,8 @@ struct SolveOut {
 // No solve: invalid parameters or no flow at all (troute_mc_final.cu:54-63).
 __device__ __forceinline__ bool exits_early(const SegP& p, double ql, double qup, double quc, double qdp)
 {
-    return p.n_ch <= 0.0 || p.s0 <= 0.0 || p.z <= 0.0 || p.bw <= 0.0 ||
-           (ql <= 0.0 && qup <= 0.0 && quc <= 0.0 && qdp <= 0.0);
+    return fp_le0(p.n_ch) || fp_le0(p.s0) || fp_le0(p.z) || fp_le0(p.bw) ||
+           (fp_le0(ql) && fp_le0(qup) && fp_le0(quc) && fp_le0(qdp));
 }
 
 __device__ __forceinline__ SolveOut mc_solve(double dt, double qup, double quc, double qdp,
@@ -369,7 +360,7 @@ __device__ __forceinline__ SolveOut mc_solve(double dt, double qup, double quc, 
     PassOut po = {0.0, 0.0, 0.0};
     int maxiter = tol.maxiter, attempt = 0, iter = 0;
     bool need0 = true;
-    bool irregular = !(seg_regular(p, dt) && flow_regular(qup) && flow_regular(quc) && flow_regular(qdp) && flow_regular(f.qldt));
+    bool irregular = !(seg_regular(p) && value_regular(dt) && flow_regular(qup) && flow_regular(quc) && flow_regular(qdp) && flow_regular(f.qldt));
     DepthEval e0, e;
     while (true) {
         secant_pass(p, f, need0 ? h_0 : h, need0, h, h_0, po.Qj_0, e0, irregular, e, po);

@@ -185,6 +185,7 @@ struct troute_handle {
     bool broken = false;
 
     DBuf<SegRec> seg;
+    DBuf<ReachRec> reach;
     DBuf<int> nseg, block_level, lb_ptr_d, up_ptr, up_idx, down, done, step_base;
     DBuf<double> q, d, v, ring, tmp, qlat_buf, hist;
     DBuf<long long> tile_off, seg_map_d, reach_map_d;
@@ -222,6 +223,7 @@ struct troute_handle {
         n.n_reach_int = R_int;
         n.n_seg_int = S_int;
         n.seg = seg.p;
+        n.reach = reach.p;
         n.nseg = nseg.p;
         n.tile_off = tile_off.p;
         n.block_level = block_level.p;
@@ -241,7 +243,7 @@ struct troute_handle {
     {
         if (graph_exec) cudaGraphExecDestroy(graph_exec);
         if (graph) cudaGraphDestroy(graph);
-        seg.release();
+        seg.release(); reach.release();
         nseg.release(); block_level.release(); lb_ptr_d.release();
         up_ptr.release(); up_idx.release(); down.release(); done.release(); step_base.release();
         q.release(); d.release(); v.release(); ring.release(); tmp.release();
@@ -313,6 +315,7 @@ static void put_params(Layout& Lt, long long t, const troute_chparams& c, int qc
     r.p[5] = double2{p.ck_fac, p.z2};
     r.qcol = qcol;
     r.qscale = qscale;
+    r.flags = seg_regular(p) ? 1 : 0;
 }
 
 static SegRec empty_rec()
@@ -565,6 +568,7 @@ static int upload_layout(troute_handle* H, Layout& Lt)
     if ((rc = cuda_check(cudaMemsetAsync(H->ring.p, 0, H->ring.n * sizeof(double), st), "memset"))) return rc;
     if ((rc = cuda_check(cudaMemsetAsync(H->done.p, 0, H->done.n * sizeof(int), st), "memset"))) return rc;
     if ((rc = cuda_check(cudaMemsetAsync(H->step_base.p, 0, sizeof(int), st), "memset"))) return rc;
+    if ((rc = H->reach.alloc(std::max(1, H->R_int))) || (rc = launch_reach_recs(H->net(), H->reach.p, st))) return rc;
     if ((rc = launch_shape(H))) return rc;
     return cuda_check(cudaStreamSynchronize(st), "build sync");
 }
@@ -869,6 +873,7 @@ static int enqueue_chunk(troute_handle* H, const double* qlat_dev, int n_ts, con
     run.n_ts = n_ts;
     run.dt = H->dt;
     run.dt_half = H->dt / 2.0;
+    run.dt_regular = value_regular(H->dt);
     run.qlat = qlat_dev;
     run.qlat_ld = H->qlat_cols;
     run.wave_ptr = wave;

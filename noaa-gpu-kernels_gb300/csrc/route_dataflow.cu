@@ -38,6 +38,7 @@ constexpr int L_FETCH = L_WAIT;  // claimed a queue slot, waiting for it to be w
 #endif
 // Queued items from which on warps fill all their lanes instead of kNarrow.
 constexpr int kWideItems = TROUTE_WIDE_ITEMS;
+constexpr int kTopUpItems = 64;
 #ifndef TROUTE_SLEEP_MAX_NS
 #define TROUTE_SLEEP_MAX_NS 3200
 #endif
@@ -51,9 +52,11 @@ __device__ __forceinline__ unsigned lanemask_lt_df()
     return m;
 }
 
-__device__ __forceinline__ long long ld_volatile_ll(const long long* p)
+__device__ __forceinline__ long long ld_acquire_ll(const long long* p)
 {
-    return *reinterpret_cast<const volatile long long*>(p);
+    long long v;
+    asm volatile("ld.acquire.gpu.global.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
 }
 
 __device__ __forceinline__ unsigned long long ld_volatile_ull(const unsigned long long* p)
@@ -85,20 +88,45 @@ __device__ __forceinline__ void start_item(Lane& L, int ri, int tau, int t_base,
     L.ri = ri;
     L.tau = tau;
     L.g = t_base + tau;
-    L.ns = __ldg(net.nseg + ri);
-    L.ub = __ldg(net.up_ptr + ri);
-    L.ue = __ldg(net.up_ptr + ri + 1);
-    L.dn = __ldg(net.down + ri);
-    L.base = __ldg(net.tile_off + ri / kLanes) + (ri % kLanes);
+    const int4* rec = reinterpret_cast<const int4*>(net.reach + ri);
+    const int4 a = __ldg(rec), b = __ldg(rec + 1);
+    const int2 c = __ldg(reinterpret_cast<const int2*>(rec + 2));   // row start in up_idx, inflow column
+    L.ns = a.x;
+    L.n_up = a.y;
+    L.dn = a.z;
+    L.dn_n_up = a.w;
+    L.base = ((long long)b.y << 32) | (unsigned)b.x;
+    if (L.ns > 0) {
+        stage_seg_async(net, run, tau, L.base, slot);
+        stage_inflow_async(run, tau, c.y, slot);
+    }
+    L.inflow = kInflowStaged;
+    // sums over the upstream reaches in their order, from +0 (a first addend of -0
+    // becomes +0, as in 0.0 + -0.0)
     const double* rprev = df.rh + (size_t)tau * R;
     const double* rcur = df.rh + (size_t)(tau + 1) * R;
-    L.qup_head = 0.0;
-    L.quc_head = 0.0;
-    for (int j = L.ub; j < L.ue; ++j) {
-        const int u = __ldg(net.up_idx + j);
-        L.qup_head += __ldcg(rprev + u);
-        L.quc_head += __ldcg(rcur + u);
+    double p = 0.0, q = 0.0;
+    if (L.n_up > 0) {
+        const double p0 = __ldcg(rprev + b.z), q0 = __ldcg(rcur + b.z);
+        double p1 = 0.0, q1 = 0.0;
+        if (L.n_up > 1) {
+            p1 = __ldcg(rprev + b.w);
+            q1 = __ldcg(rcur + b.w);
+        }
+        p = fp_eq0(p0) ? 0.0 : p0;
+        q = fp_eq0(q0) ? 0.0 : q0;
+        if (L.n_up > 1) {
+            p += p1;
+            q += q1;
+        }
+        for (int j = 2; j < L.n_up; ++j) {
+            const int u = __ldg(net.up_idx + c.x + j);
+            p += __ldcg(rprev + u);
+            q += __ldcg(rcur + u);
+        }
     }
+    L.qup_head = p;
+    L.quc_head = q;
     L.q_up_old = 0.0;
     L.q_up_new = 0.0;
     L.q_last = 0.0;
@@ -178,7 +206,10 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
                 err = seen_err;
                 if (seen_avail > 0) {
                     const int held = 32 - __popc(idle);
-                    const int room = seen_avail >= kWideItems ? 32 - held : primary ? kNarrow - held : 0;
+                    // (a narrow warp with work leaves small backlogs to idle ones three
+                    // passes out of four: its atomics would mostly find nothing left)
+                    const bool top_up = held == 0 || seen_avail >= kTopUpItems || (n_pass & 3) == 0;
+                    const int room = seen_avail >= kWideItems ? 32 - held : primary && top_up ? kNarrow - held : 0;
                     const int want = min(room, seen_avail);
                     if (want > 0) {
                         const int had = atomicSub(df.n_avail, want);
@@ -232,7 +263,8 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
 
         // ---- lanes with a claimed slot: start the item once it is written ----
         if (L.mode == L_FETCH) {
-            const long long raw = ld_volatile_ll(reinterpret_cast<const long long*>(df.rq + slot));
+            // (acquire: the item's inputs were published before it was queued)
+            const long long raw = ld_acquire_ll(reinterpret_cast<const long long*>(df.rq + slot));
             const int ri = (int)(raw & 0xffffffffll);
             const int tau = (int)(raw >> 32);
             if (ri >= 0 && (ri >= R || tau < 0 || tau >= T)) {
@@ -240,7 +272,6 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
                 record_error(run.stats, TROUTE_EINVAL, ri, tau, 8);
                 failed = true;
             } else if (ri >= 0) {
-                __threadfence();  // the item's inputs were published before it was queued
                 L.ri = ri;
                 L.tau = tau;
                 L.mode = L_START;
@@ -258,6 +289,9 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
                 }
             }
         }
+
+        // ---- the inflow of segments asked for before the last pass ----
+        if (L.mode == L_SOLVE) stage_next_inflow(L, run, seg_slot);
 
         // ---- lanes starting an item, then a segment (the one inlined
         // start_item and begin_segment) ----
@@ -289,23 +323,21 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
         if (dmask && lane == 0) atomicAdd(df.n_done, (unsigned long long)__popc(dmask));
         if (L.mode == L_DONE) {
             __stcg(df.rh + (size_t)(L.tau + 1) * R + L.ri, L.q_last);
-            __stcg(net.ring + (size_t)(L.g % kRing) * R + L.ri, L.q_last);
-            net.done[L.ri] = L.g + 1;   // read by later launches only
+            // what later launches start from
+            if (L.tau + kRing >= T) __stcg(net.ring + (size_t)(L.g % kRing) * R + L.ri, L.q_last);
+            if (L.tau + 1 == T) net.done[L.ri] = L.g + 1;
             __threadfence();
-            const int nup = L.ue - L.ub;
-            if (L.tau + 1 < T) {
-                // own next step: needs its upstream reaches too
-                const int old = atomicAdd(df.cnt + (size_t)(L.tau + 1) * R + L.ri, 1);
-                if (old + 1 == nup + 1) push0 = make_int2(L.ri, L.tau + 1), npush = 1;
-            }
-            if (L.dn >= 0) {
-                const int need = (__ldg(net.up_ptr + L.dn + 1) - __ldg(net.up_ptr + L.dn)) + (L.tau > 0 ? 1 : 0);
-                const int old = atomicAdd(df.cnt + (size_t)L.tau * R + L.dn, 1);
-                if (old + 1 == need) {
-                    if (npush == 0) push0 = make_int2(L.dn, L.tau);
-                    else push1 = make_int2(L.dn, L.tau);
-                    ++npush;
-                }
+            // the reach's own next step (needs its upstream reaches too) and the reach
+            // downstream: both counters in flight together
+            const bool own = L.tau + 1 < T, down = L.dn >= 0;
+            int own_old = 0, down_old = 0;
+            if (own) own_old = atomicAdd(df.cnt + (size_t)(L.tau + 1) * R + L.ri, 1);
+            if (down) down_old = atomicAdd(df.cnt + (size_t)L.tau * R + L.dn, 1);
+            if (own && own_old == L.n_up) push0 = make_int2(L.ri, L.tau + 1), npush = 1;
+            if (down && down_old + 1 == L.dn_n_up + (L.tau > 0 ? 1 : 0)) {
+                if (npush == 0) push0 = make_int2(L.dn, L.tau);
+                else push1 = make_int2(L.dn, L.tau);
+                ++npush;
             }
             L.mode = L_IDLE;
             if (npush && (df.continue_items || narrow)) {

@@ -145,6 +145,8 @@ __global__ void __launch_bounds__(128) route_pool_kernel(NetDev net, RunDev run)
                 L.q_up_new = 0.0;
                 L.q_last = 0.0;
                 L.i = 0;
+                L.inflow = kInflowLater;
+                if (L.ns > 0) stage_seg_async(net, run, L.tau, L.base, slot);
                 L.mode = L_BEGIN;
             } else if (clock64() - L.wait_t0 > run.wait_cycles) {
                 record_error(run.stats, TROUTE_ETIMEOUT, L.ri, L.g, 1);

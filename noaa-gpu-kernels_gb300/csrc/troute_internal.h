@@ -62,9 +62,10 @@ struct __align__(128) SegRec {
     double2 p[kParamPlanes];
     double qscale;
     int qcol;
+    int flags;   // bit 0: the parameters are regular (seg_regular)
     int reach;   // internal reach of the slot (-1: a slot no segment uses)
     int pos;     // position of the segment in its reach
-    int pad[3];
+    int pad[2];
 };
 static_assert(sizeof(SegRec) == 128, "one 128-byte line per segment");
 
@@ -81,6 +82,36 @@ TR_HD inline SegP derive_seg(const troute_chparams& c)
     p.z2 = 2.0 * p.z;
     return p;
 }
+
+// Parameter ranges ([2^-40, 2^40), positive) in which the secant pass's short
+// arithmetic is proven (mc_solve.cuh).
+TR_HD inline bool value_regular(double v)
+{
+#if defined(__CUDA_ARCH__)
+    return (unsigned)(__double2hiint(v) - (983 << 20)) < (80u << 20);   // off the FP64 pipe
+#else
+    return v >= 0x1p-40 && v < 0x1p40;
+#endif
+}
+TR_HD inline bool seg_regular(const SegP& p)
+{
+    return value_regular(p.dx) && value_regular(p.bw) && value_regular(p.twcc) && value_regular(p.n_ch) &&
+           value_regular(p.ncc) && value_regular(p.s0) && value_regular(p.z) && value_regular(p.bfd) &&
+           value_regular(p.sq_s0) && value_regular(p.sq2) && value_regular(p.ck_fac) && value_regular(p.z2);
+}
+
+// What starting and publishing an item reads of its reach, in one record: the
+// routing kernel would otherwise follow four dependent loads (row pointers,
+// upstream list, first segment, its inflow column).
+struct __align__(64) ReachRec {
+    int nseg, n_up, down, down_n_up;   // down: internal reach or -1
+    long long base;                    // tile slot of the first segment
+    int up0, up1;                      // the first two upstream reaches
+    int up_ptr;                        // row start in up_idx
+    int qcol;                          // inflow column of the first segment
+    int pad[6];
+};
+static_assert(sizeof(ReachRec) == 64, "two sectors per reach");
 
 // Device counters of one run.
 struct DevStats {
@@ -100,6 +131,7 @@ struct NetDev {
     int n_reach_int;         // n_blocks * kLanes
     long long n_seg_int;     // padded tile storage
     const SegRec* seg;       // [n_seg_int] parameters, inflow column and scale
+    const ReachRec* reach;   // [n_reach_int]
     const int* nseg;         // [n_reach_int], -1 for padding lanes
     const long long* tile_off;  // [n_blocks] first segment slot of a block
     const int* block_level;  // [n_blocks]
@@ -121,6 +153,7 @@ struct RunDev {
     int n_ts;
     double dt;
     double dt_half;          // dt / 2.0
+    int dt_regular;          // value_regular(dt)
     const double* qlat;      // [n_ts][qlat_ld]
     long long qlat_ld;
     const unsigned long long* wave_ptr;  // [n_ts + n_levels] ticket prefix per wave
@@ -185,6 +218,7 @@ int compact_pairs(const float* dense, long long n_rows, float* out, long long ca
 int route_dataflow_occupancy(int* blocks_per_sm, bool warm);
 int route_dataflow_threads();
 int launch_bump_steps(int* step_base, int n_ts, void* stream);
+int launch_reach_recs(const NetDev& net, ReachRec* out, void* stream);
 int launch_fill_int(int* p, long long n, const int* value_dev, int value_host, void* stream);
 int launch_scatter(const double* src, const long long* map, long long n, double* dst,
                    void* stream);
