@@ -119,7 +119,7 @@ extern "C" int troute_mc_reach_parallel_device(const troute_chparams* p, const d
     if ((rc = device_stats(&stats))) return rc;
     if ((rc = cuda_check(cudaMemsetAsync(stats, 0, sizeof(DevStats), (cudaStream_t)stream), "memset"))) return rc;
     return launch_reach_parallel(p, ql, rs, rl, qu, qd, dp, qo, vo, dpo, uq, dt, nr, n_segments, make_tol(c),
-                                 stats, c.threads_per_block, stream);
+                                 stats, stream);
 }
 
 extern "C" int troute_mc_reach_parallel_cfg(const troute_chparams* p, const double* ql,
@@ -179,7 +179,7 @@ extern "C" int troute_mc_reach_parallel_cfg(const troute_chparams* p, const doub
     cudaEventCreate(&e1);
     cudaEventRecord(e0, st);
     rc = launch_reach_parallel(dpar, dd, di, di + nr, dd + bs, dd + 2 * bs, dd + 3 * bs, dd + 4 * bs, dd + 5 * bs,
-                               dd + 6 * bs, uq, dt, nr, (int)S, make_tol(c), dst, c.threads_per_block, st);
+                               dd + 6 * bs, uq, dt, nr, (int)S, make_tol(c), dst, st);
     cudaEventRecord(e1, st);
     if (!rc) rc = cuda_check(cudaMemcpyAsync(qo, dd + 4 * bs, Sd, cudaMemcpyDeviceToHost, st), "D2H");
     if (!rc) rc = cuda_check(cudaMemcpyAsync(vo, dd + 5 * bs, Sd, cudaMemcpyDeviceToHost, st), "D2H");

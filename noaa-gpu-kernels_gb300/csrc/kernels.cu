@@ -29,45 +29,6 @@
 namespace tr {
 
 // ---------------------------------------------------------------------------
-// Reach-parallel single step: the drop-in for kernel_mc_gpu / cpu_mc
-// (troute_mc_final.cu:141-164, :167-252). One thread per reach, segments in
-// sequence, the first segment's current inflow seeded by uq. Parameters are
-// read in the caller's AoS layout (64-byte records).
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) reach_parallel_kernel(
-    const troute_chparams* __restrict__ p, const double* __restrict__ ql,
-    const int* __restrict__ rs, const int* __restrict__ rl,
-    const double* __restrict__ qu, const double* __restrict__ qd,
-    const double* __restrict__ dp, double* __restrict__ qo, double* __restrict__ vo,
-    double* __restrict__ dpo, double uq, double dt, int nr, int n_segments, Tol tol,
-    DevStats* stats)
-{
-    __shared__ unsigned int hist_s[16];
-    if (threadIdx.x < 16) hist_s[threadIdx.x] = 0;
-    __syncthreads();
-    LocalStats ls = {0, 0, 0, 0};
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < nr; r += gridDim.x * blockDim.x) {
-        const int start = rs[r], ns = rl[r];
-        if (start < 0 || ns < 0 || (long long)start + ns > (long long)n_segments) {
-            record_error(stats, TROUTE_EINVAL, r, 0, 4);
-            continue;
-        }
-        double quc = uq;
-        for (int i = 0; i < ns; ++i) {
-            const int s = start + i;
-            const SegP sp = derive_seg(p[s]);
-            const SolveOut o = mc_solve(dt, qu[s], quc, qd[s], ql[s], sp, dp[s], tol);
-            qo[s] = o.q;
-            vo[s] = o.vel;
-            dpo[s] = o.depth;
-            quc = o.q;
-            count_solve(ls, hist_s, o);
-        }
-    }
-    flush_stats(ls, hist_s, stats);
-}
-
-// ---------------------------------------------------------------------------
 // Persistent time-skewed tree routing.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) route_kernel(NetDev net, RunDev run)
@@ -281,19 +242,6 @@ static int grid_for(long long n, int threads)
     if (g < 1) g = 1;
     if (g > 65535LL * 8) g = 65535LL * 8;
     return (int)g;
-}
-
-int launch_reach_parallel(const troute_chparams* p, const double* ql, const int* rs,
-                          const int* rl, const double* qu, const double* qd, const double* dp,
-                          double* qo, double* vo, double* dpo, double uq, double dt, int nr,
-                          int n_segments, const Tol& tol, DevStats* stats, int threads,
-                          void* stream)
-{
-    if (nr <= 0) return TROUTE_OK;
-    if (threads <= 0) threads = 128;
-    reach_parallel_kernel<<<grid_for(nr, threads), threads, 0, (cudaStream_t)stream>>>(
-        p, ql, rs, rl, qu, qd, dp, qo, vo, dpo, uq, dt, nr, n_segments, tol, stats);
-    return cuda_status(cudaGetLastError(), "reach_parallel_kernel launch");
 }
 
 int route_occupancy(int threads, int* blocks_per_sm)

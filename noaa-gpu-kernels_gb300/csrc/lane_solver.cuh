@@ -234,10 +234,9 @@ __device__ __forceinline__ bool begin_segment(Lane& L, const NetDev& net, const 
 }
 
 // Books one secant iteration of a lane whose pass produced o and (already in
-// L.e0) the upper depth's evaluation: the bracket, the stop test, and at a stop
-// the stores and the move to the next segment.
-__device__ __forceinline__ void lane_finish(Lane& L, const PassOut& o, const NetDev& net, const RunDev& run,
-                                            LocalStats& ls, unsigned int* hist_s, double2* slot)
+// L.e0) the upper depth's evaluation: the bracket and the stop test. Returns true
+// when the solve is done (L.qdc, L.h).
+__device__ __forceinline__ bool lane_book(Lane& L, const PassOut& o, const RunDev& run, LocalStats& ls)
 {
     const Tol& tol = run.tol;
     L.Qj_0 = o.Qj_0;
@@ -263,53 +262,57 @@ __device__ __forceinline__ void lane_finish(Lane& L, const PassOut& o, const Net
     } else {
         stop = fp_lt_pos(L.h, kMinDepth) || !(more && L.iter <= L.maxiter);
     }
-    if (stop) {
-        bool done = true;
-        if (L.warm == W_PLAIN && L.iter >= L.maxiter) {
-            // widen the bracket (also after the last attempt, as the reference does)
-            L.h *= 1.33;
-            L.h_0 *= 0.67;
-            L.maxiter += 25;
-            L.retried = 1;
-            if (++L.attempt < tol.attempts) {
-                L.iter = 0;
-                L.need0 = 1;
-                L.ahead = false;
-                done = false;
-            }
-        }
-        if (done) {
-            // store the segment (its velocity is derived from the final depth
-            // once the run is over, see velocity_kernel) and start the next one
-            __stcg(net.q + L.s, L.qdc);
-            __stcg(net.d + L.s, L.h);
-            if (run.q_hist) __stcg(run.q_hist + (size_t)L.tau * (size_t)net.n_seg_int + L.s, L.qdc);
-            if (run.pairs) {
-                float* pr = run.pairs + ((size_t)L.tau * (size_t)net.n_seg_int + L.s) * 9;
-                pr[0] = (float)L.qup;
-                pr[1] = (float)L.quc;
-                pr[2] = (float)L.qdp;
-                const SegP p = staged_seg(seg_buf(slot, L.i));
-                const double2 tail = seg_buf(slot, L.i)[kTailPlane * kSegSmemStride];
-                pr[3] = (float)(__ldg(run.qlat + (size_t)L.tau * (size_t)run.qlat_ld + __double2loint(tail.y)) * tail.x);
-                pr[4] = (float)p.dx;
-                pr[5] = (float)p.s0;
-                pr[6] = (float)p.n_ch;
-                pr[7] = (float)p.bw;
-                pr[8] = (float)L.h;
-            }
-            L.q_up_old = L.qdp;
-            L.q_up_new = L.qdc;
-            L.q_last = L.qdc;
-            SolveOut o;
-            o.iters = L.total;
-            o.retried = L.retried;
-            o.early = 0;
-            count_solve(ls, hist_s, o);
-            ++L.i;
-            L.mode = L.i < L.ns ? L_BEGIN : L_DONE;
+    if (!stop) return false;
+    if (L.warm == W_PLAIN && L.iter >= L.maxiter) {
+        // widen the bracket (also after the last attempt, as the reference does)
+        L.h *= 1.33;
+        L.h_0 *= 0.67;
+        L.maxiter += 25;
+        L.retried = 1;
+        if (++L.attempt < tol.attempts) {
+            L.iter = 0;
+            L.need0 = 1;
+            L.ahead = false;
+            return false;
         }
     }
+    return true;
+}
+
+// Books an iteration; at a stop stores the segment (its velocity is derived from
+// the final depth once the run is over, see velocity_kernel) and moves on to the
+// next one.
+__device__ __forceinline__ void lane_finish(Lane& L, const PassOut& o, const NetDev& net, const RunDev& run,
+                                            LocalStats& ls, unsigned int* hist_s, double2* slot)
+{
+    if (!lane_book(L, o, run, ls)) return;
+    __stcg(net.q + L.s, L.qdc);
+    __stcg(net.d + L.s, L.h);
+    if (run.q_hist) __stcg(run.q_hist + (size_t)L.tau * (size_t)net.n_seg_int + L.s, L.qdc);
+    if (run.pairs) {
+        float* pr = run.pairs + ((size_t)L.tau * (size_t)net.n_seg_int + L.s) * 9;
+        pr[0] = (float)L.qup;
+        pr[1] = (float)L.quc;
+        pr[2] = (float)L.qdp;
+        const SegP p = staged_seg(seg_buf(slot, L.i));
+        const double2 tail = seg_buf(slot, L.i)[kTailPlane * kSegSmemStride];
+        pr[3] = (float)(__ldg(run.qlat + (size_t)L.tau * (size_t)run.qlat_ld + __double2loint(tail.y)) * tail.x);
+        pr[4] = (float)p.dx;
+        pr[5] = (float)p.s0;
+        pr[6] = (float)p.n_ch;
+        pr[7] = (float)p.bw;
+        pr[8] = (float)L.h;
+    }
+    L.q_up_old = L.qdp;
+    L.q_up_new = L.qdc;
+    L.q_last = L.qdc;
+    SolveOut so;
+    so.iters = L.total;
+    so.retried = L.retried;
+    so.early = 0;
+    count_solve(ls, hist_s, so);
+    ++L.i;
+    L.mode = L.i < L.ns ? L_BEGIN : L_DONE;
 }
 
 // One evaluation pass of a lane in SOLVE mode (no-op otherwise).

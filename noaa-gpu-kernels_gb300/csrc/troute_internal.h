@@ -122,6 +122,7 @@ struct DevStats {
     int err_reach;   // internal reach of the first failure
     int err_step;    // step of the first failure
     int err_where;   // 1 own, 2 upstream, 3 downstream back-pressure, 4 bounds
+    unsigned long long ticket;   // reaches handed out (reach-parallel step)
 };
 
 // Static network description on the device (internal order).
@@ -189,12 +190,11 @@ struct DataflowDev {
     unsigned long long n_items;     // real reaches x n_ts
 };
 
-// Launch helpers implemented in kernels.cu (all asynchronous on `stream`).
+// Launch helpers (all asynchronous on `stream`).
 int launch_reach_parallel(const troute_chparams* p, const double* ql, const int* rs,
                           const int* rl, const double* qu, const double* qd, const double* dp,
                           double* qo, double* vo, double* dpo, double uq, double dt, int nr,
-                          int n_segments, const Tol& tol, DevStats* stats, int threads,
-                          void* stream);
+                          int n_segments, const Tol& tol, DevStats* stats, void* stream);
 int launch_route(const NetDev& net, const RunDev& run, int grid, int threads, void* stream);
 int route_occupancy(int threads, int* blocks_per_sm);
 int launch_route_pool(const NetDev& net, const RunDev& run, int grid, int threads, void* stream);
