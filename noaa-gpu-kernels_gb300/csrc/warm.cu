@@ -40,13 +40,6 @@ __device__ __forceinline__ bool pair_features(const float* pr, const Norm& nm, f
     return true;
 }
 
-__device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
-__device__ __forceinline__ float dsilu_f(float z)
-{
-    const float s = 1.0f / (1.0f + expf(-z));
-    return s * (1.0f + z * (1.0f - s));
-}
-
 // Per-block sums of the log features and log depth (and their squares) over
 // the valid pairs, for the standardisation. Fixed-order reductions: the
 // result does not depend on scheduling.
@@ -89,148 +82,279 @@ __global__ void __launch_bounds__(kMomThreads) warm_moments_kernel(const float* 
 }
 
 // One mini-batch block of kTrainRows samples: forward, backward, and the
-// block's gradient (part[block][kNParams]) and loss sum (loss_part[block]).
+// block's gradient (part[block][kPartLd]) and loss sum (loss_part[block]).
 // Sample i of the batch is pair (perm_a * i + perm_b) mod n, a permutation of
 // the pairs when gcd(perm_a, n) = 1. Every sum runs in a fixed order, so a
 // training run is reproducible bit for bit.
-__global__ void __launch_bounds__(kTrainRows) warm_fb_kernel(const float* __restrict__ pairs, long long n,
-                                                             long long offset, int batch, unsigned long long perm_a,
-                                                             unsigned long long perm_b, const float* __restrict__ prm,
-                                                             Norm nm, float* __restrict__ part,
-                                                             double* __restrict__ loss_part, float inv_batch)
+//
+// FP32 multiply and add rates bound it: three 64 x 64 x 64 products per block
+// (layer 2 forward, its weight gradient, its input gradient), 12.3 k cycles of an
+// SM's FP32 lanes. kGemmThreads threads hold 4 x 4 tiles of each product in
+// registers, every sum over its inner index in order (what one thread per sample
+// did with 64 threads and scalar shared-memory reads in 94 us, batch 8,192);
+// activations whose derivative is needed later stay in the registers of the
+// thread that will use them. The other kChoreThreads form the bias and last-layer
+// sums beside the products.
+constexpr int kGemmThreads = 256, kChoreThreads = 128;
+constexpr int kTLd = 68;         // row of a 64-wide tile: 16-byte aligned, banks shifted by 4
+constexpr int kPartLd = 4804;    // row of the partial gradients, 16-byte aligned
+static_assert(kTrainRows == 64 && kWHid == 64 && kPartLd >= kNParams && kPartLd % 4 == 0 && kP_W2 % 4 == 0, "tile shapes");
+
+struct FbSmem {
+    float w1[kWHid][kWIn], b1[kWHid], b2[kWHid], w3[kWHid];
+    float x[kTrainRows][kWIn], y[kTrainRows], g[kTrainRows], e[kTrainRows];
+    int valid[kTrainRows];
+    float w2[kWHid][kTLd], w2t[kWHid][kTLd];        // [out][in], [in][out]
+    float a1[kTrainRows][kTLd], a1t[kWHid][kTLd];   // [sample][unit], [unit][sample]
+    float dz2[kTrainRows][kTLd], dz2t[kWHid][kTLd];
+    float a2[kTrainRows][kWHid + 1], dz1[kTrainRows][kWHid + 1];
+};
+
+// SiLU z / (1 + e^-z) and its derivative from one exponential.
+__device__ __forceinline__ void silu_both(float z, float* a, float* d)
 {
-    extern __shared__ float sm[];
-    float* W1 = sm;                          // 512
-    float* B1 = W1 + kWHid * kWIn;           // 64
-    float* W2 = B1 + kWHid;                  // 4096
-    float* B2 = W2 + kWHid * kWHid;          // 64
-    float* W3 = B2 + kWHid;                  // 64
-    float* G = W3 + kWHid;                   // [64] d(loss)/d(out) per sample
-    float* E = G + kTrainRows;               // [64] (err^2)/2 per sample
-    float* X = E + kTrainRows;               // [64][8]
-    float* Z1 = X + kTrainRows * kWIn;       // [64][65] pre-activations, then dZ1
-    float* A1 = Z1 + kTrainRows * 65;        // [64][65]
-    float* Z2 = A1 + kTrainRows * 65;        // [64][65] pre-activations, then dZ2
+    const float t = 1.0f + expf(-z);
+    *a = z / t;
+    const float s = 1.0f / t;
+    *d = s * (1.0f + z * (1.0f - s));
+}
+
+// acc[i][j] += u[i] * v[j] over a row of each operand.
+__device__ __forceinline__ void tile_step(float (&acc)[4][4], const float* u, const float* v)
+{
+    const float4 a = *reinterpret_cast<const float4*>(u), b = *reinterpret_cast<const float4*>(v);
+    const float ai[4] = {a.x, a.y, a.z, a.w}, bj[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] += ai[i] * bj[j];
+}
+
+// Programmatic dependent launch: what follows waits for the kernel before.
+__device__ __forceinline__ void wait_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__global__ void __launch_bounds__(kGemmThreads + kChoreThreads, 1)
+    warm_fb_kernel(const float* __restrict__ pairs, long long n, long long offset, int batch, unsigned long long perm_a,
+                   unsigned long long perm_b, const float* prm, Norm nm, float* __restrict__ part,
+                   double* __restrict__ loss_part, float inv_batch)
+{
+    extern __shared__ __align__(16) unsigned char fb_smem[];
+    FbSmem& S = *reinterpret_cast<FbSmem*>(fb_smem);
     const int tid = threadIdx.x;
-    for (int i = tid; i < kP_B3; i += blockDim.x) W1[i] = prm[i];
+    let_next_kernel_start();
+    // the samples do not depend on the weights: fetched while the last update runs
+    if (tid < kTrainRows) {
+        const long long i = offset + (long long)blockIdx.x * kTrainRows + tid;
+        float x[kWIn] = {};
+        float y = 0.0f;
+        bool valid = false;
+        if (i < offset + batch) {
+            const unsigned long long p = (perm_a * (unsigned long long)i + perm_b) % (unsigned long long)n;
+            valid = pair_features(pairs + p * kPairW, nm, x, &y);
+            if (!valid)
+                for (int k = 0; k < kWIn; ++k) x[k] = 0.0f;
+        }
+        for (int k = 0; k < kWIn; ++k) S.x[tid][k] = x[k];
+        S.y[tid] = y;
+        S.valid[tid] = valid;
+    }
+    wait_previous_kernel();
+    // (the weights change between launches that overlap: plain loads past L1)
+    for (int i = tid; i < kP_B3; i += blockDim.x) {
+        const float v = __ldcg(prm + i);
+        if (i < kP_B1) S.w1[i / kWIn][i % kWIn] = v;
+        else if (i < kP_W2) S.b1[i - kP_B1] = v;
+        else if (i < kP_B2) {
+            const int j = (i - kP_W2) / kWHid, k = (i - kP_W2) % kWHid;
+            S.w2[j][k] = v;
+            S.w2t[k][j] = v;
+        } else if (i < kP_W3) S.b2[i - kP_B2] = v;
+        else S.w3[i - kP_W3] = v;
+    }
+    const float b3 = __ldcg(prm + kP_B3);
     __syncthreads();
-    const float b3 = prm[kP_B3];
-    const long long i = offset + (long long)blockIdx.x * kTrainRows + tid;
-    float x[kWIn] = {};
-    float y = 0.0f;
-    bool valid = false;
-    if (i < offset + batch) {
-        const unsigned long long p = (perm_a * (unsigned long long)i + perm_b) % (unsigned long long)n;
-        valid = pair_features(pairs + p * kPairW, nm, x, &y);
-        if (!valid)
-            for (int k = 0; k < kWIn; ++k) x[k] = 0.0f;
-    }
-    for (int k = 0; k < kWIn; ++k) X[tid * kWIn + k] = x[k];
-    // forward
-    for (int j = 0; j < kWHid; ++j) {
-        float z = B1[j];
-        for (int k = 0; k < kWIn; ++k) z += W1[j * kWIn + k] * x[k];
-        Z1[tid * 65 + j] = z;
-        A1[tid * 65 + j] = silu_f(z);
-    }
-    float out = b3;
-    for (int j = 0; j < kWHid; ++j) {
-        float z = B2[j];
-        for (int k = 0; k < kWHid; ++k) z += W2[j * kWHid + k] * A1[tid * 65 + k];
-        Z2[tid * 65 + j] = z;
-        out += W3[j] * silu_f(z);
-    }
-    const float err = valid ? (out - y) : 0.0f;
-    G[tid] = err * inv_batch;  // loss = sum(err^2) / (2 batch)
-    E[tid] = 0.5f * err * err;
-    __syncthreads();
-    float* gp = part + (size_t)blockIdx.x * kNParams;
-    {
-        // dw3[j] = sum_s G[s] silu(Z2[s][j]) (thread j); db3, loss (thread 0)
-        const int j = tid;
-        float acc = 0.0f;
-        for (int s = 0; s < kTrainRows; ++s) acc += G[s] * silu_f(Z2[s * 65 + j]);
-        gp[kP_W3 + j] = acc;
-        if (tid == 0) {
-            float gb = 0.0f;
-            double ls = 0.0;
-            for (int s = 0; s < kTrainRows; ++s) {
-                gb += G[s];
-                ls += (double)E[s];
+    float* gp = part + (size_t)blockIdx.x * kPartLd;
+    const bool gemm = tid < kGemmThreads;
+    const int u0 = (tid / 16) * 4, v0 = (tid % 16) * 4;   // this thread's tile
+    float d1[4][4], d2[4][4];                             // SiLU' of layer 1 and 2 (sample, unit)
+    if (gemm) {
+        // layer 1
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float a[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float z = S.b1[v0 + j];
+#pragma unroll
+                for (int k = 0; k < kWIn; ++k) z += S.w1[v0 + j][k] * S.x[u0 + i][k];
+                silu_both(z, &a[i], &d1[i][j]);
+                S.a1[u0 + i][v0 + j] = a[i];
             }
+            *reinterpret_cast<float4*>(&S.a1t[v0 + j][u0]) = make_float4(a[0], a[1], a[2], a[3]);
+        }
+    }
+    __syncthreads();
+    if (gemm) {
+        // layer 2: z2[s][j] = b2[j] + sum_k W2[j][k] a1[s][k]
+        float acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = S.b2[v0 + j];
+#pragma unroll 8
+        for (int k = 0; k < kWHid; ++k) tile_step(acc, &S.a1t[k][u0], &S.w2t[k][v0]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float a;
+                silu_both(acc[i][j], &a, &d2[i][j]);
+                S.a2[u0 + i][v0 + j] = a;
+            }
+    }
+    __syncthreads();
+    if (tid < kTrainRows) {
+        float out = b3;
+#pragma unroll 16
+        for (int j = 0; j < kWHid; ++j) out += S.w3[j] * S.a2[tid][j];
+        const float err = S.valid[tid] ? (out - S.y[tid]) : 0.0f;
+        S.g[tid] = err * inv_batch;  // loss = sum(err^2) / (2 batch)
+        S.e[tid] = 0.5f * err * err;
+    }
+    __syncthreads();
+    if (gemm) {
+        float t[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) t[i][j] = S.g[u0 + i] * S.w3[v0 + j] * d2[i][j];
+            *reinterpret_cast<float4*>(&S.dz2[u0 + i][v0]) = make_float4(t[i][0], t[i][1], t[i][2], t[i][3]);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            *reinterpret_cast<float4*>(&S.dz2t[v0 + j][u0]) = make_float4(t[0][j], t[1][j], t[2][j], t[3][j]);
+    }
+    __syncthreads();
+    if (gemm) {
+        // dW2[j][k] = sum_s dZ2[s][j] a1[s][k]
+        float acc[4][4] = {};
+#pragma unroll 8
+        for (int s = 0; s < kTrainRows; ++s) tile_step(acc, &S.dz2[s][u0], &S.a1[s][v0]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<float4*>(gp + kP_W2 + (u0 + i) * kWHid + v0) =
+                make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        // dA1[s][k] = sum_j W2[j][k] dZ2[s][j]
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+#pragma unroll 8
+        for (int j = 0; j < kWHid; ++j) tile_step(acc, &S.dz2t[j][u0], &S.w2[j][v0]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) S.dz1[u0 + i][v0 + j] = acc[i][j] * d1[i][j];
+    } else {
+        const int c = tid - kGemmThreads;
+        if (c < kWHid) {
+            float acc = 0.0f;   // dw3[j] = sum_s G[s] a2[s][j]
+#pragma unroll 16
+            for (int s = 0; s < kTrainRows; ++s) acc += S.g[s] * S.a2[s][c];
+            gp[kP_W3 + c] = acc;
+        } else {
+            const int j = c - kWHid;
+            float db = 0.0f;
+#pragma unroll 16
+            for (int s = 0; s < kTrainRows; ++s) db += S.dz2[s][j];
+            gp[kP_B2 + j] = db;
+        }
+        if (c == 0) {
+            float gb = 0.0f;
+            for (int s = 0; s < kTrainRows; ++s) gb += S.g[s];
             gp[kP_B3] = gb;
+        }
+        if (c == kWHid) {
+            double ls = 0.0;
+            for (int s = 0; s < kTrainRows; ++s) ls += (double)S.e[s];
             loss_part[blockIdx.x] = ls;
         }
     }
     __syncthreads();
-    // dZ2 (own row, in place)
-    for (int j = 0; j < kWHid; ++j) Z2[tid * 65 + j] = G[tid] * W3[j] * dsilu_f(Z2[tid * 65 + j]);
-    __syncthreads();
-    // dW2[j][k] = sum_s dZ2[s][j] A1[s][k], db2[j] (thread j)
-    {
-        const int j = tid;
-        float db = 0.0f;
-        for (int s = 0; s < kTrainRows; ++s) db += Z2[s * 65 + j];
-        gp[kP_B2 + j] = db;
-        for (int k = 0; k < kWHid; ++k) {
-            float acc = 0.0f;
-            for (int s = 0; s < kTrainRows; ++s) acc += Z2[s * 65 + j] * A1[s * 65 + k];
-            gp[kP_W2 + j * kWHid + k] = acc;
-        }
-    }
-    // dZ1 (own row, in place): dA1[k] = sum_j W2[j][k] dZ2[j]
-    for (int k = 0; k < kWHid; ++k) {
-        float da = 0.0f;
-        for (int j = 0; j < kWHid; ++j) da += W2[j * kWHid + k] * Z2[tid * 65 + j];
-        Z1[tid * 65 + k] = da * dsilu_f(Z1[tid * 65 + k]);
-    }
-    __syncthreads();
-    {
-        const int j = tid;
-        float db = 0.0f;
-        float acc[kWIn] = {};
+    if (gemm) {
+        const int j = tid / 4, k = (tid % 4) * 2;   // dW1[j][k], dW1[j][k + 1]
+        float a = 0.0f, b = 0.0f;
+#pragma unroll 16
         for (int s = 0; s < kTrainRows; ++s) {
-            const float d = Z1[s * 65 + j];
-            db += d;
-            for (int k = 0; k < kWIn; ++k) acc[k] += d * X[s * kWIn + k];
+            const float d = S.dz1[s][j];
+            a += d * S.x[s][k];
+            b += d * S.x[s][k + 1];
         }
+        gp[kP_W1 + j * kWIn + k] = a;
+        gp[kP_W1 + j * kWIn + k + 1] = b;
+    } else if (tid - kGemmThreads < kWHid) {
+        const int j = tid - kGemmThreads;
+        float db = 0.0f;
+#pragma unroll 16
+        for (int s = 0; s < kTrainRows; ++s) db += S.dz1[s][j];
         gp[kP_B1 + j] = db;
-        for (int k = 0; k < kWIn; ++k) gp[kP_W1 + j * kWIn + k] = acc[k];
     }
 }
 
-// grad[i] = sum over blocks of part[b][i], blocks in order; loss likewise.
-__global__ void warm_reduce_kernel(const float* __restrict__ part, int nblocks, float* __restrict__ grad,
-                                   const double* __restrict__ loss_part, double* __restrict__ loss_acc)
+// One AdamW step's constants; apply = 0: only the gradient is formed.
+struct AdamW {
+    float lr, b1, b2, eps, wd, c1, c2;
+    int apply;
+};
+
+// grad[i] = sum over blocks of part[b][i], blocks in order (their loads in flight
+// together), and the AdamW step of parameter i.
+constexpr int kUpdateThreads = 64, kUpdateBatch = 32;
+__global__ void __launch_bounds__(kUpdateThreads) warm_update_kernel(const float* part, int nblocks, float* __restrict__ grad,
+                                                                     float* prm, float* m, float* v, AdamW o)
 {
+    let_next_kernel_start();
+    wait_previous_kernel();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kNParams) {
-        float g = 0.0f;
-        for (int b = 0; b < nblocks; ++b) g += part[(size_t)b * kNParams + i];
-        grad[i] = g;
+    if (i >= kNParams) return;
+    float g = 0.0f;
+    for (int b0 = 0; b0 < nblocks; b0 += kUpdateBatch) {
+        float t[kUpdateBatch];
+#pragma unroll
+        for (int b = 0; b < kUpdateBatch; ++b) t[b] = b0 + b < nblocks ? __ldcg(part + (size_t)(b0 + b) * kPartLd + i) : 0.0f;
+#pragma unroll
+        for (int b = 0; b < kUpdateBatch; ++b)
+            if (b0 + b < nblocks) g += t[b];
     }
-    if (i == 0) {
-        double l = 0.0;
-        for (int b = 0; b < nblocks; ++b) l += loss_part[b];
-        *loss_acc += l;
-    }
+    grad[i] = g;
+    if (!o.apply) return;
+    // (launches overlap: what the one before wrote is read past L1)
+    const float mi = o.b1 * __ldcg(m + i) + (1.0f - o.b1) * g;
+    const float vi = o.b2 * __ldcg(v + i) + (1.0f - o.b2) * g * g;
+    m[i] = mi;
+    v[i] = vi;
+    const bool is_weight = (i < kP_B1) || (i >= kP_W2 && i < kP_B2) || (i >= kP_W3 && i < kP_B3);
+    float p = __ldcg(prm + i);
+    if (is_weight) p -= o.lr * o.wd * p;
+    p -= o.lr * (mi / o.c1) / (sqrtf(vi / o.c2) + o.eps);
+    prm[i] = p;
 }
 
-__global__ void warm_adamw_kernel(float* __restrict__ prm, const float* __restrict__ grad, float* __restrict__ m,
-                                  float* __restrict__ v, int n, float lr, float b1, float b2, float eps, float wd,
-                                  float c1, float c2)
+// Loss of each step (its blocks in order), then *loss_acc += the steps in order.
+__global__ void __launch_bounds__(256) warm_loss_kernel(const double* __restrict__ loss_part, int nblocks, int steps,
+                                                        double* __restrict__ step_loss, double* __restrict__ loss_acc)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float g = grad[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * g;
-        const float vi = b2 * v[i] + (1.0f - b2) * g * g;
-        m[i] = mi;
-        v[i] = vi;
-        const bool is_weight = (i < kP_B1) || (i >= kP_W2 && i < kP_B2) || (i >= kP_W3 && i < kP_B3);
-        float p = prm[i];
-        if (is_weight) p -= lr * wd * p;
-        p -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-        prm[i] = p;
+    for (int s = threadIdx.x; s < steps; s += blockDim.x) {
+        double l = 0.0;
+        for (int b = 0; b < nblocks; ++b) l += loss_part[(size_t)s * nblocks + b];
+        step_loss[s] = l;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double a = *loss_acc;
+        for (int s = 0; s < steps; ++s) a += step_loss[s];
+        *loss_acc = a;
     }
 }
 
@@ -322,6 +446,7 @@ struct troute_warm {
     float* d_part = nullptr;
     double* d_lpart = nullptr;
     int part_blocks = 0;
+    size_t lpart_n = 0;
 
     ~troute_warm()
     {
@@ -357,36 +482,64 @@ static int warm_alloc(troute_warm* w)
     return TROUTE_OK;
 }
 
-// Room for the per-block partials of a mini-batch of nblocks blocks.
-static int warm_parts(troute_warm* w, int nblocks)
+// Room for the partial gradients of a mini-batch of nblocks blocks, and for the
+// block losses of `steps` of them with a sum each.
+static int warm_parts(troute_warm* w, int nblocks, int steps)
 {
-    if (nblocks <= w->part_blocks) return TROUTE_OK;
-    if (w->d_part) cudaFree(w->d_part);
-    if (w->d_lpart) cudaFree(w->d_lpart);
-    w->d_part = nullptr;
-    w->d_lpart = nullptr;
-    w->part_blocks = 0;
     int rc;
-    if ((rc = warm_cuda(cudaMalloc(&w->d_part, (size_t)nblocks * kNParams * sizeof(float)), "cudaMalloc")) ||
-        (rc = warm_cuda(cudaMalloc(&w->d_lpart, (size_t)nblocks * sizeof(double)), "cudaMalloc")))
-        return rc;
-    w->part_blocks = nblocks;
+    if (nblocks > w->part_blocks) {
+        if (w->d_part) cudaFree(w->d_part);
+        w->d_part = nullptr;
+        w->part_blocks = 0;
+        if ((rc = warm_cuda(cudaMalloc(&w->d_part, (size_t)nblocks * kPartLd * sizeof(float)), "cudaMalloc"))) return rc;
+        w->part_blocks = nblocks;
+    }
+    const size_t need = (size_t)steps * ((size_t)nblocks + 1);
+    if (need > w->lpart_n) {
+        if (w->d_lpart) cudaFree(w->d_lpart);
+        w->d_lpart = nullptr;
+        w->lpart_n = 0;
+        if ((rc = warm_cuda(cudaMalloc(&w->d_lpart, need * sizeof(double)), "cudaMalloc"))) return rc;
+        w->lpart_n = need;
+    }
     return TROUTE_OK;
 }
 
-constexpr size_t kFbSmem = (size_t)(kP_B3 + 2 * kTrainRows + kTrainRows * kWIn + 3 * kTrainRows * 65) * sizeof(float);
+// Launches kernel so that it may start (up to its wait) while the one before it on
+// the stream still runs.
+template <class... P, class... A>
+static cudaError_t launch_overlapped(void (*kernel)(P...), int blocks, int threads, size_t smem, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
 
-// Gradient (into d_g) and loss sum (added to *d_loss) of one mini-batch.
-static int warm_fb(troute_warm* w, const float* pairs, long long n, long long off, int b, unsigned long long pa,
-                   unsigned long long pb, float inv_batch)
+static int warm_fb_attr()
+{
+    return warm_cuda(cudaFuncSetAttribute(warm_fb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FbSmem)),
+                     "smem attribute");
+}
+
+// One mini-batch: gradient into d_g, AdamW step o, block losses into lpart.
+static int warm_step(troute_warm* w, const float* pairs, long long n, long long off, int b, unsigned long long pa,
+                     unsigned long long pb, float inv_batch, const AdamW& o, double* lpart)
 {
     const int nblocks = (b + kTrainRows - 1) / kTrainRows;
-    int rc = warm_parts(w, nblocks);
+    const int rc = warm_cuda(launch_overlapped(warm_fb_kernel, nblocks, kGemmThreads + kChoreThreads, sizeof(FbSmem), pairs, n,
+                                               off, b, pa, pb, w->d_prm, w->nm, w->d_part, lpart, inv_batch),
+                             "training launch");
     if (rc) return rc;
-    warm_fb_kernel<<<nblocks, kTrainRows, kFbSmem>>>(pairs, n, off, b, pa, pb, w->d_prm, w->nm, w->d_part, w->d_lpart,
-                                                     inv_batch);
-    warm_reduce_kernel<<<(kNParams + 255) / 256, 256>>>(w->d_part, nblocks, w->d_g, w->d_lpart, w->d_loss);
-    return TROUTE_OK;
+    return warm_cuda(launch_overlapped(warm_update_kernel, (kNParams + kUpdateThreads - 1) / kUpdateThreads, kUpdateThreads, 0,
+                                       w->d_part, nblocks, w->d_g, w->d_prm, w->d_m, w->d_v, o),
+                     "update launch");
 }
 
 // Rounds the fp32 weights to the bf16, transposed, padded layout of the MMA path.
@@ -546,28 +699,52 @@ extern "C" int troute_warm_fit(troute_warm* w, const float* pairs_dev, long long
         (rc = warm_cuda(cudaMemset(w->d_m, 0, kNParams * sizeof(float)), "memset")) ||
         (rc = warm_cuda(cudaMemset(w->d_v, 0, kNParams * sizeof(float)), "memset")))
         return rc;
-    if ((rc = warm_cuda(cudaFuncSetAttribute(warm_fb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)kFbSmem), "smem attribute")))
-        return rc;
+    if ((rc = warm_fb_attr())) return rc;
     const long long steps_per_epoch = (n_pairs + batch - 1) / batch;
     const long long total = steps_per_epoch * epochs;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    // block losses are kept for a run of steps and summed together: one thread's
+    // sum of 128 doubles takes longer than a whole update
+    const int full_blocks = batch / kTrainRows;
+    const int keep = (int)std::min<long long>(steps_per_epoch, std::max(1, (1 << 22) / (full_blocks + 1)));
+    if ((rc = warm_parts(w, full_blocks, keep))) return rc;
+    double* const step_loss = w->d_lpart + (size_t)keep * full_blocks;
     long long step = 0;
     for (int ep = 0; ep < epochs; ++ep) {
         const unsigned long long pa = coprime_near((unsigned long long)n_pairs, hash3(seed, 31, ep) | 1ull);
         const unsigned long long pb = hash3(seed, 37, ep) % (unsigned long long)n_pairs;
         if ((rc = warm_cuda(cudaMemset(w->d_loss, 0, sizeof(double)), "memset"))) return rc;
+        int kept = 0;
         for (long long s = 0; s < steps_per_epoch; ++s, ++step) {
             const long long off = s * batch;
             const int b = (int)std::min<long long>(batch, n_pairs - off);
-            if ((rc = warm_fb(w, pairs_dev, n_pairs, off, b, pa, pb, 1.0f / (float)b))) return rc;
             // cosine decay of the step size
             const float frac = (float)step / (float)std::max<long long>(1, total - 1);
-            const float lr_t = lr * 0.5f * (1.0f + std::cos(3.14159265f * frac));
-            const float c1 = 1.0f - std::pow(b1, (float)(step + 1)), c2 = 1.0f - std::pow(b2, (float)(step + 1));
-            warm_adamw_kernel<<<(kNParams + 255) / 256, 256>>>(w->d_prm, w->d_g, w->d_m, w->d_v, kNParams, lr_t, b1,
-                                                               b2, eps, weight_decay, c1, c2);
+            AdamW o;
+            o.lr = lr * 0.5f * (1.0f + std::cos(3.14159265f * frac));
+            o.c1 = 1.0f - std::pow(b1, (float)(step + 1));
+            o.c2 = 1.0f - std::pow(b2, (float)(step + 1));
+            o.b1 = b1;
+            o.b2 = b2;
+            o.eps = eps;
+            o.wd = weight_decay;
+            o.apply = 1;
+            const int nblocks = (b + kTrainRows - 1) / kTrainRows;
+            // (a last, smaller batch is summed on its own: its rows are shorter)
+            if (kept == keep || (kept && nblocks != full_blocks)) {
+                warm_loss_kernel<<<1, 256>>>(w->d_lpart, full_blocks, kept, step_loss, w->d_loss);
+                kept = 0;
+            }
+            if ((rc = warm_step(w, pairs_dev, n_pairs, off, b, pa, pb, 1.0f / (float)b, o,
+                                w->d_lpart + (size_t)kept * full_blocks)))
+                return rc;
+            ++kept;
+            if (nblocks != full_blocks) {
+                warm_loss_kernel<<<1, 256>>>(w->d_lpart, nblocks, 1, step_loss, w->d_loss);
+                kept = 0;
+            }
         }
+        if (kept) warm_loss_kernel<<<1, 256>>>(w->d_lpart, full_blocks, kept, step_loss, w->d_loss);
         double loss = 0.0;
         if ((rc = warm_cuda(cudaMemcpy(&loss, w->d_loss, sizeof(double), cudaMemcpyDeviceToHost), "loss"))) return rc;
         // each step's loss is sum(err^2)/2 over its batch: the epoch mean per pair
@@ -589,10 +766,14 @@ extern "C" int troute_warm_grad(troute_warm* w, const float* pairs_host, int n, 
     rc = warm_cuda(cudaMemcpy(d_pairs, pairs_host, (size_t)n * kPairW * sizeof(float), cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = warm_cuda(cudaMemcpy(w->d_prm, w->prm, sizeof w->prm, cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = warm_cuda(cudaMemset(w->d_loss, 0, sizeof(double)), "memset");
-    if (!rc)
-        rc = warm_cuda(cudaFuncSetAttribute(warm_fb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFbSmem),
-                       "smem attribute");
-    if (!rc) rc = warm_fb(w, d_pairs, n, 0, n, 1, 0, 1.0f / (float)n);
+    if (!rc) rc = warm_fb_attr();
+    const int nblocks = (n + kTrainRows - 1) / kTrainRows;
+    if (!rc) rc = warm_parts(w, nblocks, 1);
+    if (!rc) rc = warm_step(w, d_pairs, n, 0, n, 1, 0, 1.0f / (float)n, AdamW{}, w->d_lpart);
+    if (!rc) {
+        warm_loss_kernel<<<1, 256>>>(w->d_lpart, nblocks, 1, w->d_lpart + nblocks, w->d_loss);
+        rc = warm_cuda(cudaGetLastError(), "loss launch");
+    }
     if (!rc) rc = warm_cuda(cudaMemcpy(grad_out, w->d_g, kNParams * sizeof(float), cudaMemcpyDeviceToHost), "D2H");
     double loss = 0.0;
     if (!rc) rc = warm_cuda(cudaMemcpy(&loss, w->d_loss, sizeof(double), cudaMemcpyDeviceToHost), "D2H");
