@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <vector>
 
@@ -81,34 +82,50 @@ __global__ void __launch_bounds__(kMomThreads) warm_moments_kernel(const float* 
     }
 }
 
-// One mini-batch block of kTrainRows samples: forward, backward, and the
-// block's gradient (part[block][kPartLd]) and loss sum (loss_part[block]).
-// Sample i of the batch is pair (perm_a * i + perm_b) mod n, a permutation of
-// the pairs when gcd(perm_a, n) = 1. Every sum runs in a fixed order, so a
-// training run is reproducible bit for bit.
+// Training steps in one cooperative launch. A step: the blocks take the
+// mini-batch's tiles of kTrainRows samples, forward and backward, and write each
+// tile's gradient (part[tile][kPartLd]) and its samples' (err^2)/2; after a grid
+// barrier each block sums its share of the parameters over the tiles in order and
+// takes the AdamW step for them; after a second one the next step begins. Sample i
+// of the epoch is pair (perm_a * i + perm_b) mod n, a permutation of the pairs when
+// gcd(perm_a, n) = 1. Every sum runs in a fixed order, so a training run is
+// reproducible bit for bit. (As two launches per step, overlapped by programmatic
+// dependent launch, 13 of a step's 30 us lay between the kernels.)
 //
-// FP32 multiply and add rates bound it: three 64 x 64 x 64 products per block
-// (layer 2 forward, its weight gradient, its input gradient), 12.3 k cycles of an
-// SM's FP32 lanes. kGemmThreads threads hold 4 x 4 tiles of each product in
-// registers, every sum over its inner index in order (what one thread per sample
-// did with 64 threads and scalar shared-memory reads in 94 us, batch 8,192);
-// activations whose derivative is needed later stay in the registers of the
-// thread that will use them. The other kChoreThreads form the bias and last-layer
-// sums beside the products.
+// FP32 multiply and add rates and shared-memory bandwidth bound it (both 64 cycles
+// of an SM per inner index): three 64 x 64 x 64 products per block (layer 2
+// forward, its weight gradient, its input gradient). kGemmThreads threads hold
+// 4 x 4 tiles of each product in registers, every sum over its inner index in order
+// (one thread per sample with scalar shared-memory reads took 94 us a batch of
+// 8,192). A thread's units are 16 apart where they are rows of the shared arrays,
+// so that reads of four consecutive inner values are free of bank conflicts and no
+// array is needed in both orders. Activations whose derivative is needed later
+// stay in the registers of the thread that will use them; the other kChoreThreads
+// form the bias and last-layer sums beside the products. (Packed f32x2
+// instructions on 2 x 4 tiles of 512 threads were no faster.)
 constexpr int kGemmThreads = 256, kChoreThreads = 128;
 constexpr int kTLd = 68;         // row of a 64-wide tile: 16-byte aligned, banks shifted by 4
 constexpr int kPartLd = 4804;    // row of the partial gradients, 16-byte aligned
 static_assert(kTrainRows == 64 && kWHid == 64 && kPartLd >= kNParams && kPartLd % 4 == 0 && kP_W2 % 4 == 0, "tile shapes");
 
-struct FbSmem {
+// The update: kUpdateRows threads per parameter fetch the partials of kUpdateTiles
+// tiles at once into shared memory; one adds them up.
+constexpr int kUpdateParams = 48, kUpdateRows = (kGemmThreads + kChoreThreads) / kUpdateParams, kUpdateTiles = 128;
+
+struct __align__(16) FbSmem {
     float w1[kWHid][kWIn], b1[kWHid], b2[kWHid], w3[kWHid];
-    float x[kTrainRows][kWIn], y[kTrainRows], g[kTrainRows], e[kTrainRows];
-    int valid[kTrainRows];
-    float w2[kWHid][kTLd], w2t[kWHid][kTLd];        // [out][in], [in][out]
-    float a1[kTrainRows][kTLd], a1t[kWHid][kTLd];   // [sample][unit], [unit][sample]
-    float dz2[kTrainRows][kTLd], dz2t[kWHid][kTLd];
+    float x[kTrainRows][kWIn], y[kTrainRows], g[kTrainRows];
+    float sums[kUpdateTiles][kUpdateParams];
+    float w2[kWHid][kTLd];                              // [out][in]
+    float a1[kTrainRows][kTLd], dz2[kTrainRows][kTLd];  // [sample][unit]
     float a2[kTrainRows][kWHid + 1], dz1[kTrainRows][kWHid + 1];
+    int valid[kTrainRows], stop;
 };
+// the arrays read and written as float4
+static_assert(offsetof(FbSmem, w1) % 16 == 0 && offsetof(FbSmem, b1) % 16 == 0 && offsetof(FbSmem, b2) % 16 == 0 &&
+                  offsetof(FbSmem, w3) % 16 == 0 && offsetof(FbSmem, x) % 16 == 0 && offsetof(FbSmem, w2) % 16 == 0 &&
+                  offsetof(FbSmem, a1) % 16 == 0 && offsetof(FbSmem, dz2) % 16 == 0,
+              "16-byte aligned");
 
 // SiLU z / (1 + e^-z) and its derivative from one exponential.
 __device__ __forceinline__ void silu_both(float z, float* a, float* d)
@@ -119,39 +136,81 @@ __device__ __forceinline__ void silu_both(float z, float* a, float* d)
     *d = s * (1.0f + z * (1.0f - s));
 }
 
-// acc[i][j] += u[i] * v[j] over a row of each operand.
-__device__ __forceinline__ void tile_step(float (&acc)[4][4], const float* u, const float* v)
+__device__ __forceinline__ void load4(const float* p, float (&v)[4])
 {
-    const float4 a = *reinterpret_cast<const float4*>(u), b = *reinterpret_cast<const float4*>(v);
-    const float ai[4] = {a.x, a.y, a.z, a.w}, bj[4] = {b.x, b.y, b.z, b.w};
+    const float4 t = *reinterpret_cast<const float4*>(p);
+    v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+}
+
+// acc[i][j] += u[i] v[j], a product and a sum each.
+__device__ __forceinline__ void tile_step(float (&acc)[4][4], const float (&u)[4], const float (&v)[4])
+{
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] += ai[i] * bj[j];
+        for (int j = 0; j < 4; ++j) acc[i][j] += u[i] * v[j];
 }
 
-// Programmatic dependent launch: what follows waits for the kernel before.
-__device__ __forceinline__ void wait_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_next_kernel_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// AdamW constants of a step.
+struct AdamStep {
+    float lr, c1, c2;
+};
 
-__global__ void __launch_bounds__(kGemmThreads + kChoreThreads, 1)
-    warm_fb_kernel(const float* __restrict__ pairs, long long n, long long offset, int batch, unsigned long long perm_a,
-                   unsigned long long perm_b, const float* prm, Norm nm, float* __restrict__ part,
-                   double* __restrict__ loss_part, float inv_batch)
+struct TrainArgs {
+    const float* pairs;
+    long long n, offset;          // pairs; first sample of the first step
+    int batch, steps;             // samples per step (the last may be shorter)
+    long long end;                // samples of the epoch
+    unsigned long long perm_a, perm_b;
+    Norm nm;
+    const AdamStep* step;         // [steps], null: gradient only
+    float b1, b2, eps, wd;
+    float *prm, *grad, *m, *v, *part, *sq_err;   // sq_err [steps][batch]
+    unsigned* barrier;            // arrivals; [1] set when a wait ran out
+};
+
+// Grid barrier in two halves; the k-th wait ends when k * gridDim.x blocks have
+// arrived, or (false, for every block soon after) when it takes too long.
+constexpr long long kBarrierCycles = 4000000000LL;   // ~2 s
+__device__ __forceinline__ void grid_arrive(unsigned* bar)
 {
-    extern __shared__ __align__(16) unsigned char fb_smem[];
-    FbSmem& S = *reinterpret_cast<FbSmem*>(fb_smem);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(bar, 1u);
+    }
+}
+__device__ __forceinline__ bool grid_wait(unsigned* bar, unsigned k, int* stop)
+{
+    if (threadIdx.x == 0) {
+        const volatile unsigned* p = bar;
+        const unsigned want = k * gridDim.x;
+        const long long t0 = clock64();
+        *stop = 0;
+        while ((int)(*p - want) < 0) {
+            if (clock64() - t0 > kBarrierCycles) atomicExch(bar + 1, 1u);
+            if (p[1]) {
+                *stop = 1;
+                break;
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return *stop == 0;
+}
+
+// Features of the tile's samples, by the first kTrainRows threads.
+__device__ __forceinline__ void load_samples(const TrainArgs& a, FbSmem& S, long long first, long long end)
+{
     const int tid = threadIdx.x;
-    let_next_kernel_start();
-    // the samples do not depend on the weights: fetched while the last update runs
     if (tid < kTrainRows) {
-        const long long i = offset + (long long)blockIdx.x * kTrainRows + tid;
         float x[kWIn] = {};
         float y = 0.0f;
         bool valid = false;
-        if (i < offset + batch) {
-            const unsigned long long p = (perm_a * (unsigned long long)i + perm_b) % (unsigned long long)n;
-            valid = pair_features(pairs + p * kPairW, nm, x, &y);
+        if (first + tid < end) {
+            const unsigned long long p = (a.perm_a * (unsigned long long)(first + tid) + a.perm_b) % (unsigned long long)a.n;
+            valid = pair_features(a.pairs + p * kPairW, a.nm, x, &y);
             if (!valid)
                 for (int k = 0; k < kWIn; ++k) x[k] = 0.0f;
         }
@@ -159,39 +218,64 @@ __global__ void __launch_bounds__(kGemmThreads + kChoreThreads, 1)
         S.y[tid] = y;
         S.valid[tid] = valid;
     }
-    wait_previous_kernel();
-    // (the weights change between launches that overlap: plain loads past L1)
-    for (int i = tid; i < kP_B3; i += blockDim.x) {
-        const float v = __ldcg(prm + i);
-        if (i < kP_B1) S.w1[i / kWIn][i % kWIn] = v;
-        else if (i < kP_W2) S.b1[i - kP_B1] = v;
-        else if (i < kP_B2) {
-            const int j = (i - kP_W2) / kWHid, k = (i - kP_W2) % kWHid;
-            S.w2[j][k] = v;
-            S.w2t[k][j] = v;
-        } else if (i < kP_W3) S.b2[i - kP_B2] = v;
-        else S.w3[i - kP_W3] = v;
+}
+
+// The weights, past L1 (other blocks wrote them). Returns b3.
+__device__ __forceinline__ float load_weights(const float* prm, FbSmem& S)
+{
+    static_assert(kP_B1 % 4 == 0 && kP_W2 % 4 == 0 && kP_B2 % 4 == 0 && kP_W3 % 4 == 0 && kP_B3 % 4 == 0, "float4 groups");
+    constexpr int kThreads = kGemmThreads + kChoreThreads, kGroups = kP_B3 / 4, kEach = (kGroups + kThreads - 1) / kThreads;
+    float4 v[kEach];
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) {
+        const int i = threadIdx.x + q * kThreads;
+        if (i < kGroups) v[q] = __ldcg(reinterpret_cast<const float4*>(prm) + i);
     }
     const float b3 = __ldcg(prm + kP_B3);
+#pragma unroll
+    for (int q = 0; q < kEach; ++q) {
+        const int i = 4 * (threadIdx.x + q * kThreads);
+        if (i >= kP_B3) break;
+        float* dst = i < kP_B1   ? &S.w1[0][0] + i
+                     : i < kP_W2 ? S.b1 + (i - kP_B1)
+                     : i < kP_B2 ? &S.w2[(i - kP_W2) / kWHid][(i - kP_W2) % kWHid]
+                     : i < kP_W3 ? S.b2 + (i - kP_B2)
+                                 : S.w3 + (i - kP_W3);
+        *reinterpret_cast<float4*>(dst) = v[q];
+    }
+    return b3;
+}
+
+// One tile: forward and backward; gradient to gp, losses to sq_err (the samples,
+// the weights and b3 are in place; ends without a barrier).
+__device__ __forceinline__ void train_tile(FbSmem& S, float b3, float inv_batch, float* gp, float* sq_err)
+{
+    const int tid = threadIdx.x;
     __syncthreads();
-    float* gp = part + (size_t)blockIdx.x * kPartLd;
     const bool gemm = tid < kGemmThreads;
-    const int u0 = (tid / 16) * 4, v0 = (tid % 16) * 4;   // this thread's tile
-    float d1[4][4], d2[4][4];                             // SiLU' of layer 1 and 2 (sample, unit)
+    const int u0 = (tid / 16) * 4, tx = tid % 16;   // this thread's samples u0 .. u0 + 3, units tx, tx + 16, ...
+    float d1[4][4], d2[4][4];                       // SiLU' of layer 1 and 2 (sample, unit)
     if (gemm) {
         // layer 1
+        float x[4][kWIn];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int k = 0; k < kWIn; k += 4) load4(&S.x[u0 + i][k], *reinterpret_cast<float(*)[4]>(&x[i][k]));
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            float a[4];
+            const int unit = tx + 16 * j;
+            float w[kWIn];
+#pragma unroll
+            for (int k = 0; k < kWIn; k += 4) load4(&S.w1[unit][k], *reinterpret_cast<float(*)[4]>(&w[k]));
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                float z = S.b1[v0 + j];
+                float z = S.b1[unit], a;
 #pragma unroll
-                for (int k = 0; k < kWIn; ++k) z += S.w1[v0 + j][k] * S.x[u0 + i][k];
-                silu_both(z, &a[i], &d1[i][j]);
-                S.a1[u0 + i][v0 + j] = a[i];
+                for (int k = 0; k < kWIn; ++k) z += w[k] * x[i][k];
+                silu_both(z, &a, &d1[i][j]);
+                S.a1[u0 + i][unit] = a;
             }
-            *reinterpret_cast<float4*>(&S.a1t[v0 + j][u0]) = make_float4(a[0], a[1], a[2], a[3]);
         }
     }
     __syncthreads();
@@ -201,16 +285,28 @@ __global__ void __launch_bounds__(kGemmThreads + kChoreThreads, 1)
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[i][j] = S.b2[v0 + j];
-#pragma unroll 8
-        for (int k = 0; k < kWHid; ++k) tile_step(acc, &S.a1t[k][u0], &S.w2t[k][v0]);
+            for (int j = 0; j < 4; ++j) acc[i][j] = S.b2[tx + 16 * j];
+#pragma unroll 4
+        for (int k = 0; k < kWHid; k += 4) {
+            float u[4][4], v[4][4];   // [row][k]
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                load4(&S.a1[u0 + i][k], u[i]);
+                load4(&S.w2[tx + 16 * i][k], v[i]);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float uq[4] = {u[0][q], u[1][q], u[2][q], u[3][q]}, vq[4] = {v[0][q], v[1][q], v[2][q], v[3][q]};
+                tile_step(acc, uq, vq);
+            }
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 float a;
                 silu_both(acc[i][j], &a, &d2[i][j]);
-                S.a2[u0 + i][v0 + j] = a;
+                S.a2[u0 + i][tx + 16 * j] = a;
             }
     }
     __syncthreads();
@@ -220,42 +316,51 @@ __global__ void __launch_bounds__(kGemmThreads + kChoreThreads, 1)
         for (int j = 0; j < kWHid; ++j) out += S.w3[j] * S.a2[tid][j];
         const float err = S.valid[tid] ? (out - S.y[tid]) : 0.0f;
         S.g[tid] = err * inv_batch;  // loss = sum(err^2) / (2 batch)
-        S.e[tid] = 0.5f * err * err;
+        sq_err[tid] = 0.5f * err * err;
     }
     __syncthreads();
     if (gemm) {
-        float t[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) t[i][j] = S.g[u0 + i] * S.w3[v0 + j] * d2[i][j];
-            *reinterpret_cast<float4*>(&S.dz2[u0 + i][v0]) = make_float4(t[i][0], t[i][1], t[i][2], t[i][3]);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            *reinterpret_cast<float4*>(&S.dz2t[v0 + j][u0]) = make_float4(t[0][j], t[1][j], t[2][j], t[3][j]);
-    }
-    __syncthreads();
-    if (gemm) {
-        // dW2[j][k] = sum_s dZ2[s][j] a1[s][k]
-        float acc[4][4] = {};
-#pragma unroll 8
-        for (int s = 0; s < kTrainRows; ++s) tile_step(acc, &S.dz2[s][u0], &S.a1[s][v0]);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-            *reinterpret_cast<float4*>(gp + kP_W2 + (u0 + i) * kWHid + v0) =
-                make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) S.dz2[u0 + i][tx + 16 * j] = S.g[u0 + i] * S.w3[tx + 16 * j] * d2[i][j];
+    }
+    __syncthreads();
+    if (gemm) {
         // dA1[s][k] = sum_j W2[j][k] dZ2[s][j]
+        float acc[4][4] = {};
+#pragma unroll 4
+        for (int j = 0; j < kWHid; j += 4) {
+            float u[4][4];   // [sample][j]
+#pragma unroll
+            for (int i = 0; i < 4; ++i) load4(&S.dz2[u0 + i][j], u[i]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float uq[4] = {u[0][q], u[1][q], u[2][q], u[3][q]};
+                const float vq[4] = {S.w2[j + q][tx], S.w2[j + q][tx + 16], S.w2[j + q][tx + 32], S.w2[j + q][tx + 48]};
+                tile_step(acc, uq, vq);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) S.dz1[u0 + i][tx + 16 * j] = acc[i][j] * d1[i][j];
+        // dW2[j][k] = sum_s dZ2[s][j] a1[s][k]; units j = u0 .. u0 + 3, k = 4 tx .. 4 tx + 3
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
 #pragma unroll 8
-        for (int j = 0; j < kWHid; ++j) tile_step(acc, &S.dz2t[j][u0], &S.w2[j][v0]);
+        for (int s = 0; s < kTrainRows; ++s) {
+            float u[4], v[4];
+            load4(&S.dz2[s][u0], u);
+            load4(&S.a1[s][4 * tx], v);
+            tile_step(acc, u, v);
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) S.dz1[u0 + i][v0 + j] = acc[i][j] * d1[i][j];
+            *reinterpret_cast<float4*>(gp + kP_W2 + (u0 + i) * kWHid + 4 * tx) =
+                make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
     } else {
         const int c = tid - kGemmThreads;
         if (c < kWHid) {
@@ -272,13 +377,9 @@ __global__ void __launch_bounds__(kGemmThreads + kChoreThreads, 1)
         }
         if (c == 0) {
             float gb = 0.0f;
+#pragma unroll 16
             for (int s = 0; s < kTrainRows; ++s) gb += S.g[s];
             gp[kP_B3] = gb;
-        }
-        if (c == kWHid) {
-            double ls = 0.0;
-            for (int s = 0; s < kTrainRows; ++s) ls += (double)S.e[s];
-            loss_part[blockIdx.x] = ls;
         }
     }
     __syncthreads();
@@ -302,52 +403,101 @@ __global__ void __launch_bounds__(kGemmThreads + kChoreThreads, 1)
     }
 }
 
-// One AdamW step's constants; apply = 0: only the gradient is formed.
-struct AdamW {
-    float lr, b1, b2, eps, wd, c1, c2;
-    int apply;
-};
-
-// grad[i] = sum over blocks of part[b][i], blocks in order (their loads in flight
-// together), and the AdamW step of parameter i.
-constexpr int kUpdateThreads = 64, kUpdateBatch = 32;
-__global__ void __launch_bounds__(kUpdateThreads) warm_update_kernel(const float* part, int nblocks, float* __restrict__ grad,
-                                                                     float* prm, float* m, float* v, AdamW o)
+// The block's share of the parameters: gradient over the tiles in order, AdamW.
+__device__ __forceinline__ void update_share(const TrainArgs& a, FbSmem& S, int tiles, int step)
 {
-    let_next_kernel_start();
-    wait_previous_kernel();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= kNParams) return;
-    float g = 0.0f;
-    for (int b0 = 0; b0 < nblocks; b0 += kUpdateBatch) {
-        float t[kUpdateBatch];
+    const int c = threadIdx.x % kUpdateParams, row = threadIdx.x / kUpdateParams;
+    const int share = (kNParams + gridDim.x - 1) / gridDim.x;
+    const int end = min(kNParams, (int)(blockIdx.x + 1) * share);
+    for (int p0 = blockIdx.x * share; p0 < end; p0 += kUpdateParams) {
+        const int i = p0 + c;
+        float g = 0.0f;
+        for (int b0 = 0; b0 < tiles; b0 += kUpdateTiles) {
+            const int n = min(kUpdateTiles, tiles - b0);
+            __syncthreads();
+            if (i < end) {
 #pragma unroll
-        for (int b = 0; b < kUpdateBatch; ++b) t[b] = b0 + b < nblocks ? __ldcg(part + (size_t)(b0 + b) * kPartLd + i) : 0.0f;
-#pragma unroll
-        for (int b = 0; b < kUpdateBatch; ++b)
-            if (b0 + b < nblocks) g += t[b];
+                for (int b = row; b < kUpdateTiles; b += kUpdateRows)
+                    if (b < n) S.sums[b][c] = __ldcg(a.part + (size_t)(b0 + b) * kPartLd + i);
+            }
+            __syncthreads();
+            if (row == 0 && i < end) {
+                if (n == kUpdateTiles) {
+#pragma unroll 32
+                    for (int b = 0; b < kUpdateTiles; ++b) g += S.sums[b][c];
+                } else {
+                    for (int b = 0; b < n; ++b) g += S.sums[b][c];
+                }
+            }
+        }
+        if (row == 0 && i < end) {
+            a.grad[i] = g;
+            if (a.step) {
+                const AdamStep o = a.step[step];
+                const float mi = a.b1 * __ldcg(a.m + i) + (1.0f - a.b1) * g;
+                const float vi = a.b2 * __ldcg(a.v + i) + (1.0f - a.b2) * g * g;
+                __stcg(a.m + i, mi);
+                __stcg(a.v + i, vi);
+                const bool is_weight = (i < kP_B1) || (i >= kP_W2 && i < kP_B2) || (i >= kP_W3 && i < kP_B3);
+                float p = __ldcg(a.prm + i);
+                if (is_weight) p -= o.lr * a.wd * p;
+                p -= o.lr * (mi / o.c1) / (sqrtf(vi / o.c2) + a.eps);
+                __stcg(a.prm + i, p);
+            }
+        }
     }
-    grad[i] = g;
-    if (!o.apply) return;
-    // (launches overlap: what the one before wrote is read past L1)
-    const float mi = o.b1 * __ldcg(m + i) + (1.0f - o.b1) * g;
-    const float vi = o.b2 * __ldcg(v + i) + (1.0f - o.b2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    const bool is_weight = (i < kP_B1) || (i >= kP_W2 && i < kP_B2) || (i >= kP_W3 && i < kP_B3);
-    float p = __ldcg(prm + i);
-    if (is_weight) p -= o.lr * o.wd * p;
-    p -= o.lr * (mi / o.c1) / (sqrtf(vi / o.c2) + o.eps);
-    prm[i] = p;
 }
 
-// Loss of each step (its blocks in order), then *loss_acc += the steps in order.
-__global__ void __launch_bounds__(256) warm_loss_kernel(const double* __restrict__ loss_part, int nblocks, int steps,
+__global__ void __launch_bounds__(kGemmThreads + kChoreThreads, 1) warm_train_kernel(const TrainArgs a)
+{
+    extern __shared__ __align__(16) unsigned char fb_smem[];
+    FbSmem& S = *reinterpret_cast<FbSmem*>(fb_smem);
+    unsigned arrivals = 0;
+    for (int s = 0; s < a.steps; ++s) {
+        const long long off = a.offset + (long long)s * a.batch;
+        const long long end = min(off + a.batch, a.end);
+        const int tiles = (int)((end - off + kTrainRows - 1) / kTrainRows);
+        const float inv_batch = 1.0f / (float)(end - off);
+        // (the first tile's samples were fetched while the last update ran)
+        if (s == 0) load_samples(a, S, off + (long long)blockIdx.x * kTrainRows, end);
+        const float b3 = load_weights(a.prm, S);
+        for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+            if (t != (int)blockIdx.x) {
+                __syncthreads();
+                load_samples(a, S, off + (long long)t * kTrainRows, end);
+            }
+            train_tile(S, b3, inv_batch, a.part + (size_t)t * kPartLd, a.sq_err + (size_t)s * a.batch + (size_t)t * kTrainRows);
+        }
+        grid_arrive(a.barrier);
+        if (s + 1 < a.steps)
+            load_samples(a, S, off + a.batch + (long long)blockIdx.x * kTrainRows, min(off + 2ll * a.batch, a.end));
+        if (!grid_wait(a.barrier, ++arrivals, &S.stop)) return;
+        update_share(a, S, tiles, s);
+        if (s + 1 < a.steps) {
+            grid_arrive(a.barrier);
+            if (!grid_wait(a.barrier, ++arrivals, &S.stop)) return;
+        }
+    }
+}
+
+// Sums of (err^2)/2 in double, in a fixed order: per block of 64 samples, per step
+// over its blocks, then *loss_acc += the steps in order.
+__global__ void __launch_bounds__(128) warm_block_loss_kernel(const float* __restrict__ sq_err, long long blocks,
+                                                              double* __restrict__ block_loss)
+{
+    const long long b = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (b >= blocks) return;
+    double l = 0.0;
+    for (int s = 0; s < kTrainRows; ++s) l += (double)sq_err[b * kTrainRows + s];
+    block_loss[b] = l;
+}
+
+__global__ void __launch_bounds__(256) warm_loss_kernel(const double* __restrict__ block_loss, int nblocks, int steps,
                                                         double* __restrict__ step_loss, double* __restrict__ loss_acc)
 {
     for (int s = threadIdx.x; s < steps; s += blockDim.x) {
         double l = 0.0;
-        for (int b = 0; b < nblocks; ++b) l += loss_part[(size_t)s * nblocks + b];
+        for (int b = 0; b < nblocks; ++b) l += block_loss[(size_t)s * nblocks + b];
         step_loss[s] = l;
     }
     __syncthreads();
@@ -444,14 +594,17 @@ struct troute_warm {
     float *d_b1 = nullptr, *d_b2 = nullptr;
     double *d_loss = nullptr, *d_mom = nullptr;
     float* d_part = nullptr;
-    double* d_lpart = nullptr;
+    double* d_lpart = nullptr;   // block and step losses
+    float* d_err = nullptr;      // (err^2)/2 of the samples of the steps kept
+    unsigned* d_bar = nullptr;   // grid barrier
+    AdamStep* d_step = nullptr;  // AdamW constants of the steps kept
     int part_blocks = 0;
     size_t lpart_n = 0;
 
     ~troute_warm()
     {
         for (void* p : {(void*)d_prm, (void*)d_m, (void*)d_v, (void*)d_g, (void*)d_w1t, (void*)d_w2t, (void*)d_w3t,
-                        (void*)d_b1, (void*)d_b2, (void*)d_loss, (void*)d_mom, (void*)d_part, (void*)d_lpart})
+                        (void*)d_b1, (void*)d_b2, (void*)d_loss, (void*)d_mom, (void*)d_part, (void*)d_lpart, (void*)d_err, (void*)d_bar, (void*)d_step})
             if (p) cudaFree(p);
     }
 };
@@ -477,6 +630,7 @@ static int warm_alloc(troute_warm* w)
         (rc = warm_cuda(cudaMalloc(&w->d_b1, kWHid * sizeof(float)), "cudaMalloc")) ||
         (rc = warm_cuda(cudaMalloc(&w->d_b2, kWHid * sizeof(float)), "cudaMalloc")) ||
         (rc = warm_cuda(cudaMalloc(&w->d_loss, sizeof(double)), "cudaMalloc")) ||
+        (rc = warm_cuda(cudaMalloc(&w->d_bar, 2 * sizeof(unsigned)), "cudaMalloc")) ||
         (rc = warm_cuda(cudaMalloc(&w->d_mom, (size_t)kMomBlocks * kMomW * sizeof(double)), "cudaMalloc")))
         return rc;
     return TROUTE_OK;
@@ -497,49 +651,75 @@ static int warm_parts(troute_warm* w, int nblocks, int steps)
     const size_t need = (size_t)steps * ((size_t)nblocks + 1);
     if (need > w->lpart_n) {
         if (w->d_lpart) cudaFree(w->d_lpart);
+        if (w->d_err) cudaFree(w->d_err);
+        if (w->d_step) cudaFree(w->d_step);
         w->d_lpart = nullptr;
+        w->d_err = nullptr;
+        w->d_step = nullptr;
         w->lpart_n = 0;
-        if ((rc = warm_cuda(cudaMalloc(&w->d_lpart, need * sizeof(double)), "cudaMalloc"))) return rc;
+        if ((rc = warm_cuda(cudaMalloc(&w->d_lpart, need * sizeof(double)), "cudaMalloc")) ||
+            (rc = warm_cuda(cudaMalloc(&w->d_err, (size_t)steps * nblocks * kTrainRows * sizeof(float)), "cudaMalloc")) ||
+            (rc = warm_cuda(cudaMalloc(&w->d_step, (size_t)steps * sizeof(AdamStep)), "cudaMalloc")))
+            return rc;
         w->lpart_n = need;
     }
     return TROUTE_OK;
 }
 
-// Launches kernel so that it may start (up to its wait) while the one before it on
-// the stream still runs.
-template <class... P, class... A>
-static cudaError_t launch_overlapped(void (*kernel)(P...), int blocks, int threads, size_t smem, A... args)
+// Adds the losses of `steps` steps of `tiles` tiles each (their samples from
+// sq_err on) to *d_loss.
+static int warm_add_losses(troute_warm* w, const float* sq_err, int tiles, int steps)
 {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    const long long blocks = (long long)tiles * steps;
+    warm_block_loss_kernel<<<(unsigned)((blocks + 127) / 128), 128>>>(sq_err, blocks, w->d_lpart);
+    warm_loss_kernel<<<1, 256>>>(w->d_lpart, tiles, steps, w->d_lpart + blocks, w->d_loss);
+    return warm_cuda(cudaGetLastError(), "loss launch");
 }
 
-static int warm_fb_attr()
+// The steps of a (a.steps of them, a.batch samples each but the last) and their
+// losses. The tiles of a batch are shared out over as many blocks as fit the GPU.
+static int warm_train(troute_warm* w, TrainArgs& a)
 {
-    return warm_cuda(cudaFuncSetAttribute(warm_fb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FbSmem)),
-                     "smem attribute");
+    int rc, dev = 0, sms = 0, bps = 0;
+    const int tiles = (a.batch + kTrainRows - 1) / kTrainRows;
+    if ((rc = warm_cuda(cudaGetDevice(&dev), "cudaGetDevice")) ||
+        (rc = warm_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr")) ||
+        (rc = warm_cuda(cudaFuncSetAttribute(warm_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FbSmem)),
+                        "smem attribute")) ||
+        (rc = warm_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, warm_train_kernel, kGemmThreads + kChoreThreads,
+                                                                      sizeof(FbSmem)),
+                        "occupancy")))
+        return rc;
+    a.nm = w->nm;
+    a.prm = w->d_prm;
+    a.grad = w->d_g;
+    a.m = w->d_m;
+    a.v = w->d_v;
+    a.part = w->d_part;
+    a.sq_err = w->d_err;
+    a.barrier = w->d_bar;
+    if ((rc = warm_cuda(cudaMemsetAsync(w->d_bar, 0, 2 * sizeof(unsigned), nullptr), "memset"))) return rc;
+    void* args[] = {&a};
+    if ((rc = warm_cuda(cudaLaunchCooperativeKernel((const void*)warm_train_kernel, dim3(std::min(tiles, sms * std::max(1, bps))),
+                                                    dim3(kGemmThreads + kChoreThreads), args, sizeof(FbSmem), nullptr),
+                        "training launch")))
+        return rc;
+    // a last, shorter batch is summed on its own
+    const long long last = std::min<long long>(a.batch, a.end - a.offset - (long long)(a.steps - 1) * a.batch);
+    const int last_tiles = (int)((last + kTrainRows - 1) / kTrainRows);
+    const int full = last_tiles == tiles ? a.steps : a.steps - 1;
+    if (full && (rc = warm_add_losses(w, w->d_err, tiles, full))) return rc;
+    if (full < a.steps && (rc = warm_add_losses(w, w->d_err + (size_t)full * a.batch, last_tiles, 1))) return rc;
+    return TROUTE_OK;
 }
 
-// One mini-batch: gradient into d_g, AdamW step o, block losses into lpart.
-static int warm_step(troute_warm* w, const float* pairs, long long n, long long off, int b, unsigned long long pa,
-                     unsigned long long pb, float inv_batch, const AdamW& o, double* lpart)
+// Whether a barrier of the training launches ran out.
+static int warm_train_status(troute_warm* w)
 {
-    const int nblocks = (b + kTrainRows - 1) / kTrainRows;
-    const int rc = warm_cuda(launch_overlapped(warm_fb_kernel, nblocks, kGemmThreads + kChoreThreads, sizeof(FbSmem), pairs, n,
-                                               off, b, pa, pb, w->d_prm, w->nm, w->d_part, lpart, inv_batch),
-                             "training launch");
+    unsigned b[2] = {0, 0};
+    const int rc = warm_cuda(cudaMemcpy(b, w->d_bar, sizeof b, cudaMemcpyDeviceToHost), "training");
     if (rc) return rc;
-    return warm_cuda(launch_overlapped(warm_update_kernel, (kNParams + kUpdateThreads - 1) / kUpdateThreads, kUpdateThreads, 0,
-                                       w->d_part, nblocks, w->d_g, w->d_prm, w->d_m, w->d_v, o),
-                     "update launch");
+    return b[1] ? set_error(TROUTE_ETIMEOUT, "training: a grid barrier ran out") : TROUTE_OK;
 }
 
 // Rounds the fp32 weights to the bf16, transposed, padded layout of the MMA path.
@@ -699,52 +879,46 @@ extern "C" int troute_warm_fit(troute_warm* w, const float* pairs_dev, long long
         (rc = warm_cuda(cudaMemset(w->d_m, 0, kNParams * sizeof(float)), "memset")) ||
         (rc = warm_cuda(cudaMemset(w->d_v, 0, kNParams * sizeof(float)), "memset")))
         return rc;
-    if ((rc = warm_fb_attr())) return rc;
     const long long steps_per_epoch = (n_pairs + batch - 1) / batch;
     const long long total = steps_per_epoch * epochs;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    // block losses are kept for a run of steps and summed together: one thread's
-    // sum of 128 doubles takes longer than a whole update
-    const int full_blocks = batch / kTrainRows;
-    const int keep = (int)std::min<long long>(steps_per_epoch, std::max(1, (1 << 22) / (full_blocks + 1)));
-    if ((rc = warm_parts(w, full_blocks, keep))) return rc;
-    double* const step_loss = w->d_lpart + (size_t)keep * full_blocks;
+    // steps per launch: their samples' losses are kept and summed afterwards (64
+    // doubles in order take as long as a tile's products)
+    const int tiles = batch / kTrainRows;
+    const int keep = (int)std::min<long long>(steps_per_epoch, std::max(1, (1 << 16) / tiles));
+    if ((rc = warm_parts(w, tiles, keep))) return rc;
+    std::vector<AdamStep> consts((size_t)keep);
     long long step = 0;
     for (int ep = 0; ep < epochs; ++ep) {
-        const unsigned long long pa = coprime_near((unsigned long long)n_pairs, hash3(seed, 31, ep) | 1ull);
-        const unsigned long long pb = hash3(seed, 37, ep) % (unsigned long long)n_pairs;
+        TrainArgs a = {};
+        a.pairs = pairs_dev;
+        a.n = n_pairs;
+        a.end = n_pairs;
+        a.batch = batch;
+        a.perm_a = coprime_near((unsigned long long)n_pairs, hash3(seed, 31, ep) | 1ull);
+        a.perm_b = hash3(seed, 37, ep) % (unsigned long long)n_pairs;
+        a.step = w->d_step;
+        a.b1 = b1;
+        a.b2 = b2;
+        a.eps = eps;
+        a.wd = weight_decay;
         if ((rc = warm_cuda(cudaMemset(w->d_loss, 0, sizeof(double)), "memset"))) return rc;
-        int kept = 0;
-        for (long long s = 0; s < steps_per_epoch; ++s, ++step) {
-            const long long off = s * batch;
-            const int b = (int)std::min<long long>(batch, n_pairs - off);
-            // cosine decay of the step size
-            const float frac = (float)step / (float)std::max<long long>(1, total - 1);
-            AdamW o;
-            o.lr = lr * 0.5f * (1.0f + std::cos(3.14159265f * frac));
-            o.c1 = 1.0f - std::pow(b1, (float)(step + 1));
-            o.c2 = 1.0f - std::pow(b2, (float)(step + 1));
-            o.b1 = b1;
-            o.b2 = b2;
-            o.eps = eps;
-            o.wd = weight_decay;
-            o.apply = 1;
-            const int nblocks = (b + kTrainRows - 1) / kTrainRows;
-            // (a last, smaller batch is summed on its own: its rows are shorter)
-            if (kept == keep || (kept && nblocks != full_blocks)) {
-                warm_loss_kernel<<<1, 256>>>(w->d_lpart, full_blocks, kept, step_loss, w->d_loss);
-                kept = 0;
+        for (long long s = 0; s < steps_per_epoch; s += keep) {
+            a.offset = s * batch;
+            a.steps = (int)std::min<long long>(keep, steps_per_epoch - s);
+            for (int k = 0; k < a.steps; ++k, ++step) {
+                // cosine decay of the step size
+                const float frac = (float)step / (float)std::max<long long>(1, total - 1);
+                consts[k].lr = lr * 0.5f * (1.0f + std::cos(3.14159265f * frac));
+                consts[k].c1 = 1.0f - std::pow(b1, (float)(step + 1));
+                consts[k].c2 = 1.0f - std::pow(b2, (float)(step + 1));
             }
-            if ((rc = warm_step(w, pairs_dev, n_pairs, off, b, pa, pb, 1.0f / (float)b, o,
-                                w->d_lpart + (size_t)kept * full_blocks)))
+            // (a pageable copy: ordered after the launch before, and done when it returns)
+            if ((rc = warm_cuda(cudaMemcpy(w->d_step, consts.data(), (size_t)a.steps * sizeof(AdamStep), cudaMemcpyHostToDevice),
+                                "step constants")) ||
+                (rc = warm_train(w, a)) || (rc = warm_train_status(w)))
                 return rc;
-            ++kept;
-            if (nblocks != full_blocks) {
-                warm_loss_kernel<<<1, 256>>>(w->d_lpart, nblocks, 1, step_loss, w->d_loss);
-                kept = 0;
-            }
         }
-        if (kept) warm_loss_kernel<<<1, 256>>>(w->d_lpart, full_blocks, kept, step_loss, w->d_loss);
         double loss = 0.0;
         if ((rc = warm_cuda(cudaMemcpy(&loss, w->d_loss, sizeof(double), cudaMemcpyDeviceToHost), "loss"))) return rc;
         // each step's loss is sum(err^2)/2 over its batch: the epoch mean per pair
@@ -766,14 +940,16 @@ extern "C" int troute_warm_grad(troute_warm* w, const float* pairs_host, int n, 
     rc = warm_cuda(cudaMemcpy(d_pairs, pairs_host, (size_t)n * kPairW * sizeof(float), cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = warm_cuda(cudaMemcpy(w->d_prm, w->prm, sizeof w->prm, cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = warm_cuda(cudaMemset(w->d_loss, 0, sizeof(double)), "memset");
-    if (!rc) rc = warm_fb_attr();
-    const int nblocks = (n + kTrainRows - 1) / kTrainRows;
-    if (!rc) rc = warm_parts(w, nblocks, 1);
-    if (!rc) rc = warm_step(w, d_pairs, n, 0, n, 1, 0, 1.0f / (float)n, AdamW{}, w->d_lpart);
-    if (!rc) {
-        warm_loss_kernel<<<1, 256>>>(w->d_lpart, nblocks, 1, w->d_lpart + nblocks, w->d_loss);
-        rc = warm_cuda(cudaGetLastError(), "loss launch");
-    }
+    if (!rc) rc = warm_parts(w, (n + kTrainRows - 1) / kTrainRows, 1);
+    TrainArgs a = {};
+    a.pairs = d_pairs;
+    a.n = n;
+    a.end = n;
+    a.batch = n;
+    a.steps = 1;
+    a.perm_a = 1;
+    if (!rc) rc = warm_train(w, a);
+    if (!rc) rc = warm_train_status(w);
     if (!rc) rc = warm_cuda(cudaMemcpy(grad_out, w->d_g, kNParams * sizeof(float), cudaMemcpyDeviceToHost), "D2H");
     double loss = 0.0;
     if (!rc) rc = warm_cuda(cudaMemcpy(&loss, w->d_loss, sizeof(double), cudaMemcpyDeviceToHost), "D2H");
