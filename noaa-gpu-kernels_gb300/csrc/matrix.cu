@@ -24,29 +24,29 @@
 // reference's float operations in its order, so the matrices are bit for bit
 // the reference's given the same coefficients.
 //
-// Step (device): y[r] = sum_k P_Q[r,k] x[k] + sum_k P_q[r,k] ql[k]. The step
-// is HBM-bound (8 bytes per stored entry, each entry a (column, value) pair
-// read by one streaming load; the ~4 MB vectors stay in L2). The sum keeps the
+// Step (device): y[r] = sum_k P_Q[r,k] x[k] + sum_k P_q[r,k] ql[k]. Each stored
+// entry is a (column, value) pair read by one streaming load. The sum keeps the
 // reference kernel's arithmetic exactly (kernel_spmv_fused,
 // linear_mc_matrix_graph.cu:174-206: lane l of 32 accumulates entries l,
 // l + 32, ... of each matrix by fused multiply-add, adds the two partials,
 // then the shuffle-down tree 16, 8, 4, 2, 1). Row lengths are heavily skewed
-// (on a 1.1 M-reach network the median row holds 1 entry, 14 % of rows hold
-// more than 32 and those hold 80 % of the entries), so rows take one of two
-// paths:
-//  - short rows (at most 32 entries in each matrix) by 4 lanes: lane p holds
-//    the reference's lanes p, p + 4, ..., p + 28, performs the tree's first
-//    three levels (offsets 16, 8, 4) in registers in the same pairing and the
-//    last two by shuffles in its 4-lane group; a warp covers 8 rows;
-//  - long rows by the whole warp, lane l being the reference's lane l, each
-//    lane issuing the loads of several of its entries before it gathers and
-//    adds them, so a row of hundreds of entries costs a few memory round
-//    trips instead of one per entry.
-// Blocks of 64 threads: a block's slot frees as soon as its two warps finish,
-// so warps held up by long rows do not keep idle warps resident. (Measured
-// on a 1.1 M-reach network, 144 steps: 8 lanes per short row in blocks of
-// 256 22.5 ms, 4 lanes in blocks of 128 16.4 ms, of 64 15.9 ms; 2 lanes
-// 23.6 ms; 8 entries per lane and batch on long rows instead of 4 slower.)
+// (on a 400,001-reach network half of the rows hold 1 entry, 14 % hold more than
+// 32 and those hold 80 % of the entries), so the rows are listed by length when
+// the matrices are built, and a persistent grid takes them from the list:
+//  - long rows (more than 32 entries in a matrix), one warp each, lane l being the
+//    reference's lane l; a batch of the next entries, of the row or of the warp's
+//    next one, is in flight while the current one gathers and adds;
+//  - short rows by class (at most 1, 4, 8, 16, 32 entries), one, two or four lanes
+//    to a row: a lane holds several of the reference's and performs the tree's
+//    levels between them in registers in the same pairing, the rest by shuffles.
+// Every lane so has work that its row needs; with four lanes and sixteen slots for
+// every short row and long rows found among them by ballot, a step took 28 M warp
+// instructions for 14.6 M entries, now 14 M. A step starts while the one before it
+// ends, with its first rows and entries already on their way. 400,001 reaches, 48
+// steps: 1,753 -> 1,270 us. What bounds it now: the L1 passes of the gathers (38 k
+// of 50 k cycles; a load of 32 columns touches 8 lines) and the 117 MB of entries
+// (17 us of 26 us a step at the copy rate). (Blocks per SM: 3 1,379 us, 4 1,269, 5
+// 1,319; entries kept in L1 1,416; batches of 2 1,302, of 6 1,357.)
 //
 // A run of n_ts steps is recorded once as a CUDA graph of n_ts launches
 // (alternating two discharge buffers) and replayed while the caller's
@@ -66,20 +66,13 @@ namespace tr {
 namespace {
 
 constexpr unsigned kFullMask = 0xffffffffu;
-#ifndef TROUTE_MAT_THREADS
-#define TROUTE_MAT_THREADS 64
-#endif
-#ifndef TROUTE_MAT_LONG_BATCH
-#define TROUTE_MAT_LONG_BATCH 4
-#endif
-#ifndef TROUTE_MAT_LANES
-#define TROUTE_MAT_LANES 4
-#endif
-constexpr int kMatThreads = TROUTE_MAT_THREADS;
-constexpr int kLanesPerRow = TROUTE_MAT_LANES;   // lanes of a short row
-constexpr int kRefPerLane = 32 / kLanesPerRow;   // the reference's lanes each of them holds
-static_assert(kLanesPerRow >= 2 && kLanesPerRow <= 16 && 32 % kLanesPerRow == 0, "lanes per short row");
-constexpr int kRowsPerBlock = kMatThreads / kLanesPerRow;
+constexpr int kMatThreads = 256;
+constexpr int kMatBlocks = 4;   // resident blocks per SM
+// Classes of short rows by their longer matrix row: a row of class c holds at most
+// kClassMax[c] entries in either matrix and takes kClassLanes[c] lanes.
+constexpr int kClasses = 5;
+constexpr int kClassMax[kClasses] = {1, 4, 8, 16, 32};
+constexpr int kClassLanes[kClasses] = {1, 1, 1, 2, 4};
 
 // Coefficients of one reach at X = 0.25 (linear_mc_matrix.cu:56-86), FP32 in
 // the reference's operation order; powf / sqrtf are CUDA's.
@@ -112,127 +105,179 @@ __global__ void mat_coeff_kernel(const troute_chparams_f32* __restrict__ p, int 
 }
 
 struct MatDev {
-    int R;
-    const int* qp;     // P_Q row pointers [R + 1]
-    const int2* qe;    // P_Q entries: (column, value bits)
-    const int* lp;     // P_q row pointers [R + 1]
-    const int2* le;    // P_q entries
+    const int2 *qe, *le;        // entries (column, value bits) of P_Q and P_q, rows in reach order
+    // rows in the order a step takes them (their places in qe / le, not copies)
+    const int4* long_rows;      // row, first entry and entries in qe, first entry in le
+    const int* long_nl;         // entries in le
+    const int4* rows;           // short rows by class: row, first entries, entries | entries << 8
+    int n_long, n_items;
+    int first_item[kClasses], first_row[kClasses], n_rows[kClasses];
 };
 
-// A row whose two matrices hold at most this many entries each is summed by
-// a group of kLanesPerRow lanes (one entry per reference lane at most);
-// longer rows by the whole warp.
-constexpr int kShortRow = 32;
 // Entries a lane loads per matrix before it gathers and adds, on long rows.
-constexpr int kLongBatch = TROUTE_MAT_LONG_BATCH;
+constexpr int kLongBatch = 4;
 
 // Entries are read once per step: streaming loads, evicted first, so the
 // gathered discharge and inflow vectors keep their place in L2.
 __device__ __forceinline__ int2 ld_entry(const int2* __restrict__ e, int k) { return __ldcs(e + k); }
 
-// Sum of one long row by the whole warp: lane l is the reference's lane l
-// (entries l, l + 32, ... of each matrix, fused multiply-add from 0, the two
-// partials added, then the shuffle-down tree 16, 8, 4, 2, 1); each lane loads
-// kLongBatch entries of each matrix, then gathers them, then adds them in
-// order. Returns the row's value in lane 0.
-__device__ __forceinline__ float long_row(const MatDev& m, const float* __restrict__ x, const float* __restrict__ ql,
-                                          int lane, int qb, int nq, int lb, int nl)
+// The previous step's discharge. A step starts while the one before it runs, so
+// the vector is not constant over the kernel's life: no read-only load.
+__device__ __forceinline__ float ld_x(const float* x)
 {
-    float sq = 0.0f, sl = 0.0f;
-    const int n = max(nq, nl);
-    for (int k = lane; k < n; k += kLongBatch * 32) {
-        int2 eq[kLongBatch], el[kLongBatch];
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(x) : "memory");
+    return v;
+}
+
+// A lane's next kLongBatch entries of each matrix of a long row: of the rq / rl
+// entries from this lane's next one on that the row has left, every 32nd.
+struct LongBatch {
+    int2 q[kLongBatch], l[kLongBatch];
+    __device__ __forceinline__ void load(const int2* __restrict__ pq, const int2* __restrict__ pl, int rq, int rl)
+    {
 #pragma unroll
         for (int j = 0; j < kLongBatch; ++j) {
-            const int kk = k + 32 * j;
-            eq[j] = kk < nq ? ld_entry(m.qe, qb + kk) : make_int2(0, 0);
-            el[j] = kk < nl ? ld_entry(m.le, lb + kk) : make_int2(0, 0);
+            q[j] = 32 * j < rq ? ld_entry(pq, 32 * j) : make_int2(0, 0);
+            l[j] = 32 * j < rl ? ld_entry(pl, 32 * j) : make_int2(0, 0);
         }
+    }
+    // sq, sl: the reference lane's sums, entries in order by fused multiply-add
+    __device__ __forceinline__ void add(const float* x, const float* __restrict__ ql, int rq, int rl, float& sq,
+                                        float& sl) const
+    {
         float xq[kLongBatch], xl[kLongBatch];
 #pragma unroll
         for (int j = 0; j < kLongBatch; ++j) {
-            const int kk = k + 32 * j;
-            xq[j] = kk < nq ? __ldg(x + eq[j].x) : 0.0f;
-            xl[j] = kk < nl ? __ldg(ql + el[j].x) : 0.0f;
+            xq[j] = 32 * j < rq ? ld_x(x + q[j].x) : 0.0f;
+            xl[j] = 32 * j < rl ? __ldg(ql + l[j].x) : 0.0f;
         }
 #pragma unroll
         for (int j = 0; j < kLongBatch; ++j) {
-            const int kk = k + 32 * j;
-            if (kk < nq) sq = __fmaf_rn(__int_as_float(eq[j].y), xq[j], sq);
-            if (kk < nl) sl = __fmaf_rn(__int_as_float(el[j].y), xl[j], sl);
+            if (32 * j < rq) sq = __fmaf_rn(__int_as_float(q[j].y), xq[j], sq);
+            if (32 * j < rl) sl = __fmaf_rn(__int_as_float(l[j].y), xl[j], sl);
         }
     }
-    float u = __fadd_rn(sq, sl);
+};
+
+// The warp's rows of one class: kLanes lanes to a row of at most kMax entries in
+// each matrix. Lane p holds the reference's lanes p, p + kLanes, ...: every entry
+// load is issued before any gather, and every gather before any sum.
+template <int kMax, int kLanes>
+__device__ __forceinline__ void short_rows(const MatDev& m, const int4* __restrict__ rec, int n_rows, int item,
+                                           const float* x, const float* __restrict__ ql,
+                                           float* __restrict__ y, int lane)
+{
+    constexpr int kSlots = kMax / kLanes;
+    const int p = lane & (kLanes - 1);
+    const int at = item * (32 / kLanes) + lane / kLanes;
+    int4 r = make_int4(-1, 0, 0, 0);
+    if (at < n_rows) r = __ldg(rec + at);
+    const int nq = r.w & 0xff, nl = r.w >> 8;
+    int2 eq[kSlots], el[kSlots];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) u = __fadd_rn(u, __shfl_down_sync(kFullMask, u, off));
-    return u;
+    for (int j = 0; j < kSlots; ++j) {
+        const int k = p + kLanes * j;
+        eq[j] = k < nq ? ld_entry(m.qe, r.y + k) : make_int2(0, 0);
+        el[j] = k < nl ? ld_entry(m.le, r.z + k) : make_int2(0, 0);
+    }
+    float xq[kSlots], xl[kSlots];
+#pragma unroll
+    for (int j = 0; j < kSlots; ++j) {
+        const int k = p + kLanes * j;
+        xq[j] = k < nq ? ld_x(x + eq[j].x) : 0.0f;
+        xl[j] = k < nl ? __ldg(ql + el[j].x) : 0.0f;
+    }
+    float s[kSlots];
+#pragma unroll
+    for (int j = 0; j < kSlots; ++j) {
+        const int k = p + kLanes * j;
+        // fma(v, x, 0) where the lane holds an entry, 0 where it holds none
+        const float sq = k < nq ? __fmaf_rn(__int_as_float(eq[j].y), xq[j], 0.0f) : 0.0f;
+        const float sl = k < nl ? __fmaf_rn(__int_as_float(el[j].y), xl[j], 0.0f) : 0.0f;
+        s[j] = __fadd_rn(sq, sl);
+        // the reference's lanes from kMax on hold 0: the tree's levels 16 .. kMax add it
+        if (kMax < 32) s[j] = __fadd_rn(s[j], 0.0f);
+    }
+    // the levels kMax / 2 .. kLanes in registers: at offset o the reference's lane v
+    // adds lane v + o; slot j holds its lane p + kLanes j, so offset o adds slot
+    // j + o / kLanes onto j
+#pragma unroll
+    for (int h = kSlots / 2; h >= 1; h >>= 1)
+#pragma unroll
+        for (int j = 0; j < h; ++j) s[j] = __fadd_rn(s[j], s[j + h]);
+    // the remaining levels inside the row's lane group (every lane takes part)
+    float u = s[0];
+#pragma unroll
+    for (int off = kLanes / 2; off >= 1; off >>= 1) u = __fadd_rn(u, __shfl_down_sync(kFullMask, u, off, kLanes));
+    if (p == 0 && r.x >= 0) y[r.x] = u;
 }
 
-__global__ void __launch_bounds__(kMatThreads) mat_step_kernel(MatDev m, const float* __restrict__ x,
-                                                               const float* __restrict__ ql, float* __restrict__ y)
+// One step. The warps of the grid take items from the list in turn: a long row
+// each, longest first, then 32 / kClassLanes rows of a class each, longest first.
+__global__ void __launch_bounds__(kMatThreads, kMatBlocks) mat_step_kernel(MatDev m, const float* x,
+                                                                            const float* __restrict__ ql,
+                                                                            float* __restrict__ y)
 {
     const int lane = threadIdx.x & 31;
-    const int p = lane & (kLanesPerRow - 1);
-    const int row = blockIdx.x * kRowsPerBlock + threadIdx.x / kLanesPerRow;
-    int qb = 0, nq = 0, lb = 0, nl = 0;
-    if (row < m.R) {
-        qb = __ldg(m.qp + row);
-        nq = __ldg(m.qp + row + 1) - qb;
-        lb = __ldg(m.lp + row);
-        nl = __ldg(m.lp + row + 1) - lb;
+    const int n_warps = gridDim.x * (kMatThreads / 32);
+    int item = blockIdx.x * (kMatThreads / 32) + (threadIdx.x >> 5);
+    // Long rows: lane l is the reference's lane l (entries l, l + 32, ... of each
+    // matrix, the two partials added, then the shuffle-down tree 16, 8, 4, 2, 1).
+    // The entries of the next batch, of this row or the next, are in flight while
+    // this batch gathers and adds; those of the first while the previous step ends.
+    int4 a = make_int4(0, 0, 0, 0), a1 = a;   // this row and the warp's next one
+    int nl = 0, nl1 = 0;
+    if (item < m.n_long) a = __ldg(m.long_rows + item), nl = __ldg(m.long_nl + item);
+    if (item + n_warps < m.n_long) a1 = __ldg(m.long_rows + item + n_warps), nl1 = __ldg(m.long_nl + item + n_warps);
+    const int2 *pq = m.qe + a.y + lane, *pl = m.le + a.w + lane;
+    int rq = a.z - lane, rl = nl - lane;
+    LongBatch now;
+    now.load(pq, pl, rq, rl);
+    // from here on the previous step's discharge is read and its input overwritten
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
+    float sq = 0.0f, sl = 0.0f;
+    while (item < m.n_long) {
+        const bool last = max(rq, rl) + lane <= kLongBatch * 32;
+        const int rq0 = rq, rl0 = rl;
+        if (last) {
+            pq = m.qe + a1.y + lane, pl = m.le + a1.w + lane;
+            rq = a1.z - lane, rl = nl1 - lane;
+        } else {
+            pq += kLongBatch * 32, pl += kLongBatch * 32;
+            rq -= kLongBatch * 32, rl -= kLongBatch * 32;
+        }
+        LongBatch then;
+        then.load(pq, pl, rq, rl);
+        now.add(x, ql, rq0, rl0, sq, sl);
+        if (last) {
+            float u = __fadd_rn(sq, sl);
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) u = __fadd_rn(u, __shfl_down_sync(kFullMask, u, off));
+            if (lane == 0) y[a.x] = u;
+            sq = sl = 0.0f;
+            item += n_warps;
+            a = a1;
+            nl1 = 0;
+            a1 = make_int4(0, 0, 0, 0);
+            if (item + n_warps < m.n_long)
+                a1 = __ldg(m.long_rows + item + n_warps), nl1 = __ldg(m.long_nl + item + n_warps);
+        }
+        now = then;
     }
-    const bool is_long = nq > kShortRow || nl > kShortRow;
-    float u = 0.0f;
-    if (!is_long) {
-        // the entry of each of the reference's lanes p, p + kLanesPerRow, ...
-        // (a short row has no other): every entry load is issued before any
-        // gather, and every gather before any sum
-        int2 eq[kRefPerLane], el[kRefPerLane];
-#pragma unroll
-        for (int j = 0; j < kRefPerLane; ++j) {
-            const int k = p + kLanesPerRow * j;
-            eq[j] = k < nq ? ld_entry(m.qe, qb + k) : make_int2(0, 0);
-            el[j] = k < nl ? ld_entry(m.le, lb + k) : make_int2(0, 0);
+    for (; item < m.n_items; item += n_warps) {
+        int c = kClasses - 1;
+        while (c > 0 && item >= m.first_item[c - 1]) --c;   // classes are listed longest first
+        const int4* rec = m.rows + m.first_row[c];
+        const int n = m.n_rows[c], k = item - m.first_item[c];
+        switch (c) {
+            case 4: short_rows<32, 4>(m, rec, n, k, x, ql, y, lane); break;
+            case 3: short_rows<16, 2>(m, rec, n, k, x, ql, y, lane); break;
+            case 2: short_rows<8, 1>(m, rec, n, k, x, ql, y, lane); break;
+            case 1: short_rows<4, 1>(m, rec, n, k, x, ql, y, lane); break;
+            default: short_rows<1, 1>(m, rec, n, k, x, ql, y, lane); break;
         }
-        float xq[kRefPerLane], xl[kRefPerLane];
-#pragma unroll
-        for (int j = 0; j < kRefPerLane; ++j) {
-            const int k = p + kLanesPerRow * j;
-            xq[j] = k < nq ? __ldg(x + eq[j].x) : 0.0f;
-            xl[j] = k < nl ? __ldg(ql + el[j].x) : 0.0f;
-        }
-        float s[kRefPerLane];
-#pragma unroll
-        for (int j = 0; j < kRefPerLane; ++j) {
-            const int k = p + kLanesPerRow * j;
-            // fma(v, x, 0) where the lane holds an entry, 0 where it holds none
-            const float sq = k < nq ? __fmaf_rn(__int_as_float(eq[j].y), xq[j], 0.0f) : 0.0f;
-            const float sl = k < nl ? __fmaf_rn(__int_as_float(el[j].y), xl[j], 0.0f) : 0.0f;
-            s[j] = __fadd_rn(sq, sl);
-        }
-        // the reference's shuffle-down levels 16 .. kLanesPerRow in registers:
-        // at offset o its lane v adds lane v + o; slot j holds its lane
-        // p + kLanesPerRow j, so offset o adds slot j + o / kLanesPerRow onto j
-#pragma unroll
-        for (int h = kRefPerLane / 2; h >= 1; h >>= 1)
-#pragma unroll
-            for (int j = 0; j < h; ++j) s[j] = __fadd_rn(s[j], s[j + h]);
-        u = s[0];
-    }
-    // the remaining levels inside the row's lane group (every lane takes part)
-#pragma unroll
-    for (int off = kLanesPerRow / 2; off >= 1; off >>= 1)
-        u = __fadd_rn(u, __shfl_down_sync(kFullMask, u, off, kLanesPerRow));
-    if (p == 0 && row < m.R && !is_long) y[row] = u;
-    // the warp's long rows, one after another, each by all 32 lanes
-    unsigned longs = __ballot_sync(kFullMask, is_long && p == 0);
-    while (longs) {
-        const int src = __ffs(longs) - 1;
-        longs &= longs - 1;
-        const int r = __shfl_sync(kFullMask, row, src);
-        const float v = long_row(m, x, ql, lane, __shfl_sync(kFullMask, qb, src), __shfl_sync(kFullMask, nq, src),
-                                 __shfl_sync(kFullMask, lb, src), __shfl_sync(kFullMask, nl, src));
-        if (lane == 0) y[r] = v;
     }
 }
 
@@ -399,7 +444,10 @@ struct troute_matrix {
     const float* g_qlat = nullptr;
     float* g_q = nullptr;
     int g_nts = 0;
-    MatDev dev() const { return MatDev{R, qp.p, qe.p, lp.p, le.p}; }
+    MArr<int4> long_rows, rows;
+    MArr<int> long_nl;
+    MatDev d{};   // the step's view of the above
+    int grid = 0;
     ~troute_matrix()
     {
         if (graph) cudaGraphExecDestroy(graph);
@@ -480,22 +528,70 @@ extern "C" int troute_matrix_create(troute_matrix** out, int n_reaches, const in
         }
         return e;
     };
+    // The step's rows: long ones by powers of two of their length, longest first and
+    // in reach order within one (whose columns overlap), then the short classes.
+    std::vector<int4> longs, shorts;
+    std::vector<int> longs_nl;
+    auto list_rows = [&] {
+        constexpr int kShort = kClassMax[kClasses - 1];
+        std::vector<int> of_class[kClasses], of_log[32];
+        for (int r = 0; r < n_reaches; ++r) {
+            const int n = std::max(PQ.ptr[r + 1] - PQ.ptr[r], Pq.ptr[r + 1] - Pq.ptr[r]);
+            if (n > kShort) {
+                of_log[31 - __builtin_clz((unsigned)n)].push_back(r);
+            } else {
+                int c = 0;
+                while (n > kClassMax[c]) ++c;
+                of_class[c].push_back(r);
+            }
+        }
+        for (int b = 31; b >= 0; --b)
+            for (const int r : of_log[b]) {
+                longs.push_back(make_int4(r, PQ.ptr[r], PQ.ptr[r + 1] - PQ.ptr[r], Pq.ptr[r]));
+                longs_nl.push_back(Pq.ptr[r + 1] - Pq.ptr[r]);
+            }
+        M->d.n_long = M->d.n_items = (int)longs.size();
+        for (int c = kClasses - 1; c >= 0; --c) {
+            M->d.first_item[c] = M->d.n_items;
+            M->d.first_row[c] = (int)shorts.size();
+            M->d.n_rows[c] = (int)of_class[c].size();
+            const int per_item = 32 / kClassLanes[c];
+            M->d.n_items += (M->d.n_rows[c] + per_item - 1) / per_item;
+            for (const int r : of_class[c])
+                shorts.push_back(make_int4(r, PQ.ptr[r], Pq.ptr[r],
+                                           (PQ.ptr[r + 1] - PQ.ptr[r]) | (Pq.ptr[r + 1] - Pq.ptr[r]) << 8));
+        }
+    };
     try {
+        list_rows();
         const std::vector<int2> eQ = pairs(PQ), eq = pairs(Pq);
         rc = mat_cuda(cudaStreamCreateWithFlags(&M->stream, cudaStreamNonBlocking), "stream");
         if (!rc && !(rc = M->qp.alloc(R1)) && !(rc = M->qe.alloc(eQ.size())) && !(rc = M->lp.alloc(R1)) &&
             !(rc = M->le.alloc(eq.size())) && !(rc = M->tmp.alloc((size_t)std::max(1, n_reaches))) &&
             !(rc = up(M->qp.p, PQ.ptr.data(), R1 * sizeof(int))) &&
             !(rc = up(M->qe.p, eQ.data(), eQ.size() * sizeof(int2))) &&
-            !(rc = up(M->lp.p, Pq.ptr.data(), R1 * sizeof(int))))
-            rc = up(M->le.p, eq.data(), eq.size() * sizeof(int2));
+            !(rc = up(M->lp.p, Pq.ptr.data(), R1 * sizeof(int))) &&
+            !(rc = up(M->le.p, eq.data(), eq.size() * sizeof(int2))) && !(rc = M->long_rows.alloc(longs.size())) &&
+            !(rc = M->long_nl.alloc(longs.size())) && !(rc = M->rows.alloc(shorts.size())) &&
+            !(rc = up(M->long_rows.p, longs.data(), longs.size() * sizeof(int4))) &&
+            !(rc = up(M->long_nl.p, longs_nl.data(), longs.size() * sizeof(int))))
+            rc = up(M->rows.p, shorts.data(), shorts.size() * sizeof(int4));
     } catch (const std::bad_alloc&) {
         rc = set_error(TROUTE_ENOMEM, "matrix upload: host memory");
     }
+    int dev = 0, sms = 0;
+    if (!rc) rc = mat_cuda(cudaGetDevice(&dev), "device");
+    if (!rc) rc = mat_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "device attribute");
     if (rc) {
         delete M;
         return rc;
     }
+    M->d.qe = M->qe.p;
+    M->d.le = M->le.p;
+    M->d.long_rows = M->long_rows.p;
+    M->d.long_nl = M->long_nl.p;
+    M->d.rows = M->rows.p;
+    M->grid = std::max(1, std::min(sms * kMatBlocks, (M->d.n_items + kMatThreads / 32 - 1) / (kMatThreads / 32)));
     *out = M;
     return TROUTE_OK;
 }
@@ -545,14 +641,22 @@ extern "C" int troute_matrix_get(const troute_matrix* M, int which, int* ptr, in
 // odd number of steps the result is copied back into the caller's buffer.
 static int enqueue_steps(troute_matrix* M, const float* qlat, int n_ts, float* q, cudaStream_t st)
 {
-    const int grid = (M->R + kRowsPerBlock - 1) / kRowsPerBlock;
-    const MatDev d = M->dev();
-    for (int t = 0; t < n_ts; ++t) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)M->grid);
+    cfg.blockDim = dim3(kMatThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute early = {};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &early;
+    int rc = TROUTE_OK;
+    for (int t = 0; t < n_ts && !rc; ++t) {
         const float* x = (t & 1) ? M->tmp.p : q;
         float* y = (t & 1) ? q : M->tmp.p;
-        mat_step_kernel<<<grid, kMatThreads, 0, st>>>(d, x, qlat + (size_t)t * (size_t)M->R, y);
+        cfg.numAttrs = t > 0;   // the first step waits for what was there before the run
+        rc = mat_cuda(cudaLaunchKernelEx(&cfg, mat_step_kernel, M->d, x, qlat + (size_t)t * (size_t)M->R, y),
+                      "matrix step launch");
     }
-    int rc = mat_cuda(cudaGetLastError(), "matrix step launch");
     if (!rc && (n_ts & 1))
         rc = mat_cuda(cudaMemcpyAsync(q, M->tmp.p, (size_t)M->R * sizeof(float), cudaMemcpyDeviceToDevice, st),
                       "matrix result copy");
