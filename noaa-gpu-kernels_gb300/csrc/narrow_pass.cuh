@@ -118,11 +118,22 @@ __device__ __forceinline__ QuadFlow quad_flow(int r, int quad, const PassFlow& f
     return o;
 }
 
-// The pass for the lanes of smask (at most kNarrow, none irregular). The whole
-// warp calls it; `warp_seg` is buffer 0 of the warp's lane 0. A lane of smask gets
-// o and its L.e0 (and what the next narrow pass starts from) as lane_eval leaves
-// them; returns whether it iterated (not after an exact evaluation at h_0 alone).
-__device__ __forceinline__ bool narrow_pass(Lane& L, unsigned smask, const RunDev& run, double2* warp_seg, PassOut& o)
+// Passes for the lanes of smask (at most kNarrow, none irregular) until one of the
+// solves needs its own lane again: it stops, starts a new attempt or the plain
+// bracket, or has a doubtful rounding. The whole warp calls it; `warp_seg` is
+// buffer 0 of the warp's lane 0. `leave(k)` is asked by every lane after pass k
+// (from 0) when all solves would go on; a lane's true ends the call too. A lane of
+// smask gets the last pass's o, its L.e0 (and what the next narrow pass starts from)
+// as lane_eval leaves them, and the passes before it booked in L; returns whether
+// the last one iterated (not after an exact evaluation at h_0 alone). extra: passes
+// before the last.
+//
+// Between its passes the state of a solve stays on its octet, and the loop around
+// (claims, item starts, publishing: 4 k cycles of a lone warp beside the pass's 8 k)
+// is not run. 200,000 segments, 24 steps: 121 -> 114 ms.
+template <typename Leave>
+__device__ __forceinline__ bool narrow_passes(Lane& L, unsigned smask, const RunDev& run, double2* warp_seg, PassOut& o,
+                                              int& extra, Leave leave)
 {
     const int lane = threadIdx.x & 31;
     const int r = lane & 3, quad = lane & ~3;
@@ -135,150 +146,204 @@ __device__ __forceinline__ bool narrow_pass(Lane& L, unsigned smask, const RunDe
     if (j > 1) m &= m - 1;
     if (j > 2) m &= m - 1;
     const int home = __ffs(m ? m : smask) - 1;
+    // passes after which the solve may go on: the warm phase has warm_k
+    const int room = (L.warm == W_ACTIVE ? run.warm_k - 1 : L.maxiter) - L.iter;
     const int flags = __shfl_sync(0xffffffffu, (L.i & 1) | (L.need0 << 1) | ((L.ahead ? 1 : 0) << 2), home);
-    const bool need0 = flags & 2, pre = !(flags & 4);
-    const double h = lane_get(L.h, home), h_0 = lane_get(L.h_0, home);
+    const int left = __shfl_sync(0xffffffffu, room, home);
+    bool need0 = flags & 2, pre = !(flags & 4);
+    double h = lane_get(L.h, home), h_0 = lane_get(L.h_0, home);
+    double q0n = lane_get(L.qmc0_n, home), Qj0n = lane_get(L.Qj0_n, home);
     const PassFlow f = {lane_get(L.qup, home), lane_get(L.quc, home), lane_get(L.qdp, home), lane_get(L.qldt, home), run.dt,
                         run.dt_half};
     const Opaque kc = opaque_constants();
-    const SegP p = staged_seg(warp_seg + home + (flags & 1) * kSegBufStride);
+    const double2* const rec = warp_seg + home + (flags & 1) * kSegBufStride;
+    // on quad A of a solve past its first pass here: what the pass before left
+    DepthEval e0 = {};
+    double Qj_before = 0.0;
+    int k = 0;
+    while (true) {
+        const SegP p = staged_seg(rec);
 
-    // ---- geometry ----
-    const double x = (B && need0) ? h_0 : h;
-    const bool wet = (__double2hiint(x) | __double2loint(x)) != 0;
-    bool unsure = !depth_regular(x);
-    const bool over = dbits(x) > dbits(p.bfd);
-    const double below = over ? p.bfd : x;
-    // depth above the bank; lane 3: h_0 - h for the secant step
-    const double diff = (r == 3 ? h_0 : x) - (r == 3 ? h : p.bfd);
-    // lane 0: WP, WP n; lane 1: A; lanes 2, 3: bw + 2 z x and its product with s0
-    double s1 = p.bw + (r < 2 ? below : p.z2) * (r == 0 ? p.sq2 : r == 1 ? p.z : x);
-    double w = s1 * (r == 0 ? p.n_ch : r == 1 ? below : p.s0);
-    if (__any_sync(0xffffffffu, over)) {
-        const double t1 = __fma_rn(r == 0 ? 2.0 : p.twcc, r >= 2 ? p.s0 : diff, r == 0 ? p.twcc : kc.neg_zero);
-        const double t2 = (r == 0 ? s1 : w) + t1;
-        const double t3 = w + t1 * p.ncc;
-        if (over) {
-            if (r == 0) s1 = t2, w = t3;
-            else w = r == 1 ? t2 : t1;
+        // ---- geometry ----
+        const double x = (B && need0) ? h_0 : h;
+        const bool wet = (__double2hiint(x) | __double2loint(x)) != 0;
+        bool unsure = !depth_regular(x);
+        const bool over = dbits(x) > dbits(p.bfd);
+        const double below = over ? p.bfd : x;
+        // depth above the bank; lane 3: h_0 - h for the secant step
+        const double diff = (r == 3 ? h_0 : x) - (r == 3 ? h : p.bfd);
+        // lane 0: WP, WP n; lane 1: A; lanes 2, 3: bw + 2 z x and its product with s0
+        double s1 = p.bw + (r < 2 ? below : p.z2) * (r == 0 ? p.sq2 : r == 1 ? p.z : x);
+        double w = s1 * (r == 0 ? p.n_ch : r == 1 ? below : p.s0);
+        if (__any_sync(0xffffffffu, over)) {
+            const double t1 = __fma_rn(r == 0 ? 2.0 : p.twcc, r >= 2 ? p.s0 : diff, r == 0 ? p.twcc : kc.neg_zero);
+            const double t2 = (r == 0 ? s1 : w) + t1;
+            const double t3 = w + t1 * p.ncc;
+            if (over) {
+                if (r == 0) s1 = t2, w = t3;
+                else w = r == 1 ? t2 : t1;
+            }
         }
-    }
-    const double P = lane_get(s1, quad), WPn = lane_get(w, quad);
-    // lane 1: R; lane 2: 2 sqrt(1+z^2) / (bw + 2 z x); lanes 0, 3: (WP n) / P
-    const double q1 = near_quot(r == 2 ? p.sq2 : r == 1 ? w : WPn, near_rcp(r == 2 ? s1 : P), unsure);
-    const double z = pow_near_one(lane_get(q1, quad | 1), r & 1, kc, unsure);
-    const double r23 = lane_get(z, quad);
-    const double sqt = lane_get(q1, quad | 2);
-    const double v = z * ((r & 1) ? 2.0 / 3.0 : 5.0 / 3.0) * ((r & 1) ? sqt : kc.one);
-    const double u = __shfl_xor_sync(0xffffffffu, v, 1);
-    const double Ck = p.ck_fac * (((r & 1) ? u : v) - ((r & 1) ? v : u));
-    const bool moves = wet && __double2hiint(Ck) > 0;
-    // lane 1: dx / Ck; lanes 0, 3: 1 / ((WP n) / P); lane 2: G = 2 tw s0 Ck dx, 1 / G
-    double G, yG, Km, it;
-    {
-        const bool g2 = r == 2;
-        const double b = r == 1 ? Ck : q1;
-        const double y0 = rcp_seed(b);
-        const double e1 = __fma_rn(g2 ? w : -b, g2 ? Ck : y0, g2 ? kc.neg_zero : kc.one);
-        const double e2 = __fma_rn(e1, g2 ? p.dx : e1, g2 ? kc.neg_zero : e1);
-        const double y = __fma_rn(y0, e2, y0);
-        G = __hiloint2double(__double2hiint(e2) + (1 << 20), __double2loint(e2));
-        const double yg0 = rcp_seed(G);
-        const double q0 = __fma_rn(g2 ? -G : (r == 1 ? p.dx : kc.one), g2 ? yg0 : y, g2 ? kc.one : kc.neg_zero);
-        const double rr = __fma_rn(g2 ? q0 : -b, q0, g2 ? q0 : (r == 1 ? p.dx : kc.one));
-        const double qq = __fma_rn(g2 ? yg0 : rr, g2 ? rr : y, g2 ? yg0 : q0);
-        unsure |= !g2 & (moves | (r != 1)) & quot_doubt(b, q0, rr);
-        it = qq;
-        // (shuffles outside the selects: the quads' moves differ)
-        G = lane_get(G, quad | 2);
-        yG = lane_get(qq, quad | 2);
-        Km = fp_max_pos(run.dt, lane_get(qq, quad | 1));
-        if (!moves) {
-            G = 1.0;
-            yG = 0.0;
-            Km = run.dt;
+        const double P = lane_get(s1, quad), WPn = lane_get(w, quad);
+        // lane 1: R; lane 2: 2 sqrt(1+z^2) / (bw + 2 z x); lanes 0, 3: (WP n) / P
+        const double q1 = near_quot(r == 2 ? p.sq2 : r == 1 ? w : WPn, near_rcp(r == 2 ? s1 : P), unsure);
+        const double z = pow_near_one(lane_get(q1, quad | 1), r & 1, kc, unsure);
+        const double r23 = lane_get(z, quad);
+        const double sqt = lane_get(q1, quad | 2);
+        const double v = z * ((r & 1) ? 2.0 / 3.0 : 5.0 / 3.0) * ((r & 1) ? sqt : kc.one);
+        const double u = __shfl_xor_sync(0xffffffffu, v, 1);
+        const double Ck = p.ck_fac * (((r & 1) ? u : v) - ((r & 1) ? v : u));
+        const bool moves = wet && __double2hiint(Ck) > 0;
+        // lane 1: dx / Ck; lanes 0, 3: 1 / ((WP n) / P); lane 2: G = 2 tw s0 Ck dx, 1 / G
+        double G, yG, Km, it;
+        {
+            const bool g2 = r == 2;
+            const double b = r == 1 ? Ck : q1;
+            const double y0 = rcp_seed(b);
+            const double e1 = __fma_rn(g2 ? w : -b, g2 ? Ck : y0, g2 ? kc.neg_zero : kc.one);
+            const double e2 = __fma_rn(e1, g2 ? p.dx : e1, g2 ? kc.neg_zero : e1);
+            const double y = __fma_rn(y0, e2, y0);
+            G = __hiloint2double(__double2hiint(e2) + (1 << 20), __double2loint(e2));
+            const double yg0 = rcp_seed(G);
+            const double q0 = __fma_rn(g2 ? -G : (r == 1 ? p.dx : kc.one), g2 ? yg0 : y, g2 ? kc.one : kc.neg_zero);
+            const double rr = __fma_rn(g2 ? q0 : -b, q0, g2 ? q0 : (r == 1 ? p.dx : kc.one));
+            const double qq = __fma_rn(g2 ? yg0 : rr, g2 ? rr : y, g2 ? yg0 : q0);
+            unsure |= !g2 & (moves | (r != 1)) & quot_doubt(b, q0, rr);
+            it = qq;
+            // (shuffles outside the selects: the quads' moves differ)
+            G = lane_get(G, quad | 2);
+            yG = lane_get(qq, quad | 2);
+            Km = fp_max_pos(run.dt, lane_get(qq, quad | 1));
+            if (!moves) {
+                G = 1.0;
+                yG = 0.0;
+                Km = run.dt;
+            }
         }
-    }
-    double AAC = lane_get(w, quad | 1);
-    bool doubt = wet & unsure;
+        double AAC = lane_get(w, quad | 1);
+        bool doubt = wet & unsure;
 
-    // ---- the lower point of this pass, unless the last narrow pass formed it ----
-    double q0 = lane_get(L.qmc0_n, home), Qj_0 = lane_get(L.Qj0_n, home);
-    double r23u = r23, itu = it;
-    if (__any_sync(0xffffffffu, pre)) {
-        const double eK = lane_get(L.e0.Km, home), eG = lane_get(L.e0.G, home), ey = lane_get(L.e0.yG, home);
-        const double eQ = lane_get(L.e0.Qmn, home), Qp = lane_get(L.Qj_0, home);
-        bool d = false;
-        const QuadFlow a = quad_flow(r, quad, f, Qp, 0, need0 ? Km : eK, need0 ? G : eG, need0 ? yG : ey, it, AAC, r23,
-                                     p.sq_s0, kc, d);
-        const double Qmn = need0 ? (wet ? a.Qmn : 0.0) : eQ;
-        const double res = lane_get(a.q - Qmn, lane | 4), qa = lane_get(a.q, lane | 4);
-        if (pre) {
-            q0 = qa;
-            Qj_0 = res;
-            doubt |= B & d;
+        // ---- the lower point of this pass, unless the last narrow pass formed it ----
+        double q0 = q0n, Qj_0 = Qj0n;
+        double r23u = r23, itu = it;
+        if (__any_sync(0xffffffffu, pre)) {
+            const double eK = lane_get(L.e0.Km, home), eG = lane_get(L.e0.G, home), ey = lane_get(L.e0.yG, home);
+            const double eQ = lane_get(L.e0.Qmn, home), Qp = lane_get(L.Qj_0, home);
+            bool d = false;
+            const QuadFlow a = quad_flow(r, quad, f, Qp, 0, need0 ? Km : eK, need0 ? G : eG, need0 ? yG : ey, it, AAC, r23,
+                                         p.sq_s0, kc, d);
+            const double Qmn = need0 ? (wet ? a.Qmn : 0.0) : eQ;
+            const double res = lane_get(a.q - Qmn, lane | 4), qa = lane_get(a.q, lane | 4);
+            if (pre) {
+                q0 = qa;
+                Qj_0 = res;
+                doubt |= B & d;
+            }
+            // quad B goes on with the upper evaluation
+            Km = lane_get(Km, lane & ~4);
+            G = lane_get(G, lane & ~4);
+            yG = lane_get(yG, lane & ~4);
+            r23u = lane_get(r23, lane & ~4);
+            itu = lane_get(it, lane & ~4);
+            AAC = lane_get(AAC, lane & ~4);
         }
-        // quad B goes on with the upper evaluation
-        Km = lane_get(Km, lane & ~4);
-        G = lane_get(G, lane & ~4);
-        yG = lane_get(yG, lane & ~4);
-        r23u = lane_get(r23, lane & ~4);
-        itu = lane_get(it, lane & ~4);
-        AAC = lane_get(AAC, lane & ~4);
-    }
 
-    // ---- quad A: upper coefficients of this pass; quad B: lower ones of the next ----
-    const QuadFlow a = quad_flow(r, quad, f, B ? Qj_0 : q0, B ? 0 : 0x3fe00000, Km, G, yG, itu, AAC, r23u, p.sq_s0, kc, doubt);
-    const bool flowing = (__double2hiint(h) | __double2loint(h)) != 0;
-    const double Qmn = flowing ? a.Qmn : 0.0;
-    const double res = a.q - Qmn;
-    doubt |= !B & fp_lt0(a.q);   // the negative-flow fallbacks (troute_mc_final.cu:125-130)
+        // ---- quad A: upper coefficients of this pass; quad B: lower ones of the next ----
+        const QuadFlow a = quad_flow(r, quad, f, B ? Qj_0 : q0, B ? 0 : 0x3fe00000, Km, G, yG, itu, AAC, r23u, p.sq_s0, kc, doubt);
+        const bool flowing = (__double2hiint(h) | __double2loint(h)) != 0;
+        const double Qmn = flowing ? a.Qmn : 0.0;
+        const double res = a.q - Qmn;
+        doubt |= !B & fp_lt0(a.q);   // the negative-flow fallbacks (troute_mc_final.cu:125-130)
 
-    // ---- secant step, on every lane of the octet ----
-    const double Qj = lane_get(res, lane & ~7);
-    const double hd = lane_get(diff, quad | 3);
-    // lane 0: Qj (h_0 - h); lane 1: Qj_0 - Qj
-    const double n = __fma_rn((r & 1) ? kc.one : Qj, neg_if(r & 1, (r & 1) ? Qj : hd), (r & 1) ? Qj_0 : kc.neg_zero);
-    const double dQ = lane_get(n, quad | 1), num = lane_get(n, quad);
-    const bool slope = !fp_eq0(dQ);
-    bool d2 = false;
-    const double q2 = near_quot(num, near_rcp(dQ), d2);
-    double h_1 = slope ? h - q2 : h;
-    if (fp_lt0(h_1)) h_1 = h;
-    doubt |= slope & (d2 | !numerator_regular(num));
+        // ---- secant step, on every lane of the octet ----
+        const double Qj = lane_get(res, lane & ~7);
+        const double hd = lane_get(diff, quad | 3);
+        // lane 0: Qj (h_0 - h); lane 1: Qj_0 - Qj
+        const double n = __fma_rn((r & 1) ? kc.one : Qj, neg_if(r & 1, (r & 1) ? Qj : hd), (r & 1) ? Qj_0 : kc.neg_zero);
+        const double dQ = lane_get(n, quad | 1), num = lane_get(n, quad);
+        const bool slope = !fp_eq0(dQ);
+        bool d2 = false;
+        const double q2 = near_quot(num, near_rcp(dQ), d2);
+        double h_1 = slope ? h - q2 : h;
+        if (fp_lt0(h_1)) h_1 = h;
+        doubt |= slope & (d2 | !numerator_regular(num));
 
-    // ---- back to the solve's own lane ----
-    const unsigned bad = __ballot_sync(0xffffffffu, doubt);
-    const int src = (8 * __popc(smask & ((1u << lane) - 1u))) & 31;
-    DepthEval e;
-    e.Km = lane_get(Km, src);
-    e.G = lane_get(G, src);
-    e.yG = lane_get(yG, src);
-    e.Qmn = lane_get(Qmn, src);
-    PassOut po;
-    po.Qj_0 = lane_get(Qj_0, src);
-    po.qdc = lane_get(a.q, src);
-    po.h_1 = lane_get(h_1, src);
-    const double qn = lane_get(a.q, src + 4), rn = lane_get(res, src + 4);
-    if (!((smask >> lane) & 1u)) return false;
-    if ((bad >> src) & 0xffu) {
-        const SegP pl = staged_seg(warp_seg + lane + (L.i & 1) * kSegBufStride);
-        const PassFlow fl = {L.qup, L.quc, L.qdp, L.qldt, run.dt, run.dt_half};
-        redo_pass(pl, fl, L.need0 ? L.h_0 : L.h, L.need0, L.h, L.h_0, L.Qj_0, L.e0, L.irregular, e, po);
+        // ---- the next pass here, if every solve goes on ----
+        const unsigned bad = __ballot_sync(0xffffffffu, doubt);
+        const double nh = fp_max0(h_1);
+        const bool on = ((bad >> (lane & ~7)) & 0xffu) == 0 && k + 1 <= left && !fp_lt_pos(nh, kMinDepth) &&
+                        secant_more(h, h_1, run.tol);
+        if (__all_sync(0xffffffffu, on) && !__any_sync(0xffffffffu, leave(k))) {
+            e0.Km = Km;
+            e0.G = G;
+            e0.yG = yG;
+            e0.Qmn = Qmn;
+            Qj_before = Qj_0;
+            h_0 = fp_max0(h);
+            h = nh;
+            q0n = lane_get(a.q, lane | 4);
+            Qj0n = lane_get(res, lane | 4);
+            need0 = pre = false;
+            ++k;
+            continue;
+        }
+
+        // ---- back to the solve's own lane ----
+        const int src = (8 * __popc(smask & ((1u << lane) - 1u))) & 31;
+        const bool member = (smask >> lane) & 1u;
+        extra = k;
+        if (k > 0) {
+            const double hh = lane_get(h, src), hh_0 = lane_get(h_0, src);
+            if (member) {
+                L.h = hh;
+                L.h_0 = hh_0;
+                L.iter += k;
+                L.total += k;
+                L.need0 = 0;
+            }
+            if (bad) {
+                DepthEval b;
+                b.Km = lane_get(e0.Km, src);
+                b.G = lane_get(e0.G, src);
+                b.yG = lane_get(e0.yG, src);
+                b.Qmn = lane_get(e0.Qmn, src);
+                const double qb = lane_get(Qj_before, src);
+                if (member) {
+                    L.e0 = b;
+                    L.Qj_0 = qb;
+                }
+            }
+        }
+        DepthEval e;
+        e.Km = lane_get(Km, src);
+        e.G = lane_get(G, src);
+        e.yG = lane_get(yG, src);
+        e.Qmn = lane_get(Qmn, src);
+        PassOut po;
+        po.Qj_0 = lane_get(Qj_0, src);
+        po.qdc = lane_get(a.q, src);
+        po.h_1 = lane_get(h_1, src);
+        const double qn = lane_get(a.q, src + 4), rn = lane_get(res, src + 4);
+        if (!member) return false;
+        if ((bad >> src) & 0xffu) {
+            const SegP pl = staged_seg(warp_seg + lane + (L.i & 1) * kSegBufStride);
+            const PassFlow fl = {L.qup, L.quc, L.qdp, L.qldt, run.dt, run.dt_half};
+            redo_pass(pl, fl, L.need0 ? L.h_0 : L.h, L.need0, L.h, L.h_0, L.Qj_0, L.e0, L.irregular, e, po);
+            L.e0 = e;
+            L.ahead = false;
+            const bool iterated = !L.need0;
+            L.need0 = 0;
+            o = po;
+            return iterated;
+        }
         L.e0 = e;
-        L.ahead = false;
-        const bool iterated = !L.need0;
         L.need0 = 0;
+        L.ahead = true;
+        L.qmc0_n = qn;
+        L.Qj0_n = rn;
         o = po;
-        return iterated;
+        return true;
     }
-    L.e0 = e;
-    L.need0 = 0;
-    L.ahead = true;
-    L.qmc0_n = qn;
-    L.Qj0_n = rn;
-    o = po;
-    return true;
 }
 
 }  // namespace tr

@@ -170,10 +170,13 @@ __global__ void __launch_bounds__(kReachThreads, 3) reach_parallel_kernel(const 
         if (smask) {
             PassOut o;
             bool iterated = false;
-            if (__popc(smask) <= kNarrow && !__any_sync(kAll, L.mode == L_SOLVE && L.irregular))
-                iterated = narrow_pass(L, smask, a.run, warp_seg, o);
-            else if (L.mode == L_SOLVE)
+            if (__popc(smask) <= kNarrow && !__any_sync(kAll, L.mode == L_SOLVE && L.irregular)) {
+                const bool waits = L.mode == L_IDLE && (ready || left > 0 || more);
+                int extra;
+                iterated = narrow_passes(L, smask, a.run, warp_seg, o, extra, [&](int) { return waits; });
+            } else if (L.mode == L_SOLVE) {
                 iterated = lane_eval(L, a.run, slot, o);
+            }
             if (iterated && lane_book(L, o, a.run, ls)) {
                 a.qo[L.s] = L.qdc;
                 a.dpo[L.s] = L.h;

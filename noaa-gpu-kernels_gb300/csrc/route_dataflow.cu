@@ -65,6 +65,16 @@ __device__ __forceinline__ unsigned long long ld_volatile_ull(const unsigned lon
 }
 }  // namespace
 
+// How many more items a warp that holds `held` takes while `avail` are queued. (A
+// narrow warp with work leaves small backlogs to idle ones three passes out of
+// four: its atomics would mostly find nothing left.)
+__device__ __forceinline__ int claim_room(int avail, int held, bool primary, unsigned long long n_pass)
+{
+    if (avail >= kWideItems) return 32 - held;
+    const bool top_up = held == 0 || avail >= kTopUpItems || (n_pass & 3) == 0;
+    return primary && top_up ? kNarrow - held : 0;
+}
+
 // Loads the reach head inflows of (ri, tau) (all its dependencies are
 // complete) and starts its first segment.
 __device__ __forceinline__ void start_item(Lane& L, int ri, int tau, int t_base, const NetDev& net,
@@ -205,12 +215,7 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
             if (lane == 0) {
                 err = seen_err;
                 if (seen_avail > 0) {
-                    const int held = 32 - __popc(idle);
-                    // (a narrow warp with work leaves small backlogs to idle ones three
-                    // passes out of four: its atomics would mostly find nothing left)
-                    const bool top_up = held == 0 || seen_avail >= kTopUpItems || (n_pass & 3) == 0;
-                    const int room = seen_avail >= kWideItems ? 32 - held : primary && top_up ? kNarrow - held : 0;
-                    const int want = min(room, seen_avail);
+                    const int want = min(claim_room(seen_avail, 32 - __popc(idle), primary, n_pass), seen_avail);
                     if (want > 0) {
                         const int had = atomicSub(df.n_avail, want);
                         n = max(0, min(want, had));
@@ -308,10 +313,27 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
             n_solve++;
             PassOut o;
             bool iterated = false;
-            if (__popc(smask) <= kNarrow && !__any_sync(kFullMask, L.mode == L_SOLVE && L.irregular))
-                iterated = narrow_pass(L, smask, run, warp_seg, o);
-            else if (L.mode == L_SOLVE)
+            if (__popc(smask) <= kNarrow && !__any_sync(kFullMask, L.mode == L_SOLVE && L.irregular)) {
+                const unsigned held = __ballot_sync(kFullMask, L.mode != L_IDLE);
+                const bool fetching = L.mode == L_FETCH;
+                int extra;
+                iterated = narrow_passes(L, smask, run, warp_seg, o, extra, [&](int k) {
+                    bool out = fetching;
+                    if (lane == 0) {
+                        out |= seen_err != 0 || (seen_avail > 0 && claim_room(seen_avail, __popc(held), primary, n_pass + k + 1) > 0);
+                        seen_avail = ld_volatile_int(df.n_avail);
+                        seen_err = ld_volatile_int(&run.stats->error);
+                    }
+                    if (k == 0 && L.mode == L_SOLVE) stage_next_inflow(L, run, seg_slot);
+                    return out;
+                });
+                n_pass += extra;
+                n_solve += extra;
+                n_busy += (unsigned long long)extra * __popc(smask);
+                n_idle += (unsigned long long)extra * (32 - __popc(held));
+            } else if (L.mode == L_SOLVE) {
                 iterated = lane_eval(L, run, seg_slot, o);
+            }
             if (iterated) lane_finish(L, o, net, run, ls, hist_s, seg_slot);
         }
 
