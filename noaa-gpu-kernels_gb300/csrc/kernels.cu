@@ -122,23 +122,6 @@ __global__ void __launch_bounds__(128) route_kernel(NetDev net, RunDev run)
     flush_stats(ls, hist_s, run.stats);
 }
 
-__global__ void reach_rec_kernel(NetDev net, ReachRec* __restrict__ out)
-{
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < net.n_reach_int; r += gridDim.x * blockDim.x) {
-        ReachRec c = {};
-        c.nseg = net.nseg[r];
-        c.down = net.down[r];
-        c.up_ptr = net.up_ptr[r];
-        c.n_up = net.up_ptr[r + 1] - c.up_ptr;
-        if (c.down >= 0) c.down_n_up = net.up_ptr[c.down + 1] - net.up_ptr[c.down];
-        if (c.n_up > 0) c.up0 = net.up_idx[c.up_ptr];
-        if (c.n_up > 1) c.up1 = net.up_idx[c.up_ptr + 1];
-        c.base = net.tile_off[r / kLanes] + r % kLanes;
-        if (c.nseg > 0) c.qcol = net.seg[c.base].qcol;
-        out[r] = c;
-    }
-}
-
 __global__ void bump_steps_kernel(int* step_base, int n_ts) { *step_base += n_ts; }
 
 __global__ void fill_int_kernel(int* p, long long n, const int* value_dev, int value_host)
@@ -261,13 +244,6 @@ int launch_bump_steps(int* step_base, int n_ts, void* stream)
 {
     bump_steps_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(step_base, n_ts);
     return cuda_status(cudaGetLastError(), "bump_steps launch");
-}
-
-int launch_reach_recs(const NetDev& net, ReachRec* out, void* stream)
-{
-    if (net.n_reach_int <= 0) return TROUTE_OK;
-    reach_rec_kernel<<<grid_for(net.n_reach_int, 256), 256, 0, (cudaStream_t)stream>>>(net, out);
-    return cuda_status(cudaGetLastError(), "reach records launch");
 }
 
 int launch_fill_int(int* p, long long n, const int* value_dev, int value_host, void* stream)

@@ -185,7 +185,9 @@ struct troute_handle {
     bool broken = false;
 
     DBuf<SegRec> seg;
-    DBuf<ReachRec> reach;
+    DBuf<ItemRec> item;
+    DBuf<int> item_up;
+    int n_item = 0;
     DBuf<int> nseg, block_level, lb_ptr_d, up_ptr, up_idx, down, done, step_base;
     DBuf<double> q, d, v, ring, tmp, qlat_buf, hist;
     DBuf<long long> tile_off, seg_map_d, reach_map_d;
@@ -195,7 +197,7 @@ struct troute_handle {
     DBuf<int> df_cnt;
     DBuf<int2> df_rq, df_heads;
     DBuf<double> df_rh;
-    int n_heads = 0, R_real = 0;
+    int n_heads = 0;
     DBuf<DevStats> stats;
     int hist_ts = 0;
     // learned warm start and its training data
@@ -223,7 +225,6 @@ struct troute_handle {
         n.n_reach_int = R_int;
         n.n_seg_int = S_int;
         n.seg = seg.p;
-        n.reach = reach.p;
         n.nseg = nseg.p;
         n.tile_off = tile_off.p;
         n.block_level = block_level.p;
@@ -243,7 +244,7 @@ struct troute_handle {
     {
         if (graph_exec) cudaGraphExecDestroy(graph_exec);
         if (graph) cudaGraphDestroy(graph);
-        seg.release(); reach.release();
+        seg.release(); item.release(); item_up.release();
         nseg.release(); block_level.release(); lb_ptr_d.release();
         up_ptr.release(); up_idx.release(); down.release(); done.release(); step_base.release();
         q.release(); d.release(); v.release(); ring.release(); tmp.release();
@@ -293,13 +294,15 @@ static int launch_shape(troute_handle* H)
 
 // Host image of everything a handle uploads (internal order).
 struct Layout {
-    int R_user = 0, S_user = 0, n_levels = 0, NB = 0, R_int = 0, n_heads = 0, R_real = 0;
+    int R_user = 0, S_user = 0, n_levels = 0, NB = 0, R_int = 0;
     long long S_int = 0;  // tiles + 1 trash slot
     std::vector<int> user_seg_start, user_seg_len;
     std::vector<int> lb_ptr, block_level, nseg, up_ptr, up_idx, down_i;
     std::vector<long long> tile_off, seg_map, reach_map;  // seg_map: -1 for uncovered segments
-    std::vector<int2> heads;
     std::vector<SegRec> recs;    // parameters, inflow column and scale per tile slot
+    std::vector<ItemRec> items;
+    std::vector<int> item_up;
+    std::vector<int2> heads;
 };
 
 // A tile slot's record: derived parameters, inflow column, inflow scale.
@@ -338,7 +341,6 @@ static int build_layout(const Forest& f, const std::vector<troute_chparams>& par
     const int R = f.R;
     Lt.R_user = R;
     Lt.S_user = f.S;
-    Lt.R_real = R;
     Lt.user_seg_start = f.seg_start;
     Lt.user_seg_len = f.seg_len;
 
@@ -410,11 +412,6 @@ static int build_layout(const Forest& f, const std::vector<troute_chparams>& par
             Lt.up_ptr[ri + 1] = (int)Lt.up_idx.size();
         }
     }
-    // items ready at the start of a run: reaches without upstream reaches, step 0
-    for (int ri = 0; ri < Lt.R_int; ++ri)
-        if (Lt.nseg[ri] >= 0 && Lt.up_ptr[ri + 1] == Lt.up_ptr[ri]) Lt.heads.push_back(int2{ri, 0});
-    Lt.n_heads = (int)Lt.heads.size();
-
     // parameters in tile order
     Lt.recs.assign((size_t)Lt.S_int, empty_rec());
     for (int s = 0; s < f.S; ++s) {
@@ -442,7 +439,6 @@ static void replicate_layout(const Layout& B, const std::vector<troute_chparams>
     const int S = B.S_user, R = B.R_user, L = B.n_levels;
     E.R_user = R * M;
     E.S_user = S * M;
-    E.R_real = B.R_real * M;
     E.n_levels = L;
     E.NB = B.NB * M;
     E.R_int = E.NB * kLanes;
@@ -492,9 +488,6 @@ static void replicate_layout(const Layout& B, const std::vector<troute_chparams>
             for (int k = B.up_ptr[ri]; k < B.up_ptr[ri + 1]; ++k)
                 E.up_idx[E.up_ptr[ni] + (k - B.up_ptr[ri])] = new_reach(m, B.up_idx[k]);
         }
-    for (int m = 0; m < M; ++m)
-        for (const int2& h : B.heads) E.heads.push_back(int2{new_reach(m, h.x), 0});
-    E.n_heads = (int)E.heads.size();
     E.reach_map.resize((size_t)E.R_user);
     E.seg_map.resize((size_t)E.S_user);
     for (int m = 0; m < M; ++m) {
@@ -520,13 +513,64 @@ static void replicate_layout(const Layout& B, const std::vector<troute_chparams>
         }
 }
 
+// Segments of an item of the ready-queue kernel (0: whole reaches) in a handle of
+// `segments`. A reach can start a step when it has finished the step before, so a
+// run takes at least its steps times the passes of its longest reach; a segment by
+// itself starts a step as soon as the segment before it has made that step, and
+// reaches are pipelines. An item costs its start and its publishing, which matters
+// when the lanes are full. Whole / two / one segment: 1,000 segments, 288 steps
+// 37.4 / 13.8 / 10.3 ms; 20,000, 96 steps 23.4 / 15.9 / 13.8; 65,000, 24 steps
+// 17.2 / 16.1 / 16.1 and at rtol 1e-8 59.4 / 53.0 / 51.7; 200,000, 24 steps 29.3 /
+// 28.7 / 31.1 and at rtol 1e-8 115.7 / 109.1 / 110.2; 530,824, 24 steps, rtol 1e-8
+// 111.3 / 107.5 / 109.6; 64 members of 20,000, 16 steps, warm start 93.9 / 95.8 /
+// 99.4; 2.7 M, 24 steps, rtol 1e-8 509 / 527 / 527.
+static int item_segments(long long segments) { return segments <= (1 << 17) ? 1 : segments <= (1 << 20) ? 2 : 0; }
+
+// The items of a layout: its reaches, or pieces of `piece` segments each (0: whole).
+static void build_items(Layout& Lt, int piece)
+{
+    std::vector<int> first((size_t)Lt.R_int + 1, 0);
+    for (int ri = 0; ri < Lt.R_int; ++ri) {
+        const int n = Lt.nseg[ri];
+        first[ri + 1] = first[ri] + (n < 0 ? 0 : piece > 0 ? std::max(1, (n + piece - 1) / piece) : 1);
+    }
+    Lt.items.assign((size_t)first[Lt.R_int], ItemRec{});
+    Lt.item_up.reserve(Lt.up_idx.size());
+    for (int ri = 0; ri < Lt.R_int; ++ri) {
+        const int n_item = first[ri + 1] - first[ri];
+        for (int j = 0; j < n_item; ++j) {
+            ItemRec& c = Lt.items[(size_t)(first[ri] + j)];
+            const bool last = j + 1 == n_item;
+            const int s0 = j * piece;
+            c.nseg = last ? Lt.nseg[ri] - s0 : piece;
+            c.base = Lt.tile_off[ri / kLanes] + ri % kLanes + (long long)s0 * kLanes;
+            if (c.nseg > 0) c.qcol = Lt.recs[(size_t)c.base].qcol;
+            if (j == 0) {
+                c.up_ptr = (int)Lt.item_up.size();
+                for (int k = Lt.up_ptr[ri]; k < Lt.up_ptr[ri + 1]; ++k) Lt.item_up.push_back(first[Lt.up_idx[k] + 1] - 1);
+                c.n_up = Lt.up_ptr[ri + 1] - Lt.up_ptr[ri];
+                if (c.n_up > 0) c.up0 = Lt.item_up[(size_t)c.up_ptr];
+                if (c.n_up > 1) c.up1 = Lt.item_up[(size_t)c.up_ptr + 1];
+                if (c.n_up == 0) Lt.heads.push_back(int2{first[ri], 0});
+            } else {
+                c.up_ptr = -1;
+                c.n_up = 1;
+                c.up0 = first[ri] + j - 1;
+            }
+            c.reach = last ? ri : -1;
+            const int dn = last ? Lt.down_i[ri] : ri;
+            c.down = dn < 0 ? -1 : last ? first[dn] : first[ri] + j + 1;
+            c.down_n_up = dn < 0 ? 0 : last ? Lt.up_ptr[dn + 1] - Lt.up_ptr[dn] : 1;
+        }
+    }
+}
+
 // Uploads a layout into a handle and allocates its state.
 static int upload_layout(troute_handle* H, Layout& Lt)
 {
     int rc;
     H->R_user = Lt.R_user;
     H->S_user = Lt.S_user;
-    H->R_real = Lt.R_real;
     H->user_seg_start = std::move(Lt.user_seg_start);
     H->user_seg_len = std::move(Lt.user_seg_len);
     H->n_levels = Lt.n_levels;
@@ -534,7 +578,11 @@ static int upload_layout(troute_handle* H, Layout& Lt)
     H->R_int = Lt.R_int;
     H->S_int = Lt.S_int;
     H->lb_ptr = Lt.lb_ptr;
-    H->n_heads = Lt.n_heads;
+    long long covered = 0;
+    for (const int n : Lt.nseg) covered += std::max(0, n);
+    build_items(Lt, item_segments(covered));
+    H->n_item = (int)Lt.items.size();
+    H->n_heads = (int)Lt.heads.size();
     H->seg_map = Lt.seg_map;
     H->reach_map = Lt.reach_map;
     const long long trash = Lt.S_int - 1;
@@ -553,6 +601,8 @@ static int upload_layout(troute_handle* H, Layout& Lt)
     if ((rc = upload(H->up_ptr, Lt.up_ptr, st))) return rc;
     if ((rc = upload(H->up_idx, Lt.up_idx.empty() ? std::vector<int>{0} : Lt.up_idx, st))) return rc;
     if ((rc = upload(H->down, Lt.down_i, st))) return rc;
+    if ((rc = upload(H->item, Lt.items.empty() ? std::vector<ItemRec>(1) : Lt.items, st))) return rc;
+    if ((rc = upload(H->item_up, Lt.item_up.empty() ? std::vector<int>{0} : Lt.item_up, st))) return rc;
     if ((rc = upload(H->df_heads, Lt.heads.empty() ? std::vector<int2>{int2{0, 0}} : Lt.heads, st))) return rc;
     if ((rc = upload(H->seg_map_d, seg_map_dev.empty() ? std::vector<long long>{trash} : seg_map_dev, st))) return rc;
     if ((rc = upload(H->reach_map_d, H->reach_map.empty() ? std::vector<long long>{0} : H->reach_map, st))) return rc;
@@ -568,7 +618,6 @@ static int upload_layout(troute_handle* H, Layout& Lt)
     if ((rc = cuda_check(cudaMemsetAsync(H->ring.p, 0, H->ring.n * sizeof(double), st), "memset"))) return rc;
     if ((rc = cuda_check(cudaMemsetAsync(H->done.p, 0, H->done.n * sizeof(int), st), "memset"))) return rc;
     if ((rc = cuda_check(cudaMemsetAsync(H->step_base.p, 0, sizeof(int), st), "memset"))) return rc;
-    if ((rc = H->reach.alloc(std::max(1, H->R_int))) || (rc = launch_reach_recs(H->net(), H->reach.p, st))) return rc;
     if ((rc = launch_shape(H))) return rc;
     return cuda_check(cudaStreamSynchronize(st), "build sync");
 }
@@ -845,8 +894,7 @@ static int plan_run(troute_handle* H, int n_ts, RunPlan* P)
     int chunk = n_ts;
     if (H->cfg.max_chunk_steps > 0) chunk = std::min(chunk, H->cfg.max_chunk_steps);
     if (H->mapping == 3) {
-        const double per_step = (double)std::max(1, H->R_int) * (sizeof(int) + sizeof(double)) +
-                                (double)std::max(1, H->R_real) * sizeof(int2) +
+        const double per_step = (double)std::max(1, H->n_item) * (sizeof(int) + sizeof(double) + sizeof(int2)) +
                                 (H->cfg.warm_start ? (double)H->S_int * sizeof(float) : 0.0);
         if (H->chunk_budget_bytes == 0) {
             size_t fr = 0, tot = 0;
@@ -895,6 +943,9 @@ static int enqueue_chunk(troute_handle* H, const double* qlat_dev, int n_ts, con
     if ((rc = cuda_check(cudaMemsetAsync(H->ticket.p, 0, sizeof(unsigned long long), st), "memset"))) return rc;
     if (H->mapping == 3) {
         DataflowDev df;
+        df.item = H->item.p;
+        df.up_idx = H->item_up.p;
+        df.n_item = H->n_item;
         df.cnt = H->df_cnt.p;
         df.rq = H->df_rq.p;
         df.rq_head = H->rq_ctr.p;
@@ -906,7 +957,7 @@ static int enqueue_chunk(troute_handle* H, const double* qlat_dev, int n_ts, con
         df.n_heads = H->n_heads;
         df.continue_items = H->cfg.schedule_flags & 1;
         df.n_primary = H->n_sms;
-        df.n_items = (unsigned long long)H->R_real * (unsigned long long)n_ts;
+        df.n_items = (unsigned long long)H->n_item * (unsigned long long)n_ts;
         if (run.warm) {
             // the launch's learned starting depths: one tcgen05 GEMM over every
             // (segment slot, step) from the state at the launch's start
@@ -998,10 +1049,10 @@ static int prepare_run(troute_handle* H, int n_ts, RunPlan* P)
     }
     if (H->cfg.warm_start && (rc = H->pred.alloc((size_t)P->chunk * H->S_int))) return rc;
     if (H->mapping == 3) {
-        const size_t R = (size_t)std::max(1, H->R_int);
+        const size_t R = (size_t)std::max(1, H->n_item);
         const size_t T = (size_t)P->chunk;
         if ((rc = H->df_cnt.alloc(T * R)) || (rc = H->df_rh.alloc((T + 1) * R)) ||
-            (rc = H->df_rq.alloc(std::max<size_t>(1, (size_t)H->R_real * T))) || (rc = H->rq_ctr.alloc(4)))
+            (rc = H->df_rq.alloc(R * T)) || (rc = H->rq_ctr.alloc(4)))
             return rc;
     }
     return TROUTE_OK;

@@ -81,15 +81,18 @@ __device__ __forceinline__ void start_item(Lane& L, int ri, int tau, int t_base,
                                            const RunDev& run, const DataflowDev& df, LocalStats& ls,
                                            unsigned int* hist_s, double2* slot)
 {
-    const int R = net.n_reach_int;
+    const int R = df.n_item;
+    const int4* rec = reinterpret_cast<const int4*>(df.item + ri);
+    const int4 a = __ldg(rec), b = __ldg(rec + 1);
+    const int2 c = __ldg(reinterpret_cast<const int2*>(rec + 2));   // row start in up_idx, inflow column
 #ifdef TROUTE_CHECK
     // self-check build (the outflow history is NaN-filled before the run):
     // every value (ri, tau) reads must already be written, and its own output
     // slot must not be
     {
         bool ok = !isnan(__ldcg(df.rh + (size_t)tau * R + ri)) && isnan(__ldcg(df.rh + (size_t)(tau + 1) * R + ri));
-        for (int j = __ldg(net.up_ptr + ri); j < __ldg(net.up_ptr + ri + 1); ++j) {
-            const int u = __ldg(net.up_idx + j);
+        for (int j = 0; j < a.y; ++j) {
+            const int u = j == 0 ? b.z : j == 1 ? b.w : __ldg(df.up_idx + c.x + j);
             ok = ok && !isnan(__ldcg(df.rh + (size_t)tau * R + u)) && !isnan(__ldcg(df.rh + (size_t)(tau + 1) * R + u));
         }
         if (!ok) record_error(run.stats, TROUTE_EINVAL, ri, t_base + tau, 7);
@@ -98,9 +101,6 @@ __device__ __forceinline__ void start_item(Lane& L, int ri, int tau, int t_base,
     L.ri = ri;
     L.tau = tau;
     L.g = t_base + tau;
-    const int4* rec = reinterpret_cast<const int4*>(net.reach + ri);
-    const int4 a = __ldg(rec), b = __ldg(rec + 1);
-    const int2 c = __ldg(reinterpret_cast<const int2*>(rec + 2));   // row start in up_idx, inflow column
     L.ns = a.x;
     L.n_up = a.y;
     L.dn = a.z;
@@ -112,7 +112,7 @@ __device__ __forceinline__ void start_item(Lane& L, int ri, int tau, int t_base,
     }
     L.inflow = kInflowStaged;
     // sums over the upstream reaches in their order, from +0 (a first addend of -0
-    // becomes +0, as in 0.0 + -0.0)
+    // becomes +0, as in 0.0 + -0.0); within a reach the value itself
     const double* rprev = df.rh + (size_t)tau * R;
     const double* rcur = df.rh + (size_t)(tau + 1) * R;
     double p = 0.0, q = 0.0;
@@ -123,14 +123,14 @@ __device__ __forceinline__ void start_item(Lane& L, int ri, int tau, int t_base,
             p1 = __ldcg(rprev + b.w);
             q1 = __ldcg(rcur + b.w);
         }
-        p = fp_eq0(p0) ? 0.0 : p0;
-        q = fp_eq0(q0) ? 0.0 : q0;
+        p = c.x >= 0 && fp_eq0(p0) ? 0.0 : p0;
+        q = c.x >= 0 && fp_eq0(q0) ? 0.0 : q0;
         if (L.n_up > 1) {
             p += p1;
             q += q1;
         }
         for (int j = 2; j < L.n_up; ++j) {
-            const int u = __ldg(net.up_idx + c.x + j);
+            const int u = __ldg(df.up_idx + c.x + j);
             p += __ldcg(rprev + u);
             q += __ldcg(rcur + u);
         }
@@ -181,7 +181,7 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
     const unsigned lt = lanemask_lt_df();
     const int t_base = __ldg(run.step_base);
     const int T = run.n_ts;
-    const int R = net.n_reach_int;
+    const int R = df.n_item;
     bool failed = false;
     unsigned long long slot = 0;
     const bool primary = blockIdx.x < (unsigned)df.n_primary;
@@ -346,8 +346,13 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
         if (L.mode == L_DONE) {
             __stcg(df.rh + (size_t)(L.tau + 1) * R + L.ri, L.q_last);
             // what later launches start from
-            if (L.tau + kRing >= T) __stcg(net.ring + (size_t)(L.g % kRing) * R + L.ri, L.q_last);
-            if (L.tau + 1 == T) net.done[L.ri] = L.g + 1;
+            if (L.tau + kRing >= T) {
+                const int reach = __ldg(&df.item[L.ri].reach);
+                if (reach >= 0) {
+                    __stcg(net.ring + (size_t)(L.g % kRing) * net.n_reach_int + reach, L.q_last);
+                    if (L.tau + 1 == T) net.done[reach] = L.g + 1;
+                }
+            }
             __threadfence();
             // the reach's own next step (needs its upstream reaches too) and the reach
             // downstream: both counters in flight together
@@ -442,8 +447,10 @@ __global__ void dataflow_init_kernel(NetDev net, RunDev run, DataflowDev df)
     const int t_base = *run.step_base;
     const int slot = ((t_base - 1) % kRing + kRing) % kRing;
     const double* src = net.ring + (size_t)slot * net.n_reach_int;
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < net.n_reach_int; r += gridDim.x * blockDim.x)
-        df.rh[r] = src[r];
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < df.n_item; r += gridDim.x * blockDim.x) {
+        const ItemRec& c = df.item[r];
+        df.rh[r] = c.reach >= 0 ? src[c.reach] : net.q[c.base + (long long)(c.nseg - 1) * kLanes];
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *df.rq_head = 0;
         *df.rq_tail = (unsigned long long)df.n_heads;
@@ -459,14 +466,14 @@ int launch_route_dataflow(const NetDev& net, const RunDev& run, const DataflowDe
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e;
 #ifdef TROUTE_CHECK
-    if ((e = cudaMemsetAsync(df.rh, 0xff, (size_t)(run.n_ts + 1) * net.n_reach_int * sizeof(double), st)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(df.rh, 0xff, (size_t)(run.n_ts + 1) * df.n_item * sizeof(double), st)) != cudaSuccess)
         return set_error(TROUTE_ECUDA, "dataflow set-up: %s", cudaGetErrorString(e));
 #endif
-    if ((e = cudaMemsetAsync(df.cnt, 0, (size_t)run.n_ts * net.n_reach_int * sizeof(int), st)) != cudaSuccess ||
+    if ((e = cudaMemsetAsync(df.cnt, 0, (size_t)run.n_ts * df.n_item * sizeof(int), st)) != cudaSuccess ||
         (e = cudaMemsetAsync(df.rq, 0xff, (size_t)df.n_items * sizeof(int2), st)) != cudaSuccess ||
         (e = cudaMemcpyAsync(df.rq, df.heads, (size_t)df.n_heads * sizeof(int2), cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
         return set_error(TROUTE_ECUDA, "dataflow set-up: %s", cudaGetErrorString(e));
-    int ig = (net.n_reach_int + 255) / 256;
+    int ig = (df.n_item + 255) / 256;
     if (ig > 4096) ig = 4096;
     if (ig < 1) ig = 1;
     dataflow_init_kernel<<<ig, 256, 0, st>>>(net, run, df);

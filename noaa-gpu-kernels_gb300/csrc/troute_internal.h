@@ -100,18 +100,21 @@ TR_HD inline bool seg_regular(const SegP& p)
            value_regular(p.sq_s0) && value_regular(p.sq2) && value_regular(p.ck_fac) && value_regular(p.z2);
 }
 
-// What starting and publishing an item reads of its reach, in one record: the
-// routing kernel would otherwise follow four dependent loads (row pointers,
-// upstream list, first segment, its inflow column).
-struct __align__(64) ReachRec {
-    int nseg, n_up, down, down_n_up;   // down: internal reach or -1
+// What the ready-queue kernel reads to start and publish an item, a reach or a piece
+// of one, in one record: it would otherwise follow four dependent loads (row
+// pointers, upstream list, first segment, its inflow column).
+// (The pieces of a reach follow one another; the first has the reach's upstream
+// reaches, through their last pieces, the last its downstream one.)
+struct __align__(64) ItemRec {
+    int nseg, n_up, down, down_n_up;   // down: item downstream or -1
     long long base;                    // tile slot of the first segment
-    int up0, up1;                      // the first two upstream reaches
-    int up_ptr;                        // row start in up_idx
+    int up0, up1;                      // the first two upstream items
+    int up_ptr;                        // row start in DataflowDev.up_idx; -1: the rest of up0's reach
     int qcol;                          // inflow column of the first segment
-    int pad[6];
+    int reach;                         // internal reach whose last piece this is, else -1
+    int pad[5];
 };
-static_assert(sizeof(ReachRec) == 64, "two sectors per reach");
+static_assert(sizeof(ItemRec) == 64, "two sectors per item");
 
 // Device counters of one run.
 struct DevStats {
@@ -132,7 +135,6 @@ struct NetDev {
     int n_reach_int;         // n_blocks * kLanes
     long long n_seg_int;     // padded tile storage
     const SegRec* seg;       // [n_seg_int] parameters, inflow column and scale
-    const ReachRec* reach;   // [n_reach_int]
     const int* nseg;         // [n_reach_int], -1 for padding lanes
     const long long* tile_off;  // [n_blocks] first segment slot of a block
     const int* block_level;  // [n_blocks]
@@ -176,18 +178,21 @@ struct RunDev {
 
 // Ready-queue state of one run of the dataflow kernel (mapping 3).
 struct DataflowDev {
-    int* cnt;                       // [n_ts][n_reach_int] completed dependencies
-    int2* rq;                       // [n_items] ready (reach, step) items
+    const ItemRec* item;            // [n_item]
+    const int* up_idx;              // upstream items of the items with an up_ptr
+    int n_item;                     // items of a step
+    int* cnt;                       // [n_ts][n_item] completed dependencies
+    int2* rq;                       // [n_items] ready (item, step) pairs
     unsigned long long* rq_head;    // claimed slots
     unsigned long long* rq_tail;    // written slots
     unsigned long long* n_done;     // completed items
     int* n_avail;                   // queued items no warp has claimed (down to minus the claims in flight)
-    double* rh;                     // [n_ts + 1][n_reach_int] reach outflow per step
-    const int2* heads;              // (headwater reach, 0) items, ready at the start
+    double* rh;                     // [n_ts + 1][n_item] outflow per step
+    const int2* heads;              // (item without upstream, 0), ready at the start
     int n_heads;
     int continue_items;             // 1: a lane continues with an item it made ready (0: in narrow warps only)
     int n_primary;                  // blocks whose warps take queued items as they come (one per SM)
-    unsigned long long n_items;     // real reaches x n_ts
+    unsigned long long n_items;     // n_item x n_ts
 };
 
 // Launch helpers (all asynchronous on `stream`).
@@ -218,7 +223,6 @@ int compact_pairs(const float* dense, long long n_rows, float* out, long long ca
 int route_dataflow_occupancy(int* blocks_per_sm, bool warm);
 int route_dataflow_threads();
 int launch_bump_steps(int* step_base, int n_ts, void* stream);
-int launch_reach_recs(const NetDev& net, ReachRec* out, void* stream);
 int launch_fill_int(int* p, long long n, const int* value_dev, int value_host, void* stream);
 int launch_scatter(const double* src, const long long* map, long long n, double* dst,
                    void* stream);
