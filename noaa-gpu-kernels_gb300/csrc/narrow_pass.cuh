@@ -30,20 +30,30 @@ constexpr int kNarrow = 4;   // solves of a narrow pass
 
 __device__ __forceinline__ double lane_get(double v, int src) { return __shfl_sync(0xffffffffu, v, src); }
 
-// Constants the compiler does not see through: a select between one of them and
-// a variable would otherwise be turned into two FP64 instructions, one for each
-// side, where the point is to share one.
-struct Opaque {
-    double one, neg_zero, neg_two;
-};
-__device__ __forceinline__ Opaque opaque_constants()
+// One of two constants with a zero low word, by a lane's role, which the compiler
+// does not see through: a select between constants would otherwise be turned into
+// two FP64 instructions, one for each side, where the point is to share one.
+__device__ __forceinline__ double role_const(bool a, double if_a, double if_not)
 {
-    Opaque k;
-    asm("mov.b64 %0, 0x3ff0000000000000;" : "=d"(k.one));
-    asm("mov.b64 %0, 0x8000000000000000;" : "=d"(k.neg_zero));
-    asm("mov.b64 %0, 0xc000000000000000;" : "=d"(k.neg_two));
-    return k;
+    int hi = a ? __double2hiint(if_a) : __double2hiint(if_not);
+    asm("" : "+r"(hi));
+    return __hiloint2double(hi, 0);
 }
+
+// What differs between the four lanes of a quad, for a solve.
+struct Role {
+    int r;              // lane of the quad
+    bool xl;            // lanes 1 and 2: X's quotient; 0 and 3: the Manning discharge
+    double one_two;     // odd lanes -2, others 1 (the powers' correction)
+    double one, neg_zero;
+    double rcp_c;       // lane 2 -0, others 1
+    double quot_c;      // lane 2 1, others -0
+    double om_x, om_c;  // X or 1 - X = om_x X + om_c
+    double neg_one;
+    double flow;        // qup, quc, qdp, 1
+    double dt2;         // lane 2 -dt/2, others dt/2
+    double qldt;
+};
 
 // v or -v, on the integer pipe
 __device__ __forceinline__ double neg_if(bool neg, double v)
@@ -53,7 +63,7 @@ __device__ __forceinline__ double neg_if(bool neg, double v)
 
 // One of x^fl(2/3) (odd = false) and x^fl(5/3) (odd = true) as pow23_53_near forms
 // them: the same instructions for both, y or 1 as the outer factor.
-__device__ __forceinline__ double pow_near_one(double x, bool odd, const Opaque& kc, bool& doubt)
+__device__ __forceinline__ double pow_near_one(double x, bool odd, const Role& kc, bool& doubt)
 {
     const int hi = __double2hiint(x);
     const int u = (hi >> 20) - (1023 - 36);
@@ -73,7 +83,7 @@ __device__ __forceinline__ double pow_near_one(double x, bool odd, const Opaque&
     const double m = odd ? y : kc.one;
     const double w0 = m * wh;
     const double we = __fma_rn(m, wl, __fma_rn(m, wh, -w0));
-    const double a = __fma_rn(w0, __fma_rn(odd ? kc.neg_two : kc.one, c, s), we);
+    const double a = __fma_rn(w0, __fma_rn(kc.one_two, c, s), we);
     const double z = w0 + a;
     const double e = a - (z - w0);
     const int h = __double2hiint(z);
@@ -83,32 +93,32 @@ __device__ __forceinline__ double pow_near_one(double x, bool odd, const Opaque&
 
 // Coefficients and discharge of one quad's evaluation: X from num / G clamped to
 // [lo, 1/2] (lo2 as in clamped_half), C1..C4 on the quad's four lanes, their sum with the flows; beside X's
-// quotient (lanes 1, 2) lanes 0 and 3 form the Manning discharge.
+// quotient (lanes 1, 2) lanes 0 and 3 form the Manning discharge. W and V hold -G
+// and 1/G on lanes 1 and 2 (1/G = 0: none), R^(2/3) and the area on 0 and 3.
 struct QuadFlow {
     double q, C4, Qmn;   // on all lanes of the quad
 };
 
-__device__ __forceinline__ QuadFlow quad_flow(int r, int quad, const PassFlow& f, double num, int lo2, double Km, double G,
-                                              double yG, double it, double AAC, double r23, double sq_s0, const Opaque& kc, bool& doubt)
+__device__ __forceinline__ QuadFlow quad_flow(const Role& k, int quad, double num, int lo2, double Km, double W, double V,
+                                              double it, double sq_s0, bool& doubt)
 {
-    const bool xl = r == 1 || r == 2;
-    const bool valid = dbits(yG) != 0;
-    const double q0 = (xl ? num : it) * (xl ? yG : AAC);
-    const double rr = __fma_rn(xl ? -G : q0, xl ? q0 : r23, xl ? num : kc.neg_zero);
-    const double qq = __fma_rn(rr, xl ? yG : sq_s0, xl ? q0 : kc.neg_zero);
-    doubt |= xl & valid & quot_doubt(G, q0, rr);
+    const bool valid = dbits(V) != 0;
+    const double q0 = (k.xl ? num : it) * V;
+    const double rr = __fma_rn(W, q0, k.xl ? num : k.neg_zero);
+    const double qq = __fma_rn(rr, k.xl ? V : sq_s0, k.xl ? q0 : k.neg_zero);
+    doubt |= k.xl & valid & quot_doubt(W, q0, rr);
     double X = clamped_half(1.0 - qq, lo2);
     if (!valid) X = 0.5;
     X = lane_get(X, quad | 1);
     QuadFlow o;
     o.Qmn = lane_get(qq, quad);
-    const double om = 1.0 - X;
-    const double t = Km * (r < 2 ? X : om);   // Km X on lanes 0, 1; Km (1 - X) on 2, 3
+    // Km X on lanes 0, 1; Km (1 - X) on 2, 3
+    const double t = Km * __fma_rn(X, k.om_x, k.om_c);
     // numerators Km X + dt/2, dt/2 - Km X, Km (1 - X) - dt/2; lane 3: the denominator
-    const double n = neg_if(r == 1, t) + neg_if(r == 2, f.dt2);
+    const double n = neg_if(k.r == 1, t) + k.dt2;
     const NearRcp rd = near_rcp(lane_get(n, quad | 3));
-    const double c = near_quot(r == 3 ? f.qldt : n, rd, doubt);
-    const double m = c * (r == 0 ? f.qup : r == 1 ? f.quc : r == 2 ? f.qdp : kc.one);
+    const double c = near_quot(k.r == 3 ? k.qldt : n, rd, doubt);
+    const double m = c * k.flow;
     const double S3 = lane_get(m, quad) + lane_get(m, quad | 1) + lane_get(m, quad | 2);
     double C4 = lane_get(m, quad | 3);
     if (__any_sync(0xffffffffu, __double2hiint(C4) < 0))
@@ -116,6 +126,17 @@ __device__ __forceinline__ QuadFlow quad_flow(int r, int quad, const PassFlow& f
     o.C4 = C4;
     o.q = S3 + C4;
     return o;
+}
+
+// secant_more(h, h_1) from h_1 = h - step without FP64 instructions, where it is
+// clearly true: the step is at least 2^-30 h, four times rtol h and four times
+// atol by the exponents (the roundings of h_1 and of h_1 - h change it by a part in
+// 2^21 at most).
+__device__ __forceinline__ bool surely_more(double h, double step, const Tol& tol)
+{
+    const int eh = (__double2hiint(h) >> 20) & 0x7ff, es = (__double2hiint(step) >> 20) & 0x7ff;
+    const int er = (__double2hiint(tol.rtol) >> 20) - 1023, ea = __double2hiint(tol.atol) >> 20;
+    return (__double2hiint(h) > 0) & (eh != 0) & (es < 0x7ff) & (es - eh >= max(er + 3, -30)) & (es >= ea + 2);
 }
 
 // Passes for the lanes of smask (at most kNarrow, none irregular) until one of the
@@ -153,13 +174,29 @@ __device__ __forceinline__ bool narrow_passes(Lane& L, unsigned smask, const Run
     bool need0 = flags & 2, pre = !(flags & 4);
     double h = lane_get(L.h, home), h_0 = lane_get(L.h_0, home);
     double q0n = lane_get(L.qmc0_n, home), Qj0n = lane_get(L.Qj0_n, home);
-    const PassFlow f = {lane_get(L.qup, home), lane_get(L.quc, home), lane_get(L.qdp, home), lane_get(L.qldt, home), run.dt,
-                        run.dt_half};
-    const Opaque kc = opaque_constants();
+    Role kc;
+    kc.r = r;
+    kc.xl = r == 1 || r == 2;
+    kc.one_two = role_const(r & 1, -2.0, 1.0);
+    kc.one = role_const(true, 1.0, 1.0);
+    kc.neg_zero = role_const(true, -0.0, -0.0);
+    kc.rcp_c = role_const(r == 2, -0.0, 1.0);
+    kc.quot_c = role_const(r == 2, 1.0, -0.0);
+    kc.om_x = role_const(r < 2, 1.0, -1.0);
+    kc.om_c = role_const(r < 2, -0.0, 1.0);
+    kc.neg_one = role_const(true, -1.0, -1.0);
+    {
+        const double up = lane_get(L.qup, home), uc = lane_get(L.quc, home), dp = lane_get(L.qdp, home);
+        kc.flow = r == 0 ? up : r == 1 ? uc : r == 2 ? dp : kc.one;
+        kc.qldt = lane_get(L.qldt, home);
+        kc.dt2 = neg_if(r == 2, run.dt_half);
+    }
     const double2* const rec = warp_seg + home + (flags & 1) * kSegBufStride;
+    // this lane's factors of the geometry: WP, A, top width (twice); n, -, s0, s0
+    const double* const c1 = reinterpret_cast<const double*>(rec + (r == 0 ? 4 : r == 1 ? 3 : 5) * kSegSmemStride) + (r != 1);
+    const double* const c2 = reinterpret_cast<const double*>(rec + (r == 0 ? 1 : 2) * kSegSmemStride) + 1;
     // on quad A of a solve past its first pass here: what the pass before left
-    DepthEval e0 = {};
-    double Qj_before = 0.0;
+    double Km_before = 0.0, W_before = 0.0, V_before = 0.0, Qmn_before = 0.0, Qj_before = 0.0;
     int k = 0;
     while (true) {
         const SegP p = staged_seg(rec);
@@ -169,12 +206,12 @@ __device__ __forceinline__ bool narrow_passes(Lane& L, unsigned smask, const Run
         const bool wet = (__double2hiint(x) | __double2loint(x)) != 0;
         bool unsure = !depth_regular(x);
         const bool over = dbits(x) > dbits(p.bfd);
-        const double below = over ? p.bfd : x;
         // depth above the bank; lane 3: h_0 - h for the secant step
         const double diff = (r == 3 ? h_0 : x) - (r == 3 ? h : p.bfd);
         // lane 0: WP, WP n; lane 1: A; lanes 2, 3: bw + 2 z x and its product with s0
-        double s1 = p.bw + (r < 2 ? below : p.z2) * (r == 0 ? p.sq2 : r == 1 ? p.z : x);
-        double w = s1 * (r == 0 ? p.n_ch : r == 1 ? below : p.s0);
+        const double xb = over & (r < 2) ? p.bfd : x;
+        double s1 = p.bw + xb * *c1;
+        double w = s1 * (r == 1 ? xb : *c2);
         if (__any_sync(0xffffffffu, over)) {
             const double t1 = __fma_rn(r == 0 ? 2.0 : p.twcc, r >= 2 ? p.s0 : diff, r == 0 ? p.twcc : kc.neg_zero);
             const double t2 = (r == 0 ? s1 : w) + t1;
@@ -184,54 +221,51 @@ __device__ __forceinline__ bool narrow_passes(Lane& L, unsigned smask, const Run
                 else w = r == 1 ? t2 : t1;
             }
         }
-        const double P = lane_get(s1, quad), WPn = lane_get(w, quad);
         // lane 1: R; lane 2: 2 sqrt(1+z^2) / (bw + 2 z x); lanes 0, 3: (WP n) / P
-        const double q1 = near_quot(r == 2 ? p.sq2 : r == 1 ? w : WPn, near_rcp(r == 2 ? s1 : P), unsure);
+        const double P = lane_get(s1, r == 2 ? lane : quad), wn = lane_get(w, r == 1 ? lane : quad);
+        const double q1 = near_quot(r == 2 ? p.sq2 : wn, near_rcp(P), unsure);
         const double z = pow_near_one(lane_get(q1, quad | 1), r & 1, kc, unsure);
-        const double r23 = lane_get(z, quad);
         const double sqt = lane_get(q1, quad | 2);
-        const double v = z * ((r & 1) ? 2.0 / 3.0 : 5.0 / 3.0) * ((r & 1) ? sqt : kc.one);
-        const double u = __shfl_xor_sync(0xffffffffu, v, 1);
-        const double Ck = p.ck_fac * (((r & 1) ? u : v) - ((r & 1) ? v : u));
+        const double v = neg_if(r & 1, z * ((r & 1) ? 2.0 / 3.0 : 5.0 / 3.0) * ((r & 1) ? sqt : kc.one));
+        const double Ck = p.ck_fac * (v + __shfl_xor_sync(0xffffffffu, v, 1));
         const bool moves = wet && __double2hiint(Ck) > 0;
         // lane 1: dx / Ck; lanes 0, 3: 1 / ((WP n) / P); lane 2: G = 2 tw s0 Ck dx, 1 / G
-        double G, yG, Km, it;
+        double W, V, Km, it;
         {
             const bool g2 = r == 2;
-            const double b = r == 1 ? Ck : q1;
+            const double b = r == 1 ? Ck : q1, nd = r == 1 ? p.dx : kc.one;
             const double y0 = rcp_seed(b);
-            const double e1 = __fma_rn(g2 ? w : -b, g2 ? Ck : y0, g2 ? kc.neg_zero : kc.one);
+            const double nb = neg_if(!g2, g2 ? w : b);
+            const double e1 = __fma_rn(nb, g2 ? Ck : y0, kc.rcp_c);
             const double e2 = __fma_rn(e1, g2 ? p.dx : e1, g2 ? kc.neg_zero : e1);
             const double y = __fma_rn(y0, e2, y0);
-            G = __hiloint2double(__double2hiint(e2) + (1 << 20), __double2loint(e2));
+            const double G = __hiloint2double(__double2hiint(e2) + (1 << 20), __double2loint(e2));
             const double yg0 = rcp_seed(G);
-            const double q0 = __fma_rn(g2 ? -G : (r == 1 ? p.dx : kc.one), g2 ? yg0 : y, g2 ? kc.one : kc.neg_zero);
-            const double rr = __fma_rn(g2 ? q0 : -b, q0, g2 ? q0 : (r == 1 ? p.dx : kc.one));
-            const double qq = __fma_rn(g2 ? yg0 : rr, g2 ? rr : y, g2 ? yg0 : q0);
+            const double ya = g2 ? yg0 : y, nG = neg_if(true, G);
+            const double q0 = __fma_rn(g2 ? nG : nd, ya, kc.quot_c);
+            const double rr = __fma_rn(g2 ? q0 : nb, q0, g2 ? q0 : nd);
+            const double qq = __fma_rn(rr, ya, g2 ? yg0 : q0);
             unsure |= !g2 & (moves | (r != 1)) & quot_doubt(b, q0, rr);
             it = qq;
             // (shuffles outside the selects: the quads' moves differ)
-            G = lane_get(G, quad | 2);
-            yG = lane_get(qq, quad | 2);
+            W = lane_get(g2 ? nG : z, quad | (kc.xl ? 2 : 0));
+            V = lane_get(r == 1 ? w : qq, quad | (kc.xl ? 2 : 1));
             Km = fp_max_pos(run.dt, lane_get(qq, quad | 1));
             if (!moves) {
-                G = 1.0;
-                yG = 0.0;
+                if (kc.xl) W = -1.0, V = 0.0;
                 Km = run.dt;
             }
         }
-        double AAC = lane_get(w, quad | 1);
         bool doubt = wet & unsure;
 
         // ---- the lower point of this pass, unless the last narrow pass formed it ----
         double q0 = q0n, Qj_0 = Qj0n;
-        double r23u = r23, itu = it;
         if (__any_sync(0xffffffffu, pre)) {
             const double eK = lane_get(L.e0.Km, home), eG = lane_get(L.e0.G, home), ey = lane_get(L.e0.yG, home);
             const double eQ = lane_get(L.e0.Qmn, home), Qp = lane_get(L.Qj_0, home);
+            const bool old = kc.xl & !need0;
             bool d = false;
-            const QuadFlow a = quad_flow(r, quad, f, Qp, 0, need0 ? Km : eK, need0 ? G : eG, need0 ? yG : ey, it, AAC, r23,
-                                         p.sq_s0, kc, d);
+            const QuadFlow a = quad_flow(kc, quad, Qp, 0, need0 ? Km : eK, old ? neg_if(true, eG) : W, old ? ey : V, it, p.sq_s0, d);
             const double Qmn = need0 ? (wet ? a.Qmn : 0.0) : eQ;
             const double res = lane_get(a.q - Qmn, lane | 4), qa = lane_get(a.q, lane | 4);
             if (pre) {
@@ -241,15 +275,13 @@ __device__ __forceinline__ bool narrow_passes(Lane& L, unsigned smask, const Run
             }
             // quad B goes on with the upper evaluation
             Km = lane_get(Km, lane & ~4);
-            G = lane_get(G, lane & ~4);
-            yG = lane_get(yG, lane & ~4);
-            r23u = lane_get(r23, lane & ~4);
-            itu = lane_get(it, lane & ~4);
-            AAC = lane_get(AAC, lane & ~4);
+            W = lane_get(W, lane & ~4);
+            V = lane_get(V, lane & ~4);
+            it = lane_get(it, lane & ~4);
         }
 
         // ---- quad A: upper coefficients of this pass; quad B: lower ones of the next ----
-        const QuadFlow a = quad_flow(r, quad, f, B ? Qj_0 : q0, B ? 0 : 0x3fe00000, Km, G, yG, itu, AAC, r23u, p.sq_s0, kc, doubt);
+        const QuadFlow a = quad_flow(kc, quad, B ? Qj_0 : q0, B ? 0 : 0x3fe00000, Km, W, V, it, p.sq_s0, doubt);
         const bool flowing = (__double2hiint(h) | __double2loint(h)) != 0;
         const double Qmn = flowing ? a.Qmn : 0.0;
         const double res = a.q - Qmn;
@@ -259,25 +291,29 @@ __device__ __forceinline__ bool narrow_passes(Lane& L, unsigned smask, const Run
         const double Qj = lane_get(res, lane & ~7);
         const double hd = lane_get(diff, quad | 3);
         // lane 0: Qj (h_0 - h); lane 1: Qj_0 - Qj
-        const double n = __fma_rn((r & 1) ? kc.one : Qj, neg_if(r & 1, (r & 1) ? Qj : hd), (r & 1) ? Qj_0 : kc.neg_zero);
+        const double n = __fma_rn(Qj, (r & 1) ? kc.neg_one : hd, (r & 1) ? Qj_0 : kc.neg_zero);
         const double dQ = lane_get(n, quad | 1), num = lane_get(n, quad);
         const bool slope = !fp_eq0(dQ);
         bool d2 = false;
         const double q2 = near_quot(num, near_rcp(dQ), d2);
         double h_1 = slope ? h - q2 : h;
-        if (fp_lt0(h_1)) h_1 = h;
+        const bool back = fp_lt0(h_1);
+        if (back) h_1 = h;
         doubt |= slope & (d2 | !numerator_regular(num));
 
         // ---- the next pass here, if every solve goes on ----
         const unsigned bad = __ballot_sync(0xffffffffu, doubt);
         const double nh = fp_max0(h_1);
-        const bool on = ((bad >> (lane & ~7)) & 0xffu) == 0 && k + 1 <= left && !fp_lt_pos(nh, kMinDepth) &&
-                        secant_more(h, h_1, run.tol);
+        bool on = ((bad >> (lane & ~7)) & 0xffu) == 0 && k + 1 <= left && !fp_lt_pos(nh, kMinDepth);
+        if (__all_sync(0xffffffffu, on)) {
+            const bool sure = slope && !back && surely_more(h, q2, run.tol);
+            if (!__all_sync(0xffffffffu, sure)) on = secant_more(h, h_1, run.tol);
+        }
         if (__all_sync(0xffffffffu, on) && !__any_sync(0xffffffffu, leave(k))) {
-            e0.Km = Km;
-            e0.G = G;
-            e0.yG = yG;
-            e0.Qmn = Qmn;
+            Km_before = Km;
+            W_before = W;
+            V_before = V;
+            Qmn_before = Qmn;
             Qj_before = Qj_0;
             h_0 = fp_max0(h);
             h = nh;
@@ -303,10 +339,10 @@ __device__ __forceinline__ bool narrow_passes(Lane& L, unsigned smask, const Run
             }
             if (bad) {
                 DepthEval b;
-                b.Km = lane_get(e0.Km, src);
-                b.G = lane_get(e0.G, src);
-                b.yG = lane_get(e0.yG, src);
-                b.Qmn = lane_get(e0.Qmn, src);
+                b.Km = lane_get(Km_before, src);
+                b.G = neg_if(true, lane_get(W_before, src + 1));
+                b.yG = lane_get(V_before, src + 1);
+                b.Qmn = lane_get(Qmn_before, src);
                 const double qb = lane_get(Qj_before, src);
                 if (member) {
                     L.e0 = b;
@@ -316,8 +352,8 @@ __device__ __forceinline__ bool narrow_passes(Lane& L, unsigned smask, const Run
         }
         DepthEval e;
         e.Km = lane_get(Km, src);
-        e.G = lane_get(G, src);
-        e.yG = lane_get(yG, src);
+        e.G = neg_if(true, lane_get(W, src + 1));
+        e.yG = lane_get(V, src + 1);
         e.Qmn = lane_get(Qmn, src);
         PassOut po;
         po.Qj_0 = lane_get(Qj_0, src);
