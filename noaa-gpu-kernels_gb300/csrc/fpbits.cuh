@@ -110,14 +110,18 @@ namespace tr {
 
 __device__ __forceinline__ int dexp(double x) { return (int)(((unsigned long long)dbits(x) >> 52) & 0x7ff); }
 
-// Quotients with three FP64 instructions each on a shared reciprocal of three.
+// Quotients with three FP64 instructions each on a shared reciprocal of two.
 //
-// near_rcp: y = 1/b within (1/2 + 2^-11) ulp. A single-precision reciprocal of
-// b's significand (relative error below 2^-21.9, argument truncation included)
-// is scaled on the integer pipe to y0; with e = RN(1 - b y0) the cubic step
-// y = RN(y0 + y0 (e + e^2)) leaves e^3 < 2^-65 before its own rounding (the
-// Newton-Raphson / Householder family, e.g. Muller et al., Handbook of
-// Floating-Point Arithmetic, chapter on division with an FMA).
+// near_rcp: y = 1/b within (1/2 + 2^-28) ulp. The single-precision reciprocal of
+// the leading 24 bits of b's significand, corrected by its residual against the
+// whole significand (first-order, in single precision: |1 - m s| < 2^-22, so that
+// the second-order term, the rounding of the correction to 2^-43 and those of the
+// residual leave a relative error below 2^-42), is scaled on the integer pipe to
+// y0; with e = RN(1 - b y0) the step y = RN(y0 + y0 e) leaves e^2 < 2^-84 before its
+// own rounding (the Newton-Raphson family, e.g. Muller et al., Handbook of
+// Floating-Point Arithmetic, chapter on division with an FMA). From the plain
+// single-precision seed the step has to be cubic, one FP64 instruction of 64 cycles
+// more; the correction is a chain of seven instructions of 4 to 5.
 //
 // near_quot: q0 = RN(a y), r = RN(a - b q0), q = RN(q0 + r y). y's error and
 // q0's rounding put q0 at most 1.5 ulp (+2^-11) from a/b (1 ulp when a's
@@ -158,11 +162,28 @@ __device__ __forceinline__ double rcp_seed(double b)
     return __hiloint2double(yh, sb << 29);
 }
 
+// 1/b with a relative error below 2^-42
+__device__ __forceinline__ double rcp_seed_fine(double b)
+{
+    const int hi = __double2hiint(b), lo = __double2loint(b);
+    const float m = __int_as_float((__funnelshift_l(lo, hi, 3) & 0x7fffff) | 0x3f800000);
+    const float ml = __fadd_rn(__int_as_float(((lo & 0x1fffffff) >> 6) | 0x3f800000), -1.0f);   // the rest times 2^23
+    float s;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(m));
+    s = fmaxf(s, 0.5f);
+    const float d = __fmaf_rn(ml, __fmul_rn(s, -0x1p-23f), __fmaf_rn(-m, s, 1.0f));
+    // s d in units of 2^-43, which are 2^10 units in the last place of a double in
+    // [1/2, 1) (s = 1 only for m = 1, where d <= 0 and the sum lies there too)
+    const int c = __float_as_int(__fmaf_rn(__fmul_rn(s, 0x1p43f), d, 12582912.0f)) - 0x4b400000;
+    const int sb = __float_as_int(s);
+    const int yh = ((sb >> 3) + (1919 << 20) - (hi & 0x7ff00000)) | (hi & 0x80000000);
+    return __longlong_as_double((((long long)yh << 32) | (unsigned)(sb << 29)) + (long long)c * 1024);
+}
+
 __device__ __forceinline__ NearRcp near_rcp(double b)
 {
-    const double y0 = rcp_seed(b);
-    const double e = __fma_rn(-b, y0, 1.0);
-    return {b, __fma_rn(y0, __fma_rn(e, e, e), y0)};
+    const double y0 = rcp_seed_fine(b);
+    return {b, __fma_rn(y0, __fma_rn(-b, y0, 1.0), y0)};
 }
 
 // Whether the quotient near q0 with residual r may round differently (see above).

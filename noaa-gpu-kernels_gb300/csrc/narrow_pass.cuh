@@ -288,11 +288,10 @@ __device__ __forceinline__ bool narrow_passes(Lane& L, unsigned smask, const Run
         doubt |= !B & fp_lt0(a.q);   // the negative-flow fallbacks (troute_mc_final.cu:125-130)
 
         // ---- secant step, on every lane of the octet ----
-        const double Qj = lane_get(res, lane & ~7);
+        // quad A, whose res is Qj: even lanes Qj (h_0 - h), odd ones Qj_0 - Qj
         const double hd = lane_get(diff, quad | 3);
-        // lane 0: Qj (h_0 - h); lane 1: Qj_0 - Qj
-        const double n = __fma_rn(Qj, (r & 1) ? kc.neg_one : hd, (r & 1) ? Qj_0 : kc.neg_zero);
-        const double dQ = lane_get(n, quad | 1), num = lane_get(n, quad);
+        const double n = __fma_rn(res, (r & 1) ? kc.neg_one : hd, (r & 1) ? Qj_0 : kc.neg_zero);
+        const double dQ = lane_get(n, (lane & ~7) | 1), num = lane_get(n, lane & ~7);
         const bool slope = !fp_eq0(dQ);
         bool d2 = false;
         const double q2 = near_quot(num, near_rcp(dQ), d2);
