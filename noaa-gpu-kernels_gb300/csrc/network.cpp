@@ -951,7 +951,8 @@ static int enqueue_chunk(troute_handle* H, const double* qlat_dev, int n_ts, con
         df.rq_head = H->rq_ctr.p;
         df.rq_tail = H->rq_ctr.p + 1;
         df.n_done = H->rq_ctr.p + 2;
-        df.n_avail = reinterpret_cast<int*>(H->rq_ctr.p + 3);
+        df.n_avail = reinterpret_cast<int2*>(H->rq_ctr.p + 3);
+        df.head_head = H->rq_ctr.p + 4;
         df.rh = H->df_rh.p;
         df.heads = H->df_heads.p;
         df.n_heads = H->n_heads;
@@ -1052,7 +1053,7 @@ static int prepare_run(troute_handle* H, int n_ts, RunPlan* P)
         const size_t R = (size_t)std::max(1, H->n_item);
         const size_t T = (size_t)P->chunk;
         if ((rc = H->df_cnt.alloc(T * R)) || (rc = H->df_rh.alloc((T + 1) * R)) ||
-            (rc = H->df_rq.alloc(R * T)) || (rc = H->rq_ctr.alloc(4)))
+            (rc = H->df_rq.alloc(R * T)) || (rc = H->rq_ctr.alloc(5)))
             return rc;
     }
     return TROUTE_OK;

@@ -186,7 +186,9 @@ struct DataflowDev {
     unsigned long long* rq_head;    // claimed slots
     unsigned long long* rq_tail;    // written slots
     unsigned long long* n_done;     // completed items
-    int* n_avail;                   // queued items no warp has claimed (down to minus the claims in flight)
+    int2* n_avail;                  // items no warp has claimed (down to minus the claims in flight): .x of the
+                                    // heads, .y of the queue
+    unsigned long long* head_head;  // claimed heads
     double* rh;                     // [n_ts + 1][n_item] outflow per step
     const int2* heads;              // (item without upstream, 0), ready at the start
     int n_heads;
