@@ -189,6 +189,9 @@ def measured_peak_hbm():
         return 6800.0, "fallback"
 
 
+PASSES = "route_dataflow_passes.md"   # FP64 warp instructions of the routing kernel's passes
+
+
 def profiled_file(key: str, name: str):
     """A `key: value` figure from a committed ncu summary under profiles/."""
     p = os.path.join(ROOT, "profiles", name)
@@ -210,15 +213,15 @@ def profiled(key: str, warm: bool):
 def critical_path_bound(T, w, n_ts: int, it_per_solve: float, sm_mhz, kernel_ms: float) -> dict:
     """The dependency graph's critical path of one bench step set against the
     FP64 pipe: the longest chain of segment solves (troute_critical_path), each
-    solve at least (iterations + 1) passes, each pass at least its FP64 warp
-    instructions x 64 cycles (one FP64 warp instruction per 64 cycles per
+    solve (iterations + 1) passes, each pass at least the FP64 warp instructions
+    of a narrow pass x 64 cycles (one FP64 warp instruction per 64 cycles per
     SMSP, however few lanes are busy)."""
     if "batch" in w:
         chain = max(T.critical_path(n["topo"], n_ts) for n in w["batch"])
     else:
         chain = T.critical_path(w["topo"], n_ts)
     out = {"segment_solves": chain, "passes_per_solve": it_per_solve + 1.0}
-    instr, src = profiled_file("fp64_instr_per_solving_pass", "route_dataflow_instmix_tree200k.md")
+    instr, src = profiled_file("fp64_instr_narrow_pass", PASSES)
     if instr is None:
         return out
     pass_us = instr * 64.0 / float(sm_mhz or 2070.0)
@@ -725,7 +728,8 @@ def run_ours(args, dist: Dist):
 
     # roofline: the FP64 pipe (the bound) from this run's own solving warp passes,
     # against the measured FP64 issue rate; the HBM fraction beside it
-    instr, instr_src = profiled_file("fp64_instr_per_solving_pass", "route_dataflow_instmix_tree200k.md")
+    instr, instr_src = profiled_file("fp64_instr_mean_pass_" + ("batched" if "members" in w or "batch" in w else "single"),
+                                     PASSES)
     fp64_warp_instr = stats["solve_passes"] * (instr or 0.0)
     achieved = fp64_warp_instr * 32 / (kernel_ms / 1e3) / 1e12
     peak = fp64_rate["warp_instr_per_s"] * 32 / 1e12

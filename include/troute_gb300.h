@@ -54,7 +54,7 @@ typedef struct troute_cfg {
     double atol;            /* absolute depth change that ends the secant loop */
     int maxiter;            /* iteration cap of the first attempt (+25 per retry) */
     int attempts;           /* bracket-widening attempts */
-    int threads_per_block;  /* 0: autotuned / default */
+    int threads_per_block;  /* 0: autotuned / default (mapping 1) */
     int blocks_per_sm;      /* 0: occupancy-derived */
     long long wait_cycles;  /* bound on each device-side wait without progress, SM clocks; 0: ~4 s */
     int warm_start;         /* 1: learned warm start (needs troute_set_warm_start; mapping 3) */
@@ -63,7 +63,8 @@ typedef struct troute_cfg {
     int mapping;            /* reach-to-warp mapping: 0 auto (3), 1 one level-block per
                                warp, 2 per-lane refill in level-block order,
                                3 per-lane refill from the ready queue */
-    int schedule_flags;     /* mapping 3, bit 0: a lane continues with an item it made ready */
+    int schedule_flags;     /* mapping 3, bit 0: a lane continues with an item it made ready in
+                               every warp (0: in warps of at most four items) */
     int max_chunk_steps;    /* steps routed per launch (0: as many as a third of free memory allows) */
     int record_pairs;       /* 1: every solve of a run keeps its training pair (troute_get_pairs) */
     int record_start;       /* 1: every solve of a run keeps its learned starting depth

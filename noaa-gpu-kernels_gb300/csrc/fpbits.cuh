@@ -78,35 +78,8 @@ __device__ __forceinline__ bool fp_abs_gt(double a, double b)
 // as IEEE maxNum returns the non-NaN operand)
 __device__ __forceinline__ double fp_max0(double x) { return fp_gt0(x) ? x : 0.0; }
 
-// fmin(c, x) for c > 0 not NaN and x >= +0 or NaN (a NaN x gives c), and
 // fmax(c, x) for c > 0 not NaN and any x (x <= c or NaN gives c)
-__device__ __forceinline__ double fp_min_pos(double c, double x)
-{
-    const long long b = dbits(x);
-    return (b >= 0 && b < dbits(c)) ? x : c;
-}
 __device__ __forceinline__ double fp_max_pos(double c, double x) { return fp_gt_pos(x, c) ? x : c; }
-
-// 2.0 * a * b * c * d as the reference writes it, (((2a) b) c) d, given the
-// undoubled chain g1 = a b, g2 = g1 c, g = g2 d (all positive). Doubling
-// commutes with rounding while a product stays in the normal range, so when
-// g1, g2 and g are at least 2^-1021 and 2g is finite the result is exactly
-// 2g, formed by raising g's exponent on the integer pipe; otherwise it is
-// evaluated as written.
-__device__ __forceinline__ double twice_chain(double g1, double g2, double g, double a, double b, double c, double d)
-{
-    const unsigned e1 = (unsigned)((unsigned long long)dbits(g1) >> 52) & 0x7ffu;
-    const unsigned e2 = (unsigned)((unsigned long long)dbits(g2) >> 52) & 0x7ffu;
-    const unsigned e3 = (unsigned)((unsigned long long)dbits(g) >> 52) & 0x7ffu;
-    // exponents 2..0x7fd: the exact products are normal and their doubles finite
-    if (e1 - 2u < 0x7fcu && e2 - 2u < 0x7fcu && e3 - 2u < 0x7fcu)
-        return __longlong_as_double(dbits(g) + (1ll << 52));
-    return 2.0 * a * b * c * d;
-}
-
-}  // namespace tr
-
-namespace tr {
 
 __device__ __forceinline__ int dexp(double x) { return (int)(((unsigned long long)dbits(x) >> 52) & 0x7ff); }
 
@@ -253,17 +226,5 @@ __device__ __forceinline__ bool quot_gt_pos(double a, double b, double c)
 
 // |x| on the integer pipe
 __device__ __forceinline__ double fp_abs(double x) { return __longlong_as_double(dbits(x) & 0x7fffffffffffffffll); }
-
-// x is finite (not infinite, not NaN)
-__device__ __forceinline__ bool fp_finite(double x) { return (dbits(x) & kInfBits) != kInfBits; }
-
-// 0.5 * x: for an exponent field of 2..0x7fe the product is x with the field
-// lowered by one, exactly (the result stays normal); zeros, subnormals,
-// the smallest normals, infinities and NaN take the multiplication.
-__device__ __forceinline__ double fp_half(double x)
-{
-    const unsigned e = (unsigned)((unsigned long long)dbits(x) >> 52) & 0x7ffu;
-    return (e - 2u < 0x7fdu) ? __longlong_as_double(dbits(x) - (1ll << 52)) : 0.5 * x;
-}
 
 }  // namespace tr

@@ -24,7 +24,7 @@
 // A pass exists in two forms with the same results bit for bit.
 //  - secant_pass: what the solves run. The FP64 pipe bounds every routing
 //    kernel (one FP64 warp instruction holds an SMSP's pipe for 64 cycles), so
-//    the pass is written to issue few of them: about 148 in bank, against 237
+//    the pass is written to issue few of them: about 141 in bank, against 237
 //    before (IEEE divisions, 5-instruction shared quotients, 35-instruction
 //    powers, the lower depth's X denominator formed anew). Quotients and powers
 //    come from near_quot and pow23_53_near, decisions are taken on the integer

@@ -4,8 +4,10 @@
 // instruction costs 64-66 cycles whatever the number of its active lanes
 // (measured, dependent or not, with one to four warps per SM): the time of a
 // run is then the longest chain of passes times the FP64 instructions of a
-// pass. Here the idle lanes take part, so that a pass issues 64 FP64 warp
-// instructions instead of 148:
+// pass. Here the idle lanes take part, so that a pass issues 67 FP64 warp
+// instructions instead of 141 (a lone warp: 6.4 k cycles a pass against 12.0 k; three
+// warps per scheduler share its FP64 pipe, so that from five solves on the full pass
+// is the better one):
 //  - the eight lanes of a solve form two quads. Within a quad the lanes evaluate
 //    at the same time what one lane evaluates in turn: the geometry's linear
 //    forms, the reciprocals (wetted perimeter, top width; celerity, conveyance),

@@ -1,8 +1,9 @@
 // Persistent tree routing driven by a ready queue (reach-to-warp mapping 3).
 //
-// The (reach, step) items of a run form a DAG: (r, t) needs (u, t) for every
-// upstream reach u (its current-step outflow, the reach head's quc) and
-// (r, t-1) (its own previous state). Instead of handing items out in a fixed
+// The (item, step) pairs of a run form a DAG, an item r being a reach or a piece of
+// one (item_segments in network.cpp): (r, t) needs (u, t) for every upstream item u
+// (its current-step outflow, the item head's quc) and (r, t-1) (its own previous
+// state). Instead of handing items out in a fixed
 // order and letting lanes wait on them, each item carries a counter of
 // completed dependencies; the lane that completes the last dependency of an
 // item appends the item to a global ready queue, and idle lanes pop only from
@@ -17,9 +18,10 @@
 //               nothing else is ready
 //   rq[i]       the other items in the order they became ready (atomic tail);
 //               idle lanes claim slots (atomic head); -1 = not yet written
-//   rh[t+1][r]  outflow of reach r at step t of this run, rh[0][r] the
+//   rh[t+1][r]  outflow of item r at step t of this run, rh[0][r] the
 //               outflow of the step before the run (from the 4-slot ring of
-//               the handle's state); a whole run is kept, so upstream reaches
+//               the handle's state, within a reach from the discharge); a whole
+//               run is kept, so upstream reaches
 //               never wait for downstream ones to consume a value.
 // In a warp of few items (and with continue_items in every warp) the lane that
 // makes an item ready continues with it itself (the downstream item when two
@@ -172,7 +174,7 @@ __device__ __forceinline__ void start_item(Lane& L, int ri, int tau, int t_base,
 
 // Threads per block, and the register budget: resident blocks per SM the
 // allocation is sized for, or (TROUTE_DF_MAXNREG) a register cap. Three blocks
-// of 128 (164 registers; 178 without the bound, which would leave two): four
+// of 128 (168 registers; 178 without the bound, which would leave two): four
 // blocks spill 176 B and are slower everywhere (64 members of a 20,000-segment
 // tree, warm start, 16 steps: 128.5 against 124.0 ms; a 200,000-segment tree, 24
 // steps: 218 against 196 ms), 64-thread blocks at 14-16 warps likewise.
