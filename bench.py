@@ -212,7 +212,9 @@ def profiled(key: str, warm: bool):
 
 def critical_path_bound(T, w, n_ts: int, it_per_solve: float, sm_mhz, kernel_ms: float) -> dict:
     """The dependency graph's critical path of one bench step set against the
-    FP64 pipe: the longest chain of segment solves (troute_critical_path), each
+    FP64 pipe: the longest chain of segment solves when a reach takes its steps
+    one after another (troute_critical_path; networks of up to 1,048,576 segments
+    are routed in pieces of reaches, whose chain is shorter), each
     solve (iterations + 1) passes, each pass at least the FP64 warp instructions
     of a narrow pass x 64 cycles (one FP64 warp instruction per 64 cycles per
     SMSP, however few lanes are busy)."""
