@@ -13,6 +13,7 @@
 #include <cstring>
 #include <vector>
 
+#include "train_buffers.h"
 #include "warm.cuh"
 
 namespace tr {
@@ -22,7 +23,6 @@ namespace tr {
 constexpr int kP_W1 = 0, kP_B1 = kP_W1 + kWHid * kWIn, kP_W2 = kP_B1 + kWHid, kP_B2 = kP_W2 + kWHid * kWHid,
               kP_W3 = kP_B2 + kWHid, kP_B3 = kP_W3 + kWHid, kNParams = kP_B3 + 1;
 constexpr int kPairW = 9;  // qup quc qdp ql dx s0 n bw depth
-constexpr int kTrainRows = 64;
 
 struct Norm {
     float mu[kWIn], sd[kWIn], mu_y, sd_y;
@@ -105,7 +105,6 @@ __global__ void __launch_bounds__(kMomThreads) warm_moments_kernel(const float* 
 // instructions on 2 x 4 tiles of 512 threads were no faster.)
 constexpr int kGemmThreads = 256, kChoreThreads = 128;
 constexpr int kTLd = 68;         // row of a 64-wide tile: 16-byte aligned, banks shifted by 4
-constexpr int kPartLd = 4804;    // row of the partial gradients, 16-byte aligned
 static_assert(kTrainRows == 64 && kWHid == 64 && kPartLd >= kNParams && kPartLd % 4 == 0 && kP_W2 % 4 == 0, "tile shapes");
 
 // The update: kUpdateRows threads per parameter fetch the partials of kUpdateTiles
@@ -150,11 +149,6 @@ __device__ __forceinline__ void tile_step(float (&acc)[4][4], const float (&u)[4
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] += u[i] * v[j];
 }
-
-// AdamW constants of a step.
-struct AdamStep {
-    float lr, c1, c2;
-};
 
 struct TrainArgs {
     const float* pairs;
@@ -588,23 +582,18 @@ struct troute_warm {
     Norm nm;
     bool trained = false;
     // device: fp32 master copy, AdamW moments, gradient; bf16 inference layout;
-    // per-block partial gradients / losses / moments of the training kernels
+    // epoch loss, per-block moments, grid barrier and buffers of the training launches
     float *d_prm = nullptr, *d_m = nullptr, *d_v = nullptr, *d_g = nullptr;
     __nv_bfloat16 *d_w1t = nullptr, *d_w2t = nullptr, *d_w3t = nullptr;
     float *d_b1 = nullptr, *d_b2 = nullptr;
     double *d_loss = nullptr, *d_mom = nullptr;
-    float* d_part = nullptr;
-    double* d_lpart = nullptr;   // block and step losses
-    float* d_err = nullptr;      // (err^2)/2 of the samples of the steps kept
-    unsigned* d_bar = nullptr;   // grid barrier
-    AdamStep* d_step = nullptr;  // AdamW constants of the steps kept
-    int part_blocks = 0;
-    size_t lpart_n = 0;
+    unsigned* d_bar = nullptr;
+    TrainBuffers buf;
 
     ~troute_warm()
     {
         for (void* p : {(void*)d_prm, (void*)d_m, (void*)d_v, (void*)d_g, (void*)d_w1t, (void*)d_w2t, (void*)d_w3t,
-                        (void*)d_b1, (void*)d_b2, (void*)d_loss, (void*)d_mom, (void*)d_part, (void*)d_lpart, (void*)d_err, (void*)d_bar, (void*)d_step})
+                        (void*)d_b1, (void*)d_b2, (void*)d_loss, (void*)d_mom, (void*)d_bar})
             if (p) cudaFree(p);
     }
 };
@@ -636,43 +625,13 @@ static int warm_alloc(troute_warm* w)
     return TROUTE_OK;
 }
 
-// Room for the partial gradients of a mini-batch of nblocks blocks, and for the
-// block losses of `steps` of them with a sum each.
-static int warm_parts(troute_warm* w, int nblocks, int steps)
-{
-    int rc;
-    if (nblocks > w->part_blocks) {
-        if (w->d_part) cudaFree(w->d_part);
-        w->d_part = nullptr;
-        w->part_blocks = 0;
-        if ((rc = warm_cuda(cudaMalloc(&w->d_part, (size_t)nblocks * kPartLd * sizeof(float)), "cudaMalloc"))) return rc;
-        w->part_blocks = nblocks;
-    }
-    const size_t need = (size_t)steps * ((size_t)nblocks + 1);
-    if (need > w->lpart_n) {
-        if (w->d_lpart) cudaFree(w->d_lpart);
-        if (w->d_err) cudaFree(w->d_err);
-        if (w->d_step) cudaFree(w->d_step);
-        w->d_lpart = nullptr;
-        w->d_err = nullptr;
-        w->d_step = nullptr;
-        w->lpart_n = 0;
-        if ((rc = warm_cuda(cudaMalloc(&w->d_lpart, need * sizeof(double)), "cudaMalloc")) ||
-            (rc = warm_cuda(cudaMalloc(&w->d_err, (size_t)steps * nblocks * kTrainRows * sizeof(float)), "cudaMalloc")) ||
-            (rc = warm_cuda(cudaMalloc(&w->d_step, (size_t)steps * sizeof(AdamStep)), "cudaMalloc")))
-            return rc;
-        w->lpart_n = need;
-    }
-    return TROUTE_OK;
-}
-
 // Adds the losses of `steps` steps of `tiles` tiles each (their samples from
 // sq_err on) to *d_loss.
 static int warm_add_losses(troute_warm* w, const float* sq_err, int tiles, int steps)
 {
     const long long blocks = (long long)tiles * steps;
-    warm_block_loss_kernel<<<(unsigned)((blocks + 127) / 128), 128>>>(sq_err, blocks, w->d_lpart);
-    warm_loss_kernel<<<1, 256>>>(w->d_lpart, tiles, steps, w->d_lpart + blocks, w->d_loss);
+    warm_block_loss_kernel<<<(unsigned)((blocks + 127) / 128), 128>>>(sq_err, blocks, w->buf.loss.p);
+    warm_loss_kernel<<<1, 256>>>(w->buf.loss.p, tiles, steps, w->buf.loss.p + blocks, w->d_loss);
     return warm_cuda(cudaGetLastError(), "loss launch");
 }
 
@@ -695,8 +654,8 @@ static int warm_train(troute_warm* w, TrainArgs& a)
     a.grad = w->d_g;
     a.m = w->d_m;
     a.v = w->d_v;
-    a.part = w->d_part;
-    a.sq_err = w->d_err;
+    a.part = w->buf.part.p;
+    a.sq_err = w->buf.err.p;
     a.barrier = w->d_bar;
     if ((rc = warm_cuda(cudaMemsetAsync(w->d_bar, 0, 2 * sizeof(unsigned), nullptr), "memset"))) return rc;
     void* args[] = {&a};
@@ -708,8 +667,8 @@ static int warm_train(troute_warm* w, TrainArgs& a)
     const long long last = std::min<long long>(a.batch, a.end - a.offset - (long long)(a.steps - 1) * a.batch);
     const int last_tiles = (int)((last + kTrainRows - 1) / kTrainRows);
     const int full = last_tiles == tiles ? a.steps : a.steps - 1;
-    if (full && (rc = warm_add_losses(w, w->d_err, tiles, full))) return rc;
-    if (full < a.steps && (rc = warm_add_losses(w, w->d_err + (size_t)full * a.batch, last_tiles, 1))) return rc;
+    if (full && (rc = warm_add_losses(w, w->buf.err.p, tiles, full))) return rc;
+    if (full < a.steps && (rc = warm_add_losses(w, w->buf.err.p + (size_t)full * a.batch, last_tiles, 1))) return rc;
     return TROUTE_OK;
 }
 
@@ -882,11 +841,9 @@ extern "C" int troute_warm_fit(troute_warm* w, const float* pairs_dev, long long
     const long long steps_per_epoch = (n_pairs + batch - 1) / batch;
     const long long total = steps_per_epoch * epochs;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    // steps per launch: their samples' losses are kept and summed afterwards (64
-    // doubles in order take as long as a tile's products)
     const int tiles = batch / kTrainRows;
-    const int keep = (int)std::min<long long>(steps_per_epoch, std::max(1, (1 << 16) / tiles));
-    if ((rc = warm_parts(w, tiles, keep))) return rc;
+    const int keep = train_steps_kept(steps_per_epoch, tiles);
+    if ((rc = warm_cuda(w->buf.reserve(tiles, keep), "cudaMalloc"))) return rc;
     std::vector<AdamStep> consts((size_t)keep);
     long long step = 0;
     for (int ep = 0; ep < epochs; ++ep) {
@@ -897,7 +854,7 @@ extern "C" int troute_warm_fit(troute_warm* w, const float* pairs_dev, long long
         a.batch = batch;
         a.perm_a = coprime_near((unsigned long long)n_pairs, hash3(seed, 31, ep) | 1ull);
         a.perm_b = hash3(seed, 37, ep) % (unsigned long long)n_pairs;
-        a.step = w->d_step;
+        a.step = w->buf.step.p;
         a.b1 = b1;
         a.b2 = b2;
         a.eps = eps;
@@ -914,7 +871,7 @@ extern "C" int troute_warm_fit(troute_warm* w, const float* pairs_dev, long long
                 consts[k].c2 = 1.0f - std::pow(b2, (float)(step + 1));
             }
             // (a pageable copy: ordered after the launch before, and done when it returns)
-            if ((rc = warm_cuda(cudaMemcpy(w->d_step, consts.data(), (size_t)a.steps * sizeof(AdamStep), cudaMemcpyHostToDevice),
+            if ((rc = warm_cuda(cudaMemcpy(w->buf.step.p, consts.data(), (size_t)a.steps * sizeof(AdamStep), cudaMemcpyHostToDevice),
                                 "step constants")) ||
                 (rc = warm_train(w, a)) || (rc = warm_train_status(w)))
                 return rc;
@@ -940,7 +897,7 @@ extern "C" int troute_warm_grad(troute_warm* w, const float* pairs_host, int n, 
     rc = warm_cuda(cudaMemcpy(d_pairs, pairs_host, (size_t)n * kPairW * sizeof(float), cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = warm_cuda(cudaMemcpy(w->d_prm, w->prm, sizeof w->prm, cudaMemcpyHostToDevice), "H2D");
     if (!rc) rc = warm_cuda(cudaMemset(w->d_loss, 0, sizeof(double)), "memset");
-    if (!rc) rc = warm_parts(w, (n + kTrainRows - 1) / kTrainRows, 1);
+    if (!rc) rc = warm_cuda(w->buf.reserve((n + kTrainRows - 1) / kTrainRows, 1), "cudaMalloc");
     TrainArgs a = {};
     a.pairs = d_pairs;
     a.n = n;
