@@ -46,7 +46,8 @@ struct DevPtr {
     ~DevPtr() { if (p) cudaFree(p); }
 };
 
-// Counter buffers of troute_mc_reach_parallel_device: one per (host thread,
+// Statistics buffers of troute_mc_reach_parallel_device, which nothing reads back
+// (overlapping calls of a thread may mix theirs): one per (host thread,
 // device), so a thread that switches devices never hands a kernel another
 // GPU's memory, and two threads never share one. Freed when the thread exits
 // (errors ignored: at process exit the runtime may already be unloading).

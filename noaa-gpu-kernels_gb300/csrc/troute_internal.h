@@ -125,7 +125,6 @@ struct DevStats {
     int err_reach;   // internal reach of the first failure
     int err_step;    // step of the first failure
     int err_where;   // 1 own, 2 upstream, 3 downstream back-pressure, 4 bounds
-    unsigned long long ticket;   // reaches handed out (reach-parallel step)
 };
 
 // Static network description on the device (internal order).
