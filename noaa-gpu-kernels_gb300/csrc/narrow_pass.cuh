@@ -158,6 +158,10 @@ template <typename Leave>
 __device__ __forceinline__ bool narrow_passes(Lane& L, unsigned smask, const RunDev& run, double2* warp_seg, PassOut& o,
                                               int& extra, Leave leave)
 {
+    // The solves' own lanes filled the segment buffers (plain stores, or cp.async they
+    // waited for) that the other lanes read here, and may fill them again afterwards;
+    // shuffles and votes order no memory, so the barriers here and behind the loop do.
+    __syncwarp();
     const int lane = threadIdx.x & 31;
     const int r = lane & 3, quad = lane & ~3;
     const bool B = lane & 4;
@@ -326,6 +330,7 @@ __device__ __forceinline__ bool narrow_passes(Lane& L, unsigned smask, const Run
         }
 
         // ---- back to the solve's own lane ----
+        __syncwarp();
         const int src = (8 * __popc(smask & ((1u << lane) - 1u))) & 31;
         const bool member = (smask >> lane) & 1u;
         extra = k;
