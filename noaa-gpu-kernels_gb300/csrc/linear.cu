@@ -494,18 +494,19 @@ struct DArr {
     int alloc(size_t count)
     {
         if (count <= n && p) return TROUTE_OK;
-        if (p) cudaFree(p);
-        p = nullptr;
-        n = 0;
+        release();
         const cudaError_t e = cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T));
         if (e != cudaSuccess) return set_error(TROUTE_ENOMEM, "cudaMalloc: %s", cudaGetErrorString(e));
         n = count;
         return TROUTE_OK;
     }
-    ~DArr()
+    void release()
     {
         if (p) cudaFree(p);
+        p = nullptr;
+        n = 0;
     }
+    ~DArr() { release(); }
 };
 
 int lin_cuda(cudaError_t e, const char* what)
@@ -572,14 +573,6 @@ extern "C" int troute_linear_coeffs(const troute_chparams_f32* params, int n_seg
         c4oq[i] = h[i].w;
     }
     return TROUTE_OK;
-}
-
-template <typename T>
-static int lin_upload(DArr<T>& arr, const std::vector<T>& v)
-{
-    const int rc = arr.alloc(v.size());
-    if (rc || v.empty()) return rc;
-    return lin_cuda(cudaMemcpy(arr.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice), "upload");
 }
 
 // Paths and the segments in path order of a validated network.
@@ -661,17 +654,26 @@ static int lin_build(troute_linear* L, const troute_topo* topo, const float* c1,
 }
 
 // The sweeps of 2^k shallow paths each, of one depth (a path may wait for a
-// shallower one, never for one in its own warp).
-static int lin_items(troute_linear* L, int k)
+// shallower one, never for one in its own warp). Copied on the stream of the kernel
+// that reads them: a copy on the legacy stream may still be on its way then.
+static int lin_items(troute_linear* L, int k, cudaStream_t st)
 {
     if (L->items[k].p) return TROUTE_OK;
     std::vector<int2> v;
     const int w = 1 << k;
-    for (size_t d = 0; d + 1 < L->depth_ptr.size(); ++d)
-        for (int p = L->depth_ptr[d]; p < std::min(L->depth_ptr[d + 1], L->deep_from); p += w)
-            v.push_back(int2{p, std::min(w, std::min(L->depth_ptr[d + 1], L->deep_from) - p)});
-    L->n_items[k] = (int)v.size();
-    return lin_upload(L->items[k], v);
+    try {
+        for (size_t d = 0; d + 1 < L->depth_ptr.size(); ++d)
+            for (int p = L->depth_ptr[d]; p < std::min(L->depth_ptr[d + 1], L->deep_from); p += w)
+                v.push_back(int2{p, std::min(w, std::min(L->depth_ptr[d + 1], L->deep_from) - p)});
+    } catch (const std::bad_alloc&) {
+        return set_error(TROUTE_ENOMEM, "linear sweeps: host memory");
+    }
+    int rc = L->items[k].alloc(v.size());
+    if (!rc && !v.empty())
+        rc = lin_cuda(cudaMemcpyAsync(L->items[k].p, v.data(), v.size() * sizeof(int2), cudaMemcpyHostToDevice, st), "upload");
+    if (rc) L->items[k].release();
+    else L->n_items[k] = (int)v.size();
+    return rc;
 }
 
 extern "C" int troute_linear_create(troute_linear** out, const troute_topo* topo, const float* c1, const float* c2,
@@ -772,7 +774,7 @@ extern "C" int troute_linear_run_device(troute_linear* L, const float* qlat_dev,
         // shallow paths: 8 steps per lane, up to 8 lanes each
         int lc = 0;
         while (lc < 3 && (8 << lc) < d.T) ++lc;
-        if ((rc = lin_items(L, 5 - lc))) return rc;
+        if ((rc = lin_items(L, 5 - lc, st))) return rc;
         d.items = L->items[5 - lc].p;
         d.n_items = L->n_items[5 - lc];
         if ((rc = lin_cuda(cudaMemsetAsync(L->out.p, 0xff, (size_t)L->n_paths * (size_t)d.Tp * sizeof(unsigned), st),
@@ -814,10 +816,11 @@ extern "C" int troute_linear_route(const troute_topo* topo, const float* c1, con
     if (rc) return rc;
     DArr<float> q, ql;
     if ((rc = q.alloc(S)) || (rc = ql.alloc((size_t)n_ts * S)) ||
-        (rc = lin_cuda(cudaMemcpy(q.p, q0, S * sizeof(float), cudaMemcpyHostToDevice), "H2D")) ||
-        (rc = lin_cuda(cudaMemcpy(ql.p, qlat_ts, (size_t)n_ts * S * sizeof(float), cudaMemcpyHostToDevice), "H2D")) ||
+        (rc = lin_cuda(cudaMemcpyAsync(q.p, q0, S * sizeof(float), cudaMemcpyHostToDevice, L->stream), "H2D")) ||
+        (rc = lin_cuda(cudaMemcpyAsync(ql.p, qlat_ts, (size_t)n_ts * S * sizeof(float), cudaMemcpyHostToDevice, L->stream), "H2D")) ||
         (rc = troute_linear_run_device(L, ql.p, n_ts, q.p, 0, nullptr)) ||
-        (rc = lin_cuda(cudaMemcpy(q_out, q.p, S * sizeof(float), cudaMemcpyDeviceToHost), "D2H"))) {
+        (rc = lin_cuda(cudaMemcpyAsync(q_out, q.p, S * sizeof(float), cudaMemcpyDeviceToHost, L->stream), "D2H")) ||
+        (rc = lin_cuda(cudaStreamSynchronize(L->stream), "D2H"))) {
         troute_linear_destroy(L);
         return rc;
     }

@@ -576,6 +576,8 @@ extern "C" int troute_matrix_create(troute_matrix** out, int n_reaches, const in
             !(rc = up(M->long_rows.p, longs.data(), longs.size() * sizeof(int4))) &&
             !(rc = up(M->long_nl.p, longs_nl.data(), longs.size() * sizeof(int))))
             rc = up(M->rows.p, shorts.data(), shorts.size() * sizeof(int4));
+        // the copies may still be on their way, and the run's streams do not wait for this one
+        if (!rc) rc = mat_cuda(cudaStreamSynchronize(nullptr), "matrix upload");
     } catch (const std::bad_alloc&) {
         rc = set_error(TROUTE_ENOMEM, "matrix upload: host memory");
     }
@@ -712,8 +714,8 @@ extern "C" int troute_matrix_route(int n_reaches, const int* up_ptr, const int* 
     const size_t R = (size_t)n_reaches;
     MArr<float> q, ql;
     if ((rc = q.alloc(R)) || (rc = ql.alloc((size_t)n_ts * R)) ||
-        (rc = mat_cuda(cudaMemcpy(q.p, q0, R * sizeof(float), cudaMemcpyHostToDevice), "H2D")) ||
-        (rc = mat_cuda(cudaMemcpy(ql.p, qlat_ts, (size_t)n_ts * R * sizeof(float), cudaMemcpyHostToDevice), "H2D")) ||
+        (rc = mat_cuda(cudaMemcpyAsync(q.p, q0, R * sizeof(float), cudaMemcpyHostToDevice, M->stream), "H2D")) ||
+        (rc = mat_cuda(cudaMemcpyAsync(ql.p, qlat_ts, (size_t)n_ts * R * sizeof(float), cudaMemcpyHostToDevice, M->stream), "H2D")) ||
         (rc = troute_matrix_run_device(M, ql.p, n_ts, q.p, nullptr)) ||
         (rc = mat_cuda(cudaStreamSynchronize(M->stream), "matrix run")) ||
         (rc = mat_cuda(cudaMemcpy(q_out, q.p, R * sizeof(float), cudaMemcpyDeviceToHost), "D2H"))) {

@@ -699,7 +699,8 @@ static int warm_publish(troute_warm* w)
         (rc = warm_cuda(cudaMemcpy(w->d_b1, w->prm + kP_B1, kWHid * 4, cudaMemcpyHostToDevice), "H2D")) ||
         (rc = warm_cuda(cudaMemcpy(w->d_b2, w->prm + kP_B2, kWHid * 4, cudaMemcpyHostToDevice), "H2D")))
         return rc;
-    return TROUTE_OK;
+    // the routing streams that read them do not wait for this one
+    return warm_cuda(cudaStreamSynchronize(nullptr), "H2D");
 }
 
 namespace tr {
