@@ -289,7 +289,8 @@ struct DeepRing {
 };
 
 // The warp waits until *p >= want; false (for all its lanes) when the budget runs
-// out or another warp failed.
+// out or another warp failed. What was done before the flag was raised (behind a
+// fence) is then done for the warp.
 __device__ __forceinline__ bool wait_smem(const LinRun& d, const volatile int* p, int want)
 {
     bool ok = true;
@@ -301,6 +302,7 @@ __device__ __forceinline__ bool wait_smem(const LinRun& d, const volatile int* p
             ok = *reinterpret_cast<volatile int*>(d.error) == 0;
         }
     }
+    __threadfence_block();
     return __all_sync(kFull, ok);
 }
 
@@ -333,6 +335,7 @@ __global__ void __launch_bounds__(32 * (NP + 1), 1) lin_deep_kernel(const LinRun
                 for (int i = 0; i < rounds; ++i) {
                     if ((i & 7) == 0) {
                         __syncwarp();
+                        __threadfence_block();   // the rounds' reads, before their slots are filled again
                         if (c == 0) R.rounds = i;
                         if (i < n && !wait_smem(d, &R.full[(i >> 3) % (W / 8)], (i >> 3) + 1)) break;
                         __syncwarp();

@@ -29,3 +29,13 @@ def test_narrow_passes_read_other_lanes_buffers_between_barriers():
     assert len(reads) >= 4
     assert any(b < min(reads) for b in barriers), "no barrier before the first read of another lane's buffer"
     assert any(max(reads) < b < body.index("return") for b in barriers), "no barrier between the reads and the return"
+
+
+def test_deep_paths_ring_is_handed_over_behind_fences():
+    """Both flags of the ring: a fence between the accesses and the raising of the
+    flag, and one between the seen flag and the accesses."""
+    wait = function("linear.cu", "wait_smem")
+    assert re.search(r"while.*\}\s*\}\s*__threadfence_block\(\);\s*return __all_sync", wait, re.S)
+    body = function("linear.cu", "lin_deep_kernel")
+    for flag in (r"R\.rounds = i;", r"R\.full\[b %"):
+        assert re.search(r"__syncwarp\(\);\s*__threadfence_block\(\);\s*if \(c == 0\) " + flag, body), flag
