@@ -22,7 +22,9 @@
 // Paths are ordered by depth (their deepest chain of reaches): one is only fed by
 // shallower ones, so handing them out in that order can wait but not deadlock. The
 // outflows are their own flags: the array is filled with a NaN that no operation
-// produces, and a reader looks until it finds another value (bounded).
+// produces, and a reader looks until it finds another value, or until a whole wait
+// budget has passed in which no sweep anywhere came to its end or 64 rounds on (14 to
+// 130 us; a count every eight rounds costs 0.1 ms of 2.6).
 // What bounds it: the longest path's rounds (the 2.7 M-segment network: 7,400
 // segments), so deep paths get a block each and the fewest steps per lane; the many
 // short ones share warps and take 8 steps per lane, their bound being the loads.
@@ -106,9 +108,37 @@ struct LinRun {
     const float* qlat;              // [T][S]
     const int2* items;              // {first path, paths} of a warp's sweep, shallow first
     int n_items;
-    int* ticket;
+    int* ticket;                    // sweeps taken; a warp or block asks again at the end of one
+    int* progress;                  // counts 64 rounds of a sweep
     int* error;                     // 0 ok, TROUTE_ETIMEOUT
     long long wait_cycles;
+};
+
+// A wait's budget starts again with whatever has been done anywhere since it began.
+struct LinBudget {
+    const LinRun& d;
+    long long t0;
+    int seen;
+    __device__ __forceinline__ explicit LinBudget(const LinRun& run) : d(run)
+    {
+        t0 = clock64();
+        seen = done();
+    }
+    __device__ __forceinline__ int done() const
+    {
+        return *reinterpret_cast<volatile int*>(d.ticket) + *reinterpret_cast<volatile int*>(d.progress);
+    }
+    // whether the wait goes on; it does not once a wait anywhere has run out
+    __device__ __forceinline__ bool left()
+    {
+        if (clock64() - t0 > d.wait_cycles) {
+            const int now = done();
+            if (now == seen) atomicCAS(d.error, 0, TROUTE_ETIMEOUT);
+            seen = now;
+            t0 = clock64();
+        }
+        return *reinterpret_cast<volatile int*>(d.error) == 0;
+    }
 };
 
 __device__ __forceinline__ unsigned ld_out(const unsigned* p) { return *reinterpret_cast<const volatile unsigned*>(p); }
@@ -118,14 +148,11 @@ __device__ __forceinline__ float wait_out(const LinRun& d, const unsigned* p)
 {
     unsigned v = ld_out(p);
     if (v == kUnset) {
-        const long long t0 = clock64();
+        LinBudget budget(d);
         do {
             __nanosleep(100);
             v = ld_out(p);
-            if (v == kUnset && (clock64() - t0 > d.wait_cycles || *reinterpret_cast<volatile int*>(d.error))) {
-                atomicCAS(d.error, 0, TROUTE_ETIMEOUT);
-                v = 0;
-            }
+            if (v == kUnset && !budget.left()) v = 0;
         } while (v == kUnset);
     }
     return __uint_as_float(v);
@@ -218,6 +245,7 @@ __global__ void __launch_bounds__(128) lin_shallow_kernel(const LinRun d, int lc
             for (int j = 0; j < K; ++j) o[j] = 0.0f;
             const int rounds = n_max + lanes - 1;
             for (int i = 0; i < rounds; ++i) {
+                if ((i & 63) == 63 && lane == 0) atomicAdd(d.progress, 1);
                 const int k = i - c;
                 float q = __shfl_up_sync(kFull, q_end, 1, C);
                 if (live && k >= 0 && k < n) {
@@ -295,11 +323,10 @@ __device__ __forceinline__ bool wait_smem(const LinRun& d, const volatile int* p
 {
     bool ok = true;
     if (*p < want) {
-        const long long t0 = clock64();
+        LinBudget budget(d);
         while (ok && *p < want) {
             __nanosleep(20);
-            if (clock64() - t0 > d.wait_cycles) atomicCAS(d.error, 0, TROUTE_ETIMEOUT);
-            ok = *reinterpret_cast<volatile int*>(d.error) == 0;
+            ok = budget.left();
         }
     }
     __threadfence_block();
@@ -338,6 +365,7 @@ __global__ void __launch_bounds__(32 * (NP + 1), 1) lin_deep_kernel(const LinRun
                         __threadfence_block();   // the rounds' reads, before their slots are filled again
                         if (c == 0) R.rounds = i;
                         if (i < n && !wait_smem(d, &R.full[(i >> 3) % (W / 8)], (i >> 3) + 1)) break;
+                        if (c == 0 && (i & 63) == 0) atomicAdd(d.progress, 1);   // (arrives before the next fence)
                         __syncwarp();
                     }
                     const int k = i - c;
@@ -452,7 +480,7 @@ __global__ void lin_init_kernel(LinRun d, int n_paths, float* out0)
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n_paths; p += gridDim.x * blockDim.x)
         out0[p] = d.Q[d.seg[d.path_ptr[p + 1] - 1].idx];
     if (blockIdx.x == 0 && threadIdx.x < 2) d.ticket[threadIdx.x] = 0;
-    if (blockIdx.x == 0 && threadIdx.x == 2) *d.error = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 2) *d.error = *d.progress = 0;
 }
 
 // Segment records in path order, one thread per reach: reach r's segments start at
@@ -529,7 +557,7 @@ struct troute_linear {
     long long S = 0;
     std::vector<int> depth_ptr;      // paths of each depth (shallow first)
     int deep_from = 0;               // first path that gets a warp of its own
-    DArr<int> path_ptr, ups, ctr;    // ctr: two tickets, error
+    DArr<int> path_ptr, ups, ctr;    // ctr: two tickets, error, progress
     DArr<LinSeg> seg;
     DArr<float> out0;
     DArr<unsigned> out;
@@ -644,7 +672,7 @@ static int lin_build(troute_linear* L, const troute_topo* topo, const float* c1,
         (rc = put(d_up, up, (size_t)R + 1)) || (rc = put(d_ui, ui, nnz)) || (rc = put(d_main, main_up.data(), R)) ||
         (rc = put(d_path, path.data(), R)) || (rc = put(d_off, off.data(), R)) ||
         (rc = put(L->path_ptr, ptr.data(), (size_t)P + 1)) || (rc = put(L->deep, deep.data(), deep.size())) ||
-        (rc = L->seg.alloc((size_t)ptr[P])) || (rc = L->ups.alloc(nnz)) || (rc = L->out0.alloc(P)) || (rc = L->ctr.alloc(3)))
+        (rc = L->seg.alloc((size_t)ptr[P])) || (rc = L->ups.alloc(nnz)) || (rc = L->out0.alloc(P)) || (rc = L->ctr.alloc(4)))
         return rc;
     for (int k = 0; k < 4; ++k)
         if ((rc = put(d_c[k], cs[k], (size_t)S))) return rc;
@@ -772,6 +800,7 @@ extern "C" int troute_linear_run_device(troute_linear* L, const float* qlat_dev,
         d.Q = q_dev;
         d.qlat = qlat_dev + (size_t)t0 * (size_t)L->S;
         d.error = L->ctr.p + 2;
+        d.progress = L->ctr.p + 3;
         d.wait_cycles = wait_cycles > 0 ? wait_cycles : 8000000000LL;
         d.ticket = L->ctr.p;
         // shallow paths: 8 steps per lane, up to 8 lanes each
