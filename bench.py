@@ -210,18 +210,43 @@ def profiled(key: str, warm: bool):
     return profiled_file(key, "route_dataflow_warm_ens256.md" if warm else "route_kernel_c1.md")
 
 
+def routed_pieces(topo: dict, segments: int) -> dict:
+    """A network as the ready-queue kernel takes it in a handle of `segments`: its
+    reaches in pieces of one segment up to 131,072 segments, of two up to 1,048,576
+    (item_segments in network.cpp), whole above."""
+    piece = 1 if segments <= 1 << 17 else 2 if segments <= 1 << 20 else 0
+    if not piece:
+        return topo
+    ln = np.asarray(topo["reach_seg_len"], np.int64)
+    n = np.maximum(1, -(-ln // piece))                 # pieces of each reach
+    first = np.cumsum(n) - n
+    reach = np.repeat(np.arange(len(ln)), n)
+    j = np.arange(n.sum()) - first[reach]
+    up_ptr = np.asarray(topo["reach_up_ptr"], np.int64)
+    up_idx = np.asarray(topo["reach_up_idx"], np.int64)
+    ups = np.where(j == 0, np.diff(up_ptr)[reach], 1)
+    ptr = np.concatenate([[0], np.cumsum(ups)])
+    idx = np.repeat(np.arange(len(j)) - 1, ups)        # the piece before ...
+    idx[np.repeat(j == 0, ups)] = first[up_idx] + n[up_idx] - 1   # ... or the upstream reaches' last ones
+    return {"n_segments": int(topo["n_segments"]),
+            "reach_seg_start": (np.asarray(topo["reach_seg_start"])[reach] + piece * j).astype(np.int32),
+            "reach_seg_len": np.minimum(piece, ln[reach] - piece * j).astype(np.int32),
+            "reach_up_ptr": ptr.astype(np.int32), "reach_up_idx": idx.astype(np.int32)}
+
+
 def critical_path_bound(T, w, n_ts: int, it_per_solve: float, sm_mhz, kernel_ms: float) -> dict:
     """The dependency graph's critical path of one bench step set against the
     FP64 pipe: the longest chain of segment solves when a reach takes its steps
-    one after another (troute_critical_path; networks of up to 1,048,576 segments
-    are routed in pieces of reaches, whose chain is shorter), each
+    one after another (troute_critical_path), each
     solve (iterations + 1) passes, each pass at least the FP64 warp instructions
     of a narrow pass x 64 cycles (one FP64 warp instruction per 64 cycles per
-    SMSP, however few lanes are busy)."""
-    if "batch" in w:
-        chain = max(T.critical_path(n["topo"], n_ts) for n in w["batch"])
-    else:
-        chain = T.critical_path(w["topo"], n_ts)
+    SMSP, however few lanes are busy). `as_routed`: the same for what the kernel
+    waits for, the chain of the pieces that reaches of smaller networks are routed
+    in, and solves of `iterations` passes, as one begun by a narrow pass evaluates
+    its two first depths together. Both take the mean solve; a chain that is waited
+    for has longer ones."""
+    nets = [n["topo"] for n in w["batch"]] if "batch" in w else [w["topo"]]
+    chain = max(T.critical_path(t, n_ts) for t in nets)
     out = {"segment_solves": chain, "passes_per_solve": it_per_solve + 1.0}
     instr, src = profiled_file("fp64_instr_narrow_pass", PASSES)
     if instr is None:
@@ -230,6 +255,10 @@ def critical_path_bound(T, w, n_ts: int, it_per_solve: float, sm_mhz, kernel_ms:
     bound_ms = chain * (it_per_solve + 1.0) * pass_us / 1e3
     out.update({"fp64_instr_per_pass": instr, "instr_source": f"profiles/{src}", "pass_us_min": pass_us,
                 "lower_bound_ms": bound_ms, "kernel_ms": kernel_ms, "kernel_over_bound": kernel_ms / bound_ms})
+    routed = max(T.critical_path(routed_pieces(t, w["S"]), n_ts) for t in nets)
+    routed_ms = routed * it_per_solve * pass_us / 1e3
+    out["as_routed"] = {"segment_solves": routed, "passes_per_solve": it_per_solve, "lower_bound_ms": routed_ms,
+                        "kernel_over_bound": kernel_ms / routed_ms}
     return out
 
 
@@ -730,8 +759,8 @@ def run_ours(args, dist: Dist):
 
     # roofline: the FP64 pipe (the bound) from this run's own solving warp passes,
     # against the measured FP64 issue rate; the HBM fraction beside it
-    instr, instr_src = profiled_file("fp64_instr_mean_pass_" + ("batched" if "members" in w or "batch" in w else "single"),
-                                     PASSES)
+    batched = "members" in w or "batch" in w
+    instr, instr_src = profiled_file("fp64_instr_mean_pass_" + ("batched" if batched else "single"), PASSES)
     fp64_warp_instr = stats["solve_passes"] * (instr or 0.0)
     achieved = fp64_warp_instr * 32 / (kernel_ms / 1e3) / 1e12
     peak = fp64_rate["warp_instr_per_s"] * 32 / 1e12
@@ -745,7 +774,10 @@ def run_ours(args, dist: Dist):
                               "instructions per solving pass x 32 lanes / launch time; peak = the FP64 issue rate "
                               "measured in this run (troute_measure_fp64_rate, independent DMUL chains on every SM) "
                               "x 32 lanes; the solver has no FMA contraction, so an FP64 lane operation is a flop",
-                "fp64_instr_per_solving_pass": instr, "instr_source": f"profiles/{instr_src} (ncu instruction mix)",
+                "fp64_instr_per_solving_pass": instr,
+                "instr_source": f"profiles/{instr_src} (ncu instruction mix of "
+                                + ("an ensemble of 256 members of 20,000 segments)" if batched else
+                                   "a 200,000-segment tree, whose mean of full and narrow passes is taken)"),
                 "fp64_peak_warp_instr_per_s": fp64_rate["warp_instr_per_s"],
                 "traffic_source": f"scaled: DRAM bytes per segment-step of the ncu capture in profiles/{tr_src} x "
                                   f"the segment-steps of one launch (this launch is too large to capture)",
