@@ -98,7 +98,7 @@ __device__ __forceinline__ double pow_near_one(double x, bool odd, const Role& k
 // quotient (lanes 1, 2) lanes 0 and 3 form the Manning discharge. W and V hold -G
 // and 1/G on lanes 1 and 2 (1/G = 0: none), R^(2/3) and the area on 0 and 3.
 struct QuadFlow {
-    double q, C4, Qmn;   // on all lanes of the quad
+    double q, Qmn;   // on all lanes of the quad
 };
 
 __device__ __forceinline__ QuadFlow quad_flow(const Role& k, int quad, double num, int lo2, double Km, double W, double V,
@@ -125,7 +125,6 @@ __device__ __forceinline__ QuadFlow quad_flow(const Role& k, int quad, double nu
     double C4 = lane_get(m, quad | 3);
     if (__any_sync(0xffffffffu, __double2hiint(C4) < 0))
         if (lo2 && fp_lt0(C4) && fp_abs_gt(C4, S3)) C4 = -S3;
-    o.C4 = C4;
     o.q = S3 + C4;
     return o;
 }
@@ -152,8 +151,8 @@ __device__ __forceinline__ bool surely_more(double h, double step, const Tol& to
 // before the last.
 //
 // Between its passes the state of a solve stays on its octet, and the loop around
-// (claims, item starts, publishing: 4 k cycles of a lone warp beside the pass's 8 k)
-// is not run. 200,000 segments, 24 steps: 121 -> 114 ms.
+// (claims, item starts, publishing: 4 k cycles of a lone warp beside the pass's 6.4 k)
+// is not run. 200,000 segments, 24 steps: 121 -> 114 ms, when a pass took 7.3 k.
 template <typename Leave>
 __device__ __forceinline__ bool narrow_passes(Lane& L, unsigned smask, const RunDev& run, double2* warp_seg, PassOut& o,
                                               int& extra, Leave leave)

@@ -883,7 +883,7 @@ static void wave_prefix(const std::vector<int>& lb_ptr, int L, int n_ts, std::ve
 
 // A run of n_ts steps is routed in chunks whose per-step scratch (dependency
 // counters, ready-queue entries and outflow history of the dataflow kernel,
-// ~20 B per reach-step) fits a memory budget: cfg.max_chunk_steps if set,
+// 20 B per item and step) fits a memory budget: cfg.max_chunk_steps if set,
 // else a third of the free device memory at the first run.
 struct RunPlan {
     int chunk = 0, n_full = 0, rem = 0;

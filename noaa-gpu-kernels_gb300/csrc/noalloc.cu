@@ -9,7 +9,8 @@
 // scratch memory, the per-block solve counters, in a fixed array compiled
 // into the library. Every GPU that loads the library holds that array (about
 // 1.7 MB) until the process exits. The caller still passes every input and
-// output array.
+// output array. It runs one thread per reach, so a warp takes as long as its longest
+// reach and slowest solve: for many reaches the other entry point is the faster one.
 //
 // Limits and behaviour:
 //  - at most kNoAllocMaxBlocks blocks of kNoAllocThreads reaches, i.e.

@@ -106,8 +106,7 @@ __device__ __forceinline__ int claim(int* avail, unsigned long long* head, int w
 // Loads the reach head inflows of (ri, tau) (all its dependencies are
 // complete) and starts its first segment.
 __device__ __forceinline__ void start_item(Lane& L, int ri, int tau, int t_base, const NetDev& net,
-                                           const RunDev& run, const DataflowDev& df, LocalStats& ls,
-                                           unsigned int* hist_s, double2* slot)
+                                           const RunDev& run, const DataflowDev& df, double2* slot)
 {
     const int R = df.n_item;
     const int4* rec = reinterpret_cast<const int4*>(df.item + ri);
@@ -330,7 +329,7 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
 
         // ---- lanes starting an item, then a segment (the one inlined
         // start_item and begin_segment) ----
-        if (L.mode == L_START) start_item(L, L.ri, L.tau, t_base, net, run, df, ls, hist_s, seg_slot);
+        if (L.mode == L_START) start_item(L, L.ri, L.tau, t_base, net, run, df, seg_slot);
         if (L.mode == L_BEGIN) L.mode = begin_segment(L, net, run, ls, hist_s, seg_slot) ? L_SOLVE : L_DONE;
 
         // ---- one pass of the solving lanes ----
@@ -470,8 +469,8 @@ __global__ void TROUTE_DF_BOUNDS route_dataflow_kernel(NetDev net, RunDev run, D
     flush_stats(ls, hist_s, run.stats);
 }
 
-// Run set-up on the device: queue tail = number of headwater items (already
-// copied to the queue front), rh[0] = outflow of the step before the run.
+// Run set-up on the device: the queue starts empty, the heads are a list of their own
+// with n_avail.x of them to be claimed; rh[0] = outflow of the step before the run.
 __global__ void dataflow_init_kernel(NetDev net, RunDev run, DataflowDev df)
 {
     const int t_base = *run.step_base;
