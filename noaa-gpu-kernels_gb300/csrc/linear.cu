@@ -116,44 +116,65 @@ struct LinRun {
 
 // A wait's budget starts again with whatever has been done anywhere since it began.
 struct LinBudget {
-    const LinRun& d;
-    long long t0;
+    const int *ticket, *progress;
+    int* error;
+    long long wait_cycles, t0;
     int seen;
-    __device__ __forceinline__ explicit LinBudget(const LinRun& run) : d(run)
+    __device__ __forceinline__ explicit LinBudget(const LinRun& d)
+        : ticket(d.ticket), progress(d.progress), error(d.error), wait_cycles(d.wait_cycles)
     {
         t0 = clock64();
         seen = done();
     }
     __device__ __forceinline__ int done() const
     {
-        return *reinterpret_cast<volatile int*>(d.ticket) + *reinterpret_cast<volatile int*>(d.progress);
+        return *reinterpret_cast<const volatile int*>(ticket) + *reinterpret_cast<const volatile int*>(progress);
     }
     // whether the wait goes on; it does not once a wait anywhere has run out
     __device__ __forceinline__ bool left()
     {
-        if (clock64() - t0 > d.wait_cycles) {
+        if (clock64() - t0 > wait_cycles) {
             const int now = done();
-            if (now == seen) atomicCAS(d.error, 0, TROUTE_ETIMEOUT);
+            if (now == seen) atomicCAS(error, 0, TROUTE_ETIMEOUT);
             seen = now;
             t0 = clock64();
         }
-        return *reinterpret_cast<volatile int*>(d.error) == 0;
+        return *reinterpret_cast<volatile int*>(error) == 0;
     }
 };
 
 __device__ __forceinline__ unsigned ld_out(const unsigned* p) { return *reinterpret_cast<const volatile unsigned*>(p); }
 
-// The outflow at p, waited for.
+// The outflow at p, waited for. In line for the shallow sweeps, which a call costs
+// registers (2.7 M segments, 48 steps 2.60 -> 2.79 ms), and for deep paths of one or two
+// steps a lane; a call where the deep paths' loading warps have many places to wait
+// (144 steps: 55.0 -> 62.8 G segment-steps/s).
+__device__ __noinline__ unsigned wait_on(LinBudget budget, const unsigned* p)
+{
+    unsigned v;
+    do {
+        __nanosleep(100);
+        v = ld_out(p);
+        if (v == kUnset && !budget.left()) v = 0;
+    } while (v == kUnset);
+    return v;
+}
+
+template <bool kCall>
 __device__ __forceinline__ float wait_out(const LinRun& d, const unsigned* p)
 {
     unsigned v = ld_out(p);
     if (v == kUnset) {
         LinBudget budget(d);
-        do {
-            __nanosleep(100);
-            v = ld_out(p);
-            if (v == kUnset && !budget.left()) v = 0;
-        } while (v == kUnset);
+        if (kCall) {
+            v = wait_on(budget, p);
+        } else {
+            do {
+                __nanosleep(100);
+                v = ld_out(p);
+                if (v == kUnset && !budget.left()) v = 0;
+            } while (v == kUnset);
+        }
     }
     return __uint_as_float(v);
 }
@@ -169,12 +190,13 @@ struct LinData {
 
 // Inflow of a reach with more than two upstream reaches: their outflows and the
 // path's own (`own`), added in the network's order from 0.
+template <bool kCall>
 __device__ __forceinline__ float sum_many(const LinRun& d, int up, int n_up, int t, float own)
 {
     float sum = 0.0f;
     for (int m = 0; m < n_up; ++m) {
         const int u = __ldg(d.ups + up + m);
-        sum += u < 0 ? own : t < 0 ? __ldg(d.out0 + u) : wait_out(d, d.out + (size_t)u * (size_t)d.Tp + t);
+        sum += u < 0 ? own : t < 0 ? __ldg(d.out0 + u) : wait_out<kCall>(d, d.out + (size_t)u * (size_t)d.Tp + t);
     }
     return sum;
 }
@@ -253,10 +275,10 @@ __global__ void __launch_bounds__(128) lin_shallow_kernel(const LinRun d, int lc
                     float po = above_q;
                     // (a headwater's first segment is the path's first: o and po are 0)
                     if (x.kind == kMany) {
-                        po = sum_many(d, x.up, x.n_up, t0 - 1, po);
+                        po = sum_many<false>(d, x.up, x.n_up, t0 - 1, po);
 #pragma unroll
                         for (int j = 0; j < K; ++j)
-                            if (j < nk) o[j] = sum_many(d, x.up, x.n_up, t0 + j, o[j]);
+                            if (j < nk) o[j] = sum_many<false>(d, x.up, x.n_up, t0 + j, o[j]);
                     } else if (x.kind != kInner) {
                         // sums from +0, as written: 0 + own (+ light)
                         po = 0.0f + po;
@@ -264,10 +286,10 @@ __global__ void __launch_bounds__(128) lin_shallow_kernel(const LinRun d, int lc
                         for (int j = 0; j < K; ++j) o[j] = 0.0f + o[j];
                         if (x.kind == kTwo) {
                             const unsigned* u = d.out + (size_t)x.up * (size_t)d.Tp + t0;
-                            po += t0 && x.up_prev == kUnset ? wait_out(d, u - 1) : __uint_as_float(x.up_prev);
+                            po += t0 && x.up_prev == kUnset ? wait_out<false>(d, u - 1) : __uint_as_float(x.up_prev);
 #pragma unroll
                             for (int j = 0; j < K; ++j)
-                                if (j < nk) o[j] += x.un[j] == kUnset ? wait_out(d, u + j) : __uint_as_float(x.un[j]);
+                                if (j < nk) o[j] += x.un[j] == kUnset ? wait_out<false>(d, u + j) : __uint_as_float(x.un[j]);
                         }
                     }
                     above_q = q;
@@ -336,6 +358,7 @@ __device__ __forceinline__ bool wait_smem(const LinRun& d, const volatile int* p
 template <int K, int W, int NP>
 __global__ void __launch_bounds__(32 * (NP + 1), 1) lin_deep_kernel(const LinRun d)
 {
+    constexpr bool kCall = K > 2;   // waiting for other paths
     static_assert(W % 8 == 0 && W >= 40 + 8, "a batch's slots are free 40 rounds after its segments were first used");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     DeepRing<K, W>& R = *reinterpret_cast<DeepRing<K, W>*>(smem_raw);
@@ -380,10 +403,10 @@ __global__ void __launch_bounds__(32 * (NP + 1), 1) lin_deep_kernel(const LinRun
                         if (c == 0) q = R.q0[s];
                         float po;
                         if (R.kind[s] == kMany) {
-                            po = sum_many(d, R.up[s], R.n_up[s], t0 - 1, above_q);
+                            po = sum_many<kCall>(d, R.up[s], R.n_up[s], t0 - 1, above_q);
 #pragma unroll
                             for (int j = 0; j < K; ++j)
-                                if (j < nk) o[j] = sum_many(d, R.up[s], R.n_up[s], t0 + j, o[j]);
+                                if (j < nk) o[j] = sum_many<kCall>(d, R.up[s], R.n_up[s], t0 + j, o[j]);
                         } else {
                             po = (above_q + z) + R.light_prev[s][c];
 #pragma unroll
@@ -456,11 +479,11 @@ __global__ void __launch_bounds__(32 * (NP + 1), 1) lin_deep_kernel(const LinRun
                             if (k0 + u0 + u < n && c < lanes) {
                                 // (only a light outflow can be unset: a value is never waited for elsewhere)
                                 const unsigned* row = d.out + (size_t)su * (size_t)d.Tp + t0;
-                                R.light_prev[s][c] = t0 && prev[u] == kUnset ? wait_out(d, row - 1) : __uint_as_float(prev[u]);
+                                R.light_prev[s][c] = t0 && prev[u] == kUnset ? wait_out<kCall>(d, row - 1) : __uint_as_float(prev[u]);
 #pragma unroll
                                 for (int j = 0; j < K; ++j) {
                                     R.ql[s][j][c] = ql[u][j];
-                                    R.light[s][j][c] = un[u][j] == kUnset ? wait_out(d, row + j) : __uint_as_float(un[u][j]);
+                                    R.light[s][j][c] = un[u][j] == kUnset ? wait_out<kCall>(d, row + j) : __uint_as_float(un[u][j]);
                                 }
                             }
                         }
