@@ -130,7 +130,8 @@ int troute_mc_reach_parallel_cfg(const troute_chparams* p, const double* ql,
                                  double uq, double dt, int nr,
                                  const troute_cfg* cfg, troute_stats* stats);
 /* Device-pointer form of kernel_mc_gpu (all arrays on the device, n_segments
- * = total segments); asynchronous on `stream` (a cudaStream_t, 0 = default).
+ * = total segments); asynchronous on `stream` (a cudaStream_t, 0 = default);
+ * calls may overlap on several streams and in captured graphs.
  * A reach whose segment range lies outside [0, n_segments) is skipped (its
  * outputs are left unwritten). A CUDA error already pending on the calling
  * thread is reported and left pending; nothing is launched. */
@@ -418,7 +419,8 @@ int troute_linear_create(troute_linear** h, const troute_topo* topo, const float
 int troute_linear_destroy(troute_linear* h);
 /* n_ts steps of device lateral inflow [n_ts][n_segments] (float); q_dev
  * [n_segments] holds the discharge before the run and after it. Synchronous;
- * wait_cycles bounds each device wait without progress (0: ~4 s). */
+ * wait_cycles bounds each device wait without progress (0: ~4 s; a path shows
+ * its progress every 64 segments, ~0.1 ms). */
 int troute_linear_run_device(troute_linear* h, const float* qlat_ts_device, int n_ts, float* q_device,
                              long long wait_cycles, void* stream);
 /* One-shot host form of cpu_linear_mc's arguments: coefficients, lateral

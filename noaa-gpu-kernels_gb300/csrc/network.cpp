@@ -518,12 +518,15 @@ static void replicate_layout(const Layout& B, const std::vector<troute_chparams>
 // run takes at least its steps times the passes of its longest reach; a segment by
 // itself starts a step as soon as the segment before it has made that step, and
 // reaches are pipelines. An item costs its start and its publishing, which matters
-// when the lanes are full. Whole / two / one segment: 1,000 segments, 288 steps
-// 37.4 / 13.8 / 10.3 ms; 20,000, 96 steps 23.4 / 15.9 / 13.8; 65,000, 24 steps
-// 17.2 / 16.1 / 16.1 and at rtol 1e-8 59.4 / 53.0 / 51.7; 200,000, 24 steps 29.3 /
-// 28.7 / 31.1 and at rtol 1e-8 115.7 / 109.1 / 110.2; 530,824, 24 steps, rtol 1e-8
-// 111.3 / 107.5 / 109.6; 64 members of 20,000, 16 steps, warm start 93.9 / 95.8 /
-// 99.4; 2.7 M, 24 steps, rtol 1e-8 509 / 527 / 527.
+// when the lanes are full. From a developed state, whole / two / one segment: 1,000
+// segments, 288 steps 35.8 / 14.7 / 11.1 ms; 20,000, 96 steps 29.1 / 22.6 / 22.0;
+// 24 steps at rtol 1e-8: 65,000 72.7 / 68.4 / 68.2; 131,000 105.0 / 98.5 / 99.4;
+// 200,000 120.9 / 116.5 / 118.1; 530,824 197.5 / 194.7 / 196.5; 1 M 265.9 / 268.4 /
+// 280.9; 2.7 M 499.6 / 508.7 / 521.8; 64 members of 20,000, 16 steps, warm start
+// 91.0 / 88.4 / 89.0. The lines lie where the next form has caught up at the tight
+// tolerance. (At the reference tolerance solves are short and whole reaches are ahead
+// earlier, 24 steps: 65,000 24.5 / 25.4 / 26.7; 131,000 34.0 / 36.5 / 41.5; 200,000
+// 40.5 / 45.2 / 49.4.)
 static int item_segments(long long segments) { return segments <= (1 << 17) ? 1 : segments <= (1 << 20) ? 2 : 0; }
 
 // The items of a layout: its reaches, or pieces of `piece` segments each (0: whole).

@@ -172,11 +172,14 @@ __device__ __forceinline__ void start_item(Lane& L, int ri, int tau, int t_base,
 }
 
 // Threads per block, and the register budget: resident blocks per SM the
-// allocation is sized for, or (TROUTE_DF_MAXNREG) a register cap. Three blocks
-// of 128 (168 registers; 178 without the bound, which would leave two): four
-// blocks spill 176 B and are slower everywhere (64 members of a 20,000-segment
-// tree, warm start, 16 steps: 128.5 against 124.0 ms; a 200,000-segment tree, 24
-// steps: 218 against 196 ms), 64-thread blocks at 14-16 warps likewise.
+// allocation is sized for, or (TROUTE_DF_MAXNREG) a register cap. Two / three / four
+// blocks of 128 take 226 / 168 / 128 registers and spill none / 196 B of stores and
+// 208 of loads / 646 and 708. Three is the best where all lanes are full, which is
+// where the work is largest: 64 members of a 2.7 M-segment network, warm start, 8
+// steps 4,640 / 4,198 ms. A single network waits for its longest path, which the
+// spills lengthen: 1,000 segments, 288 steps 10.0 / 11.1 / 13.9 ms; 200,000, 24 steps,
+// rtol 1e-8 111 / 116 / 132; 64 members of 20,000, warm start, 16 steps 85 / 91 / 105;
+// 2.7 M, 24 steps, rtol 1e-8 485 / 502 / 540.
 #ifndef TROUTE_DF_THREADS
 #define TROUTE_DF_THREADS 128
 #endif
