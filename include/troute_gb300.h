@@ -420,7 +420,7 @@ int troute_linear_destroy(troute_linear* h);
 /* n_ts steps of device lateral inflow [n_ts][n_segments] (float); q_dev
  * [n_segments] holds the discharge before the run and after it. Synchronous;
  * wait_cycles bounds each device wait without progress (0: ~4 s; a path shows
- * its progress every 64 segments, ~0.1 ms). */
+ * its progress at its end and every 64 segments). */
 int troute_linear_run_device(troute_linear* h, const float* qlat_ts_device, int n_ts, float* q_device,
                              long long wait_cycles, void* stream);
 /* One-shot host form of cpu_linear_mc's arguments: coefficients, lateral

@@ -23,8 +23,8 @@
 // shallower ones, so handing them out in that order can wait but not deadlock. The
 // outflows are their own flags: the array is filled with a NaN that no operation
 // produces, and a reader looks until it finds another value, or until a whole wait
-// budget has passed in which no sweep anywhere came to its end or 64 rounds on (14 to
-// 130 us; a count every eight rounds costs 0.1 ms of 2.6).
+// budget has passed in which no sweep anywhere came to its end or 64 rounds on (14 us
+// of a deep path at 48 steps; a count every eight rounds costs 0.1 ms of 2.6).
 // What bounds it: the longest path's rounds (the 2.7 M-segment network: 7,400
 // segments), so deep paths get a block each and the fewest steps per lane; the many
 // short ones share warps and take 8 steps per lane, their bound being the loads.
